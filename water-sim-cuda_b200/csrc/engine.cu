@@ -65,12 +65,10 @@ struct mpm_engine {
     long long g_total = 0;      // grid nodes
     long long cells_total = 0;  // cells of all bins (incl. each overflow bin)
     long long bins_total = 0;   // bin entries: nb + 2 per scene
-    long long bins_scan = 0;    // bins scanned: nb + 1 per scene
+    long long bins_scan = 0;    // bins that can hold particles: nb + 1 per scene
     SimParams* d_prm = nullptr;
     long long* d_poff = nullptr;     // S + 1 first slots
     long long* d_goff = nullptr;     // S + 1 first nodes
-    long long* d_itemoff = nullptr;  // S + 1 first P2G items
-    long long* d_clroff = nullptr;   // S + 1 first listed bins of the set being cleared
     mpm::SceneTable table{};
 
     bool initialized = false;
@@ -102,20 +100,20 @@ struct mpm_engine {
     float4* accum = nullptr;
     float4* vgrid = nullptr;
     float* sdf = nullptr;
-    // Binning: two counter sets (cell counts, bin counts, bin lists) in one
-    // allocation, the bin and cell starts of the current order, and ctl =
-    // {list lengths of set 0 (S), of set 1 (S), P2G work, G2P work, crowded-cell
-    // list length, crowded-cell entries taken}.
+    // Binning: two counter sets (cell counts, bin lists, bin counts) in one
+    // allocation, the bin starts and P2G's item descriptors of the current
+    // order, and ctl = {list lengths of sets 0 and 1, P2G work, crowded-cell
+    // list length}.
     void* bins_mem = nullptr;
     void* tiles_mem = nullptr;  // grid-update tile marks: stamp, mark[bins_total], dirty[bins_total]
     mpm::TileMarks tiles{};
     mpm::BinSet bins[2] = {};
     int32_t* bstart = nullptr;
-    int32_t* cstart = nullptr;
-    uint8_t* corder = nullptr;  // P2G's order of each listed bin's cells
     int32_t* bpart = nullptr;  // chunk sums of the bin scan: scenes x scan_chunks
     int scan_chunks = 1;
+    int2* desc = nullptr;
     uint32_t* ctl = nullptr;
+    mpm::OrderCtl order{};
     uint32_t* d_flags = nullptr;  // [0] health bits, [1] kernel status bits
     uint32_t wait_test = 0;       // MPM_WAIT_TEST_* (test hooks of the bounded device waits)
 
@@ -320,11 +318,11 @@ mpm_status alloc_particles(mpm_engine* e, long long n, int max_n, size_t sort_by
     return MPM_OK;
 }
 
-// Words of one counter set: cell counts, bin counts and bin lists, rounded up
-// to 256 bytes so that the second set's cell counts stay 16-byte aligned for
-// vector access.
+// Words of one counter set: cell counts, bin list (two words per entry) and
+// bin counts, rounded up to 256 bytes so that the second set's cell counts
+// stay 16-byte aligned for vector access.
 size_t bins_set_words(const mpm_engine* e) {
-    return align_up((size_t)e->cells_total + 2 * (size_t)e->bins_total, 64);
+    return align_up((size_t)e->cells_total + 3 * (size_t)e->bins_total, 64);
 }
 size_t bins_bytes(const mpm_engine* e) { return 2 * bins_set_words(e) * sizeof(uint32_t); }
 size_t tiles_bytes(const mpm_engine* e) { return (size_t)(1 + e->bins_total) * sizeof(uint32_t) + (size_t)e->bins_total; }
@@ -334,11 +332,15 @@ void carve_bins(mpm_engine* e) {
     for (int k = 0; k < 2; ++k) {
         uint32_t* s = base + k * bins_set_words(e);  // cell counts first: 16-byte aligned
         e->bins[k].ccount = s;
-        e->bins[k].bcount = s + e->cells_total;
-        e->bins[k].blist = reinterpret_cast<int32_t*>(e->bins[k].bcount + e->bins_total);
-        e->bins[k].nlist = e->ctl + k * e->scenes;
+        e->bins[k].blist = reinterpret_cast<int2*>(s + e->cells_total);  // cells come in 128s: 8-byte aligned
+        e->bins[k].bcount = s + e->cells_total + 2 * e->bins_total;
+        e->bins[k].nlist = e->ctl + k;
     }
+    e->order.work = e->ctl + 2;
+    e->order.crowded = e->ctl + 3;
 }
+constexpr int kCtlWords = 4;
+constexpr size_t kCtlBytes = kCtlWords * sizeof(uint32_t);
 
 // Uploads the scene table (after the particle offsets change).
 mpm_status upload_table(mpm_engine* e) {
@@ -361,6 +363,27 @@ mpm_status upload_table(mpm_engine* e) {
 // (grid_block 0), else none: every node is updated.
 mpm::TileMarks active_tiles(const mpm_engine* e) { return e->tune.grid_block == 0 ? e->tiles : mpm::TileMarks{}; }
 
+// The ordering by counter set `par`, and P2G from parity `par` with the
+// parameters of `sc`.
+int enqueue_order(mpm_engine* e, int par) {
+    return mpm::launch_bin_order(e->table, e->n, e->bins_scan, e->bins[par], e->bins[1 - par], e->order, e->bstart,
+                                 e->bpart, e->scan_chunks, e->pcell, e->ccur, e->gidx, e->desc, e->crowd, e->crowd_cap,
+                                 e->tune.p2g_cell_cap, active_tiles(e), e->d_flags + 1, e->stream);
+}
+int enqueue_p2g(mpm_engine* e, const mpm::SceneTable& sc, int par) {
+    return mpm::launch_p2g(sc, e->n, e->bins_scan, e->P[par], e->gidx, e->bins[par], e->desc, e->crowd, e->crowd_cap,
+                           e->order, e->accum, e->d_flags + 1, e->stream, e->tune.p2g_ctas_per_sm);
+}
+
+// A substep begun with mpm_substep_partial is given up: its ordering's
+// counters (OrderCtl) are zeroed for the next one.
+mpm_status abandon_partial(mpm_engine* e) {
+    if (e->partial_stage != 0)
+        CK(e, cudaMemsetAsync(e->order.work, 0, 2 * sizeof(uint32_t), e->stream));
+    e->partial_stage = 0;
+    return MPM_OK;
+}
+
 // Enqueues stages `from`..`upto` (MPM_STAGE_*) of one substep from parity
 // `par`, for all scenes.  With `marks` (only while capturing a graph), records
 // marks[0..4] as event-record nodes before the ordering and after each stage.
@@ -371,17 +394,11 @@ int enqueue_substep(mpm_engine* e, int par, int from, int upto, const cudaEvent_
         if (marks) cudaEventRecordWithFlags(marks[k], st, cudaEventRecordExternal);
     };
     int launches = 0;
-    uint32_t* work = e->ctl + 2 * e->scenes;
     mark(0);
-    if (from <= MPM_STAGE_SORT && upto >= MPM_STAGE_SORT)
-        launches += mpm::launch_bin_order(sc, e->n, e->bins_scan, e->bins[par], e->bins[1 - par], e->bstart, e->cstart,
-                                          e->pcell, e->ccur, e->gidx, e->corder, e->d_itemoff, e->d_clroff, work, e->bpart,
-                                          e->scan_chunks, active_tiles(e), st);
+    if (from <= MPM_STAGE_SORT && upto >= MPM_STAGE_SORT) launches += enqueue_order(e, par);
     mark(1);
     if (from <= MPM_STAGE_P2G && upto >= MPM_STAGE_P2G)
-        launches += mpm::launch_p2g(sc, e->n, e->bins_scan, e->P[par], e->gidx, e->cstart, e->bins[par], e->corder, e->d_itemoff,
-                                    work, e->accum, e->crowd, e->crowd_cap, e->d_flags + 1, st, e->tune.p2g_ctas_per_sm,
-                                    e->tune.p2g_cell_cap);
+        launches += enqueue_p2g(e, sc, par);
     mark(2);
     if (from <= MPM_STAGE_GRID && upto >= MPM_STAGE_GRID)
         launches += mpm::launch_grid_update(sc, e->prm[0], e->g_total, e->accum, e->vgrid, e->sdf, active_tiles(e), st,
@@ -390,7 +407,7 @@ int enqueue_substep(mpm_engine* e, int par, int from, int upto, const cudaEvent_
     if (from <= MPM_STAGE_G2P && upto >= MPM_STAGE_G2P)
         launches += mpm::launch_g2p(sc, e->prm[0], e->n, e->P[par], e->P[1 - par], e->gidx, e->sigma[par],
                                     e->sigma[1 - par], e->vgrid, e->sdf, e->pcell, e->bins[1 - par],
-                                    e->d_flags, st, nullptr, e->tune.g2p_block);
+                                    e->order.crowded, e->d_flags, st, nullptr, e->tune.g2p_block);
     mark(4);
     return launches;
 }
@@ -518,7 +535,7 @@ mpm_status load_states(mpm_engine* e, const float* const* soa26_host, bool init_
     }
     // Both counter sets empty, then the imported particles filed into set 0.
     CK(e, cudaMemsetAsync(e->bins_mem, 0, bins_bytes(e), e->stream));
-    CK(e, cudaMemsetAsync(e->ctl, 0, (2 * e->scenes + 4) * sizeof(uint32_t), e->stream));
+    CK(e, cudaMemsetAsync(e->ctl, 0, kCtlBytes, e->stream));
     e->kernel_launches += mpm::launch_bin_count(e->table, e->n, e->P[0], e->pcell, e->bins[0], e->stream);
     CK(e, cudaGetLastError());
     e->parity = 0;
@@ -573,7 +590,8 @@ mpm_status export_positions(mpm_engine* e) {
 mpm_status run_steps(mpm_engine* e, int32_t nsub) {
     if (!e->initialized) return record(e, MPM_ERR_NOT_INITIALIZED, "mpm_init_particles has not been called");
     if (nsub < 0) return record(e, MPM_ERR_INVALID_ARGUMENT, "nsub < 0");
-    e->partial_stage = 0;  // a partial substep in progress is discarded (it changed no particle)
+    mpm_status st = abandon_partial(e);  // a partial substep in progress is discarded (it changed no particle)
+    if (st != MPM_OK) return st;
     if (e->accum_dirty) {
         CK(e, cudaMemsetAsync(e->accum, 0, (size_t)e->g_total * sizeof(float4), e->stream));
         e->accum_dirty = false;
@@ -722,19 +740,16 @@ mpm_status create_engine(const mpm_config* cfgs, int32_t count, int32_t device, 
         (err = cudaMalloc(&e->vgrid, (size_t)g_total * sizeof(float4))) != cudaSuccess ||
         (err = cudaMalloc(&e->sdf, (size_t)g_total * sizeof(float))) != cudaSuccess ||
         (err = cudaMalloc(&e->d_flags, 2 * sizeof(uint32_t))) != cudaSuccess ||
-        (err = cudaMalloc(&e->ctl, (2 * count + 4) * sizeof(uint32_t))) != cudaSuccess ||
+        (err = cudaMalloc(&e->ctl, kCtlBytes)) != cudaSuccess ||
         (err = cudaMalloc(&e->bins_mem, bins_bytes(e))) != cudaSuccess ||
         (err = cudaMalloc(&e->tiles_mem, tiles_bytes(e))) != cudaSuccess ||
         (err = cudaMalloc(&e->bstart, (size_t)bins_total * sizeof(int32_t))) != cudaSuccess ||
         (err = cudaMalloc(&e->bpart, (size_t)count * e->scan_chunks * sizeof(int32_t))) != cudaSuccess ||
-        (err = cudaMalloc(&e->cstart, (size_t)cells_total * sizeof(int32_t))) != cudaSuccess ||
         (err = cudaMalloc(&e->ccur, (size_t)cells_total * sizeof(int32_t))) != cudaSuccess ||
-        (err = cudaMalloc(&e->corder, (size_t)cells_total)) != cudaSuccess ||
+        (err = cudaMalloc(&e->desc, (size_t)cells_total * sizeof(int2))) != cudaSuccess ||
         (err = cudaMalloc(&e->d_prm, count * sizeof(SimParams))) != cudaSuccess ||
         (err = cudaMalloc(&e->d_poff, (count + 1) * sizeof(long long))) != cudaSuccess ||
-        (err = cudaMalloc(&e->d_goff, (count + 1) * sizeof(long long))) != cudaSuccess ||
-        (err = cudaMalloc(&e->d_itemoff, (count + 1) * sizeof(long long))) != cudaSuccess ||
-        (err = cudaMalloc(&e->d_clroff, (count + 1) * sizeof(long long))) != cudaSuccess)
+        (err = cudaMalloc(&e->d_goff, (count + 1) * sizeof(long long))) != cudaSuccess)
         return fail(cuda_fail(e, err, "cudaMalloc(grid)"));
     carve_bins(e);
     e->tiles.stamp = static_cast<uint32_t*>(e->tiles_mem);
@@ -818,8 +833,7 @@ mpm_status prepare_large(mpm_engine* e) {
         CK(e, cudaMemsetAsync(e->accum, 0, (size_t)e->g_total * sizeof(float4), e->stream));
         e->accum_dirty = false;
     }
-    e->partial_stage = 0;
-    return MPM_OK;
+    return abandon_partial(e);
 }
 
 // Advection blend of the large step: RATIO substeps under a constant
@@ -831,20 +845,15 @@ float large_blend(const mpm_engine* e) { return (float)(e->ratio + 1) / (float)(
 // learned, collection or uncorrected large-step G2P).
 int enqueue_large(mpm_engine* e, int par, const mpm::LearnArgs* learn) {
     cudaStream_t st = e->stream;
-    uint32_t* work = e->ctl + 2 * e->scenes;
     const SimParams big = large_params(e, 0);
     int launches = 0;
-    launches += mpm::launch_bin_order(e->table, e->n, e->bins_scan, e->bins[par], e->bins[1 - par], e->bstart,
-                                      e->cstart, e->pcell, e->ccur, e->gidx, e->corder, e->d_itemoff, e->d_clroff, work, e->bpart,
-                                          e->scan_chunks, active_tiles(e), st);
-    launches += mpm::launch_p2g(e->table_large, e->n, e->bins_scan, e->P[par], e->gidx, e->cstart, e->bins[par],
-                                e->corder, e->d_itemoff, work, e->accum, e->crowd, e->crowd_cap, e->d_flags + 1, st, e->tune.p2g_ctas_per_sm,
-                                e->tune.p2g_cell_cap);
+    launches += enqueue_order(e, par);
+    launches += enqueue_p2g(e, e->table_large, par);
     launches += mpm::launch_grid_update(e->table_large, big, e->g_total, e->accum, e->vgrid, e->sdf, active_tiles(e), st,
                                         e->tune.grid_block);
     launches += mpm::launch_g2p(e->table_large, big, e->n, e->P[par], e->P[1 - par], e->gidx, e->sigma[par],
-                                e->sigma[1 - par], e->vgrid, e->sdf, e->pcell, e->bins[1 - par], e->d_flags,
-                                st, learn);
+                                e->sigma[1 - par], e->vgrid, e->sdf, e->pcell, e->bins[1 - par], e->order.crowded,
+                                e->d_flags, st, learn);
     return launches;
 }
 
@@ -852,7 +861,7 @@ int enqueue_large(mpm_engine* e, int par, const mpm::LearnArgs* learn) {
 // emptied first): the state of parity `par` becomes the current one again.
 mpm_status rebin(mpm_engine* e, int par) {
     CK(e, cudaMemsetAsync(e->bins_mem, 0, bins_bytes(e), e->stream));
-    CK(e, cudaMemsetAsync(e->ctl, 0, (2 * e->scenes + 4) * sizeof(uint32_t), e->stream));
+    CK(e, cudaMemsetAsync(e->ctl, 0, kCtlBytes, e->stream));
     e->kernel_launches += mpm::launch_bin_count(e->table, e->n, e->P[par], e->pcell, e->bins[par], e->stream);
     CK(e, cudaGetLastError());
     e->parity = par;
@@ -883,7 +892,7 @@ int enqueue_fallback(mpm_engine* e, int par) {
     cudaStream_t st = e->stream;
     int launches = 0;
     launches += mpm::launch_fill(static_cast<float*>(e->bins_mem), (long long)(bins_bytes(e) / sizeof(float)), 0.0f, st);
-    launches += mpm::launch_fill(reinterpret_cast<float*>(e->ctl), 2 * e->scenes + 4, 0.0f, st);
+    launches += mpm::launch_fill(reinterpret_cast<float*>(e->ctl), kCtlWords, 0.0f, st);
     launches += mpm::launch_bin_count(e->table, e->n, e->P[par], e->pcell, e->bins[par], st);
     int q = par;
     for (int r = 0; r < e->ratio; ++r) {
@@ -896,7 +905,7 @@ int enqueue_fallback(mpm_engine* e, int par) {
         launches += mpm::launch_copy_words(e->sigma[1 - par], e->sigma[q], e->n, st);
         launches += mpm::launch_copy_words(sets + (size_t)(1 - par) * bins_set_words(e), sets + (size_t)q * bins_set_words(e),
                                            (long long)bins_set_words(e), st);
-        launches += mpm::launch_copy_words(e->ctl + (1 - par) * e->scenes, e->ctl + q * e->scenes, e->scenes, st);
+        launches += mpm::launch_copy_words(e->bins[1 - par].nlist, e->bins[q].nlist, 1, st);
     }
     return launches;
 }
@@ -1032,17 +1041,14 @@ extern "C" void mpm_destroy(mpm_engine* e) {
     free_dev(e->sdf);
     free_dev(e->bins_mem);
     free_dev(e->tiles_mem);
-    free_dev(e->bstart);
     free_dev(e->ccur);
+    free_dev(e->bstart);
     free_dev(e->bpart);
-    free_dev(e->corder);
-    free_dev(e->cstart);
+    free_dev(e->desc);
     free_dev(e->ctl);
     free_dev(e->d_prm);
     free_dev(e->d_poff);
     free_dev(e->d_goff);
-    free_dev(e->d_itemoff);
-    free_dev(e->d_clroff);
     free_dev(e->d_flags);
     free_dev(e->staging);
     free_dev(e->d_prm_large);
@@ -1182,6 +1188,7 @@ extern "C" mpm_status mpm_substep_partial(mpm_engine* e, int32_t upto) {
     // Continue the substep in progress, or start a new one.
     int from = e->partial_stage + 1;
     if (upto <= e->partial_stage) from = MPM_STAGE_SORT;
+    if (from == MPM_STAGE_SORT && (s = abandon_partial(e)) != MPM_OK) return s;
     if (from == MPM_STAGE_SORT && e->accum_dirty) {
         CK(e, cudaMemsetAsync(e->accum, 0, (size_t)e->g_total * sizeof(float4), e->stream));
         e->accum_dirty = false;
@@ -1851,7 +1858,7 @@ extern "C" mpm_status mpm_autotune(mpm_engine* e, int32_t repeats, mpm_tuning* o
         CK(e, cudaMemsetAsync(e->accum, 0, (size_t)e->g_total * sizeof(float4), e->stream));
         e->accum_dirty = false;
     }
-    e->partial_stage = 0;
+    if ((s = abandon_partial(e)) != MPM_OK) return s;
     cudaEvent_t a = nullptr, b = nullptr;
     CK(e, cudaEventCreate(&a));
     if (cudaEventCreate(&b) != cudaSuccess) {

@@ -51,16 +51,26 @@ int launch_radix_sort(const int32_t* keys, int n, const SortScratch& s, int32_t*
 // slots, cells and bins are global (device_math.cuh).  P is the
 // particle-major state, ordered by cell of the binning that produced it.
 // pcell[j] is the global cell of slot j; ccur holds one slot cursor per
-// cell, which the ordering's scatter draws the cell's slots from.  A counter set holds the cell counts (global cells), the
-// bin counts and the per-scene lists of bins that hold particles (global bin
-// entries: nb + 2 per scene), and the per-scene list lengths nlist[scene].
-// Two sets alternate: a substep orders the particles by one and its G2P
-// fills the other, which that substep clears first.
+// cell, which the ordering's scatter draws the cell's slots from.  A counter
+// set holds the cell counts (global cells), the bin counts, and the list of
+// the bins that hold particles, as (scene, bin) in the order they were first
+// reached, with its length *nlist.  Two sets alternate: a substep orders the
+// particles by one and its G2P fills the other, which that substep clears
+// first.
 struct BinSet {
     uint32_t* ccount;
+    int2* blist;
     uint32_t* bcount;
-    int32_t* blist;
     uint32_t* nlist;
+};
+
+// Counters of one substep, zero before its ordering: P2G's work units taken
+// and the length of the crowded-cell list.  The scatter resets work, G2P
+// resets crowded; an ordering whose substep is abandoned needs it zeroed by
+// the host.
+struct OrderCtl {
+    uint32_t* work;
+    uint32_t* crowded;
 };
 
 // Node tiles of the grid update, one per bin: tile (bx, by, bz) of a scene
@@ -80,32 +90,27 @@ struct TileMarks {
 // Files the n particles of P (all scenes, slot order) into an empty set.
 int launch_bin_count(const SceneTable& sc, long long n, const float* P, int32_t* pcell, const BinSet& set,
                      cudaStream_t st);
-// Order by cell from set `cur`: bstart (global first slots of every bin), cstart
-// (first slot of every cell of a listed bin), corder (P2G's order of each
-// listed bin's cells, one byte per cell, indexed like the cells), gidx[new
-// slot] = old slot, itemoff (the P2G work items of each scene: kBinZ per
-// listed bin, prefix, S + 1 entries) and clroff (the same prefix of `other`'s
-// listed bins, one per bin); clears `other` and the work counters work[0..1];
-// with tiles.mark set, advances tiles.stamp and marks the tiles the listed
-// bins of `cur` reach.
-// bins_total: sum over scenes of nb + 1.  bpart: scenes x scan_chunks ints of
-// scratch; scan_chunks = bin_scan_chunks(largest nb + 1).
+// Order by cell from set `cur`: gidx[new slot] = old slot, desc (P2G's items:
+// kBinZ per listed bin, indexed like the cells), crowd / *ctl.crowded (the
+// crowded-cell list; crowd_cap entries of room, at least n / 4 + 64); clears
+// `other`; with tiles.mark set, advances tiles.stamp and marks the tiles the
+// listed bins of `cur` reach.  bstart: the bins' first slots; bpart: scenes x
+// scan_chunks ints of scratch, scan_chunks = bin_scan_chunks(largest nb + 1).
+// bins_total: sum over scenes of nb + 1.
+// cell_cap: particles of a cell its own lane sums in P2G before the rest goes
+// to the list (0 = chosen per work item from its cells' counts).
 int launch_bin_order(const SceneTable& sc, long long n, long long bins_total, const BinSet& cur, const BinSet& other,
-                     int32_t* bstart, int32_t* cstart, const int32_t* pcell, int32_t* ccur, int32_t* gidx,
-                     uint8_t* corder, long long* itemoff, long long* clroff, uint32_t* work, int32_t* bpart,
-                     int scan_chunks, const TileMarks& tiles, cudaStream_t st);
-// Chunks of the bin scan for a scene of `bins` scanned bins.
+                     const OrderCtl& ctl, int32_t* bstart, int32_t* bpart, int scan_chunks, const int32_t* pcell,
+                     int32_t* ccur, int32_t* gidx, int2* desc, int4* crowd, int crowd_cap, int cell_cap,
+                     const TileMarks& tiles, uint32_t* status, cudaStream_t st);
+// Chunks of the bin scan for a scene of `bins` bins.
 int bin_scan_chunks(long long bins);
-// P2G over the items of `cur`; gidx maps slots of the new order to P.  Two
-// launches: the items, then the crowded-cell list they fill (crowd: scratch of
-// crowd_cap entries, at least n / 4 + 64; work[2..3] are its counters, reset
-// by the bin scan).  ctas_per_sm: persistent single-warp CTAs per SM (0 = the
-// default 12); cell_cap: particles of a cell its own lane sums before the rest
-// goes to the list (0 = chosen per work item from its cells' counts).
+// P2G over the crowded-cell list and the items of `cur`; gidx maps slots of
+// the new order to P.  ctas_per_sm: persistent single-warp CTAs per SM (0 =
+// the default 12).
 int launch_p2g(const SceneTable& sc, long long n, long long bins_total, const float* P, const int32_t* gidx,
-               const int32_t* cstart, const BinSet& cur, const uint8_t* corder, const long long* itemoff,
-               uint32_t* work, float4* accum, int4* crowd, int crowd_cap, uint32_t* status, cudaStream_t st,
-               int ctas_per_sm = 0, int cell_cap = 0);
+               const BinSet& cur, const int2* desc, const int4* crowd, int crowd_cap, const OrderCtl& ctl,
+               float4* accum, uint32_t* status, cudaStream_t st, int ctas_per_sm = 0);
 // Most P2G CTAs that fit on one SM.
 int p2g_max_ctas_per_sm();
 // p0: the parameters of scene 0, used directly when the table holds one scene.
@@ -132,11 +137,11 @@ struct LearnArgs {
 };
 
 // G2P: slot j of Pout = particle gidx[j] of Pin advanced one substep;
-// sig_out[j] = sig_in[gidx[j]]; files slot j into `next`.  learn: a large
-// step of one scene (LearnArgs), else null.
+// sig_out[j] = sig_in[gidx[j]]; files slot j into `next`; zeroes *crowded
+// (OrderCtl).  learn: a large step of one scene (LearnArgs), else null.
 int launch_g2p(const SceneTable& sc, const SimParams& p0, long long n, const float* Pin, float* Pout,
                const int32_t* gidx, const int32_t* sig_in, int32_t* sig_out, const float4* vgrid, const float* sdf,
-               int32_t* pcell, const BinSet& next, uint32_t* health, cudaStream_t st,
+               int32_t* pcell, const BinSet& next, uint32_t* crowded, uint32_t* health, cudaStream_t st,
                const LearnArgs* learn = nullptr, int block = 256);
 
 // The kernels below take one scene's SimParams and pointers already offset to

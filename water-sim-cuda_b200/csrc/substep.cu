@@ -62,22 +62,20 @@ __device__ __forceinline__ void cp_async_wait() {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Files this lane's particle under global cell `gcell` (global bin `gbin`,
-// bin `bin` of scene `scene`, whose bin entries start at `boff`) of a counter
-// set: one reduction per distinct cell of the warp (no value comes back, so
-// no lane waits on it) and one atomic per distinct bin, whose leader appends
-// the bin to its scene's list when it is the bin's first particle.  The
-// particle's place within its cell is drawn later, by the ordering's scatter.
-// Every lane of the warp must call it; lanes with gcell < 0 take part without
-// counting.
-__device__ __forceinline__ void file_particle(int gcell, int gbin, int bin, int scene, long long boff,
-                                              const BinSet& set) {
+// bin `bin` of scene `scene`) of a counter set: one reduction per distinct
+// cell of the warp (no value comes back, so no lane waits on it) and one
+// atomic per distinct bin, whose leader appends the bin to the set's list when
+// it is the bin's first particle.  The particle's place within its cell is
+// drawn later, by the ordering's scatter.  Every lane of the warp must call
+// it; lanes with gcell < 0 take part without counting.
+__device__ __forceinline__ void file_particle(int gcell, int gbin, int bin, int scene, const BinSet& set) {
     const int lane = threadIdx.x & 31;
     const uint32_t peers = __match_any_sync(0xffffffffu, gcell);
     if (gcell >= 0 && lane == __ffs(peers) - 1) atomicAdd(set.ccount + gcell, (uint32_t)__popc(peers));
     const uint32_t bpeers = __match_any_sync(0xffffffffu, gbin);
     if (gbin >= 0 && lane == __ffs(bpeers) - 1) {
         if (atomicAdd(set.bcount + gbin, (uint32_t)__popc(bpeers)) == 0u)
-            set.blist[boff + atomicAdd(set.nlist + scene, 1u)] = bin;
+            set.blist[atomicAdd(set.nlist, 1u)] = make_int2(scene, bin);
     }
 }
 
@@ -144,32 +142,30 @@ struct SceneLookup {
 
 // ------------------------------------------------------------------ P2G ----
 // P2G (p2GTransferScatter, kernels.cu:6-142).  Persistent single-warp CTAs
-// take work items from a counter; a listed bin (8 x 4 x 4 base cells) has
-// kBinZ items, and item g takes positions 32 g .. 32 g + 31 of the bin's cell
-// order (cell_order: occupied cells by count class, largest first), so the
-// lanes of a warp hold cells of similar counts and no empty ones.  The
-// counter hands out every bin's item 0 before any item 1, and so on, so the
-// longest items start first.  Lane =
-// cell: all particles of a cell scatter to the same 27 nodes, so the lane sums
-// them in registers, reading them through a ring of kRing particles fetched
-// ahead with 16-byte cp.async copies (the gather through gidx costs no
-// registers).  The lane then adds its 27 sums to the warp's footprint, the
-// bin's 10 x 6 x 6 nodes in shared memory: the lanes' cells are distinct, so
-// for one stencil offset their nodes differ and a plain read-add-write per
-// offset is race-free.  A lane sums at most `cap` particles of its cell (a
-// launch parameter; 0 = chosen per work item by item_cap); the rest of a
-// crowded cell (this Tait law resists only expansion, so compressed fluid
-// piles up) goes to a list in chunks of kCrowdChunk particles, which a
-// second launch spreads over all warps (the count order gathers a bin's
-// crowded cells in one item, and one warp working through all of their
-// particles would hold up the kernel).  The footprint's z-planes that the
-// item reached go to global memory with one vector reduction per touched
-// node.  Unlike the reference, no partial sum
-// is dropped (it drops shared-tile cells whose partial mass is <= 1e-9,
-// kernels.cu:132).
+// take work units from a counter: first the chunks of the crowded-cell list,
+// then the items.  A listed bin (8 x 4 x 4 base cells) has kBinZ items, and
+// item g takes positions 32 g .. 32 g + 31 of the bin's cell order
+// (cell_order: occupied cells by count class, largest first), so the lanes of
+// a warp hold cells of similar counts and no empty ones.  The counter hands
+// out every bin's item 0 before any item 1, and so on, so the longest items
+// start first.  Lane = cell: all particles of a cell scatter to the same 27
+// nodes, so the lane sums them in registers, reading them through a ring of
+// kRing particles fetched ahead with 16-byte cp.async copies (the gather
+// through gidx costs no registers).  The lane then adds its 27 sums to the
+// warp's footprint, the bin's 10 x 6 x 6 nodes in shared memory: the lanes'
+// cells are distinct, so for one stencil offset their nodes differ and a plain
+// read-add-write per offset is race-free.  The footprint's z-planes that the
+// item reached go to global memory with one vector reduction per touched node.
+// A lane sums at most `cap` particles of its cell; the rest of a crowded cell
+// (this Tait law resists only expansion, so compressed fluid piles up) is on
+// the list in chunks of kCrowdChunk particles: there the 32 lanes share one
+// cell, and a butterfly reduce-scatter adds up their sums.  (The count order
+// gathers a bin's crowded cells in one item, and one warp working through all
+// of their particles would hold up the kernel.)  The ordering lays out both
+// (cell_scan_kernel).  Unlike the reference, no partial sum is dropped (it
+// drops shared-tile cells whose partial mass is <= 1e-9, kernels.cu:132).
 constexpr int kP2GWarpsPerSM = 12;
 constexpr int kRing = 2;
-constexpr int kGidxStage = 256;   // gather indices of a bin staged in shared memory
 constexpr int kCellCap = 12;      // particles of a cell its own lane sums; the rest: the crowded-cell list
 constexpr int kCrowdChunk = 256;  // particles of a crowded cell per list entry
 constexpr int kTX = kBinX + 2, kTY = kBinY + 2;
@@ -284,7 +280,7 @@ __device__ __forceinline__ void p2g_stencil(const P2GParticle& r, Emit emit) {
 // cells (`full`, one per lane): for each candidate cap the loop costs
 // min(max count, cap) iterations with every lane, plus, per cell above the
 // cap, ceil((count - cap) / 32) whole-warp iterations and one reduce-scatter
-// (about 1.3 iterations) in the crowded-cell launch; the cheapest candidate
+// (about 1.3 iterations) for its list entry; the cheapest candidate
 // wins.  Every cap gives the same sums.  Caps stop at 32: a larger one makes a
 // few long items that hold up the kernel while other warps idle, whereas the
 // list spreads the rest of a crowded cell over all warps.
@@ -304,245 +300,153 @@ __device__ __forceinline__ int item_cap(int full) {
 }
 
 __global__ void __launch_bounds__(32, kP2GWarpsPerSM) p2g_kernel(SceneTable sc, const float* __restrict__ P,
-                                                                  const int32_t* __restrict__ gidx,
-                                                                  const int32_t* __restrict__ cstart, BinSet set,
-                                                                  const uint8_t* __restrict__ corder,
-                                                                  const long long* __restrict__ itemoff,
-                                                                  uint32_t* __restrict__ work,
-                                                                  float4* __restrict__ accum_all, int4* __restrict__ crowd,
-                                                                  int crowd_cap, uint32_t* __restrict__ status, int cap) {
-    pdl_wait();
+                                                                  const int32_t* __restrict__ gidx, BinSet set,
+                                                                  const int2* __restrict__ desc,
+                                                                  const int4* __restrict__ crowd, int crowd_cap,
+                                                                  OrderCtl ctl, float4* __restrict__ accum_all,
+                                                                  uint32_t* __restrict__ status) {
     __shared__ __align__(16) float4 s_ring[kRing][6][32];
     __shared__ float4 s_foot[kFootNodes];
-    __shared__ int32_t s_gidx[kGidxStage];
     const int lane = threadIdx.x;
-    const long long nitems = *reinterpret_cast<volatile const long long*>(itemoff + sc.count);
     for (int q = lane; q < kFootNodes; q += 32) s_foot[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (;;) {
-        int item = 0;
-        if (lane == 0) item = (int)atomicAdd(work, 1u);
-        item = __shfl_sync(0xffffffffu, item, 0);
-        if (item >= nitems) return;
-        // Items: kBinZ per listed bin, scene after scene, group-major within a scene.
-        const int scene = sc.count == 1 ? 0 : scene_of(itemoff, sc.count, item);
-        const SimParams p = sc.prm[scene];
-        // Group-major: every listed bin's group 0 (its most crowded cells) comes
-        // before any group 1, and so on, so that the long items start first.
-        const int local = item - (int)__ldg(itemoff + scene);
-        const int nl = (int)((__ldg(itemoff + scene + 1) - __ldg(itemoff + scene)) / kBinZ);
-        const int bin = __ldg(set.blist + p.boff + local % nl), group = local / nl;
-        if (bin >= p.nb) continue;  // the overflow bin reaches no node
-        float4* accum = accum_all + p.goff;
-        const int bxi = bin % p.nbx, byi = (bin / p.nbx) % p.nby, bzi = bin / (p.nbx * p.nby);
-        // Node origin of the footprint = base cell of the bin's first cell.
-        const int ox = bxi * kBinX - 2, oy = byi * kBinY - 2, oz = bzi * kBinZ - 2;
-        const size_t cb = (size_t)p.coff + (size_t)bin * kBinCells;
-        // This lane's cell (z * 32 + y * 8 + x in the bin), 0xFF for none.
-        const int tcell = __ldg(corder + cb + group * 32 + lane);
-        if (__ballot_sync(0xffffffffu, tcell != 0xFF) == 0u) continue;
-        const bool own = tcell != 0xFF;
-        const int cs = own ? __ldg(cstart + cb + tcell) : 0;
-        const int full = own ? (int)__ldg(set.ccount + cb + tcell) : 0;
-        // The bin's slots (its cells are consecutive in the particle order).
-        const int l0 = __ldg(cstart + cb);
-        const int l1 = __ldg(cstart + cb + kBinCells - 1) + (int)__ldg(set.ccount + cb + kBinCells - 1);
-        const bool staged = l1 - l0 <= kGidxStage;
-        if (staged)
-            for (int q = lane; q < l1 - l0; q += 32) s_gidx[q] = __ldg(gidx + l0 + q);
-        __syncwarp();
-        // Each lane sums its cell's first `icap` particles; the rest of a
-        // crowded cell goes to the crowded-cell list in chunks, which
-        // p2g_crowd_kernel spreads over all warps.
-        const int icap = cap > 0 ? cap : item_cap(full);
-        for (int off = icap; off < full; off += kCrowdChunk) {
-            const uint32_t e = atomicAdd(work + 2, 1u);
-            if (e < (uint32_t)crowd_cap)
-                crowd[e] = make_int4(scene, bin * kBinCells + tcell, cs + off, min(kCrowdChunk, full - off));
-            else
-                atomicOr(status, kStatusCrowdList);
-        }
-        const int cnt = min(full, icap);
-        const int maxc = (int)__reduce_max_sync(0xffffffffu, (unsigned)cnt);
-        float am[27], ax[27], ay[27], az[27];
-        auto src_of = [&](int s) -> const float4* {
-            const int slot = cs + s;
-            const int g = staged ? s_gidx[slot - l0] : __ldg(gidx + slot);
-            return reinterpret_cast<const float4*>(P + (size_t)g * kAFloats);
-        };
-#pragma unroll
-        for (int k = 0; k < 27; ++k) am[k] = ax[k] = ay[k] = az[k] = 0.f;
-#pragma unroll
-        for (int d = 0; d < kRing - 1; ++d) {
-            if (d < cnt) {
-                const float4* src = src_of(d);
-#pragma unroll
-                for (int v = 0; v < 6; ++v) cp_async16(&s_ring[d][v][lane], src + v);
-            }
-            cp_async_commit();
-        }
-        for (int s = 0; s < maxc; ++s) {
-            const int pf = s + kRing - 1;
-            if (pf < cnt) {
-                const float4* src = src_of(pf);
-#pragma unroll
-                for (int v = 0; v < 6; ++v) cp_async16(&s_ring[pf % kRing][v][lane], src + v);
-            }
-            cp_async_commit();
-            cp_async_wait<kRing - 1>();
-            __syncwarp();
-            if (s < cnt) {
-                const int sl = s % kRing;
-                const P2GParticle r = p2g_particle(p, s_ring[sl][0][lane], s_ring[sl][1][lane], s_ring[sl][2][lane],
-                                                   s_ring[sl][3][lane], s_ring[sl][4][lane], s_ring[sl][5][lane]);
-                // Filed under this lane's cell by construction; a mismatch is
-                // recorded, never scattered to a wrong node.
-                if (r.bx - ox != tcell % kBinX || r.by - oy != (tcell / kBinX) % kBinY || r.bz - oz != tcell / 32) {
-                    atomicOr(status, kStatusBinning);
-                } else {
-                    p2g_stencil(r, [&](int k, int, int, int, float m, float mx, float my, float mz) {
-                        am[k] += m;
-                        ax[k] += mx;
-                        ay[k] += my;
-                        az[k] += mz;
-                    });
-                }
-            }
-            __syncwarp();
-        }
-        cp_async_wait<0>();
-        // One lane per cell: distinct nodes for each stencil offset.
-        {
-            const int tx = tcell % kBinX, ty = (tcell / kBinX) % kBinY, tz = (tcell / 32) & (kBinZ - 1);
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-#pragma unroll
-                for (int b = 0; b < 3; ++b)
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        const int k = (c * 3 + b) * 3 + a;
-                        float4* d = &s_foot[((tz + c) * kTY + ty + b) * kTX + tx + a];
-                        __syncwarp();
-                        if (own) {
-                            float4 v = *d;
-                            v.x += am[k];
-                            v.y += ax[k];
-                            v.z += ay[k];
-                            v.w += az[k];
-                            *d = v;
-                        }
-                    }
-        }
-        __syncwarp();
-        // The z-planes the group's cells reach: zmin .. zmax + 2.
-        const int zmin = (int)__reduce_min_sync(0xffffffffu, own ? (unsigned)(tcell / 32) : 0xFFu);
-        const int zmax = (int)__reduce_max_sync(0xffffffffu, own ? (unsigned)(tcell / 32) : 0u);
-        for (int q = zmin * kFootPlane + lane; q < (zmax + 3) * kFootPlane; q += 32) {
-            const int x = ox + q % kTX, y = oy + (q / kTX) % kTY, z = oz + q / kFootPlane;
-            const float4 v = s_foot[q];
-            s_foot[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (node_in_grid(p, x, y, z) && (v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f))  // NaN counts
-                red_add_v4(accum + node_index(p, x, y, z), v.x, v.y, v.z, v.w);
-        }
-        __syncwarp();
-    }
-}
-
-// The crowded-cell list: each entry (scene, bin * 128 + cell, first slot,
-// count <= kCrowdChunk) is the next chunk of a crowded cell's particles.  All
-// 32 lanes take its particles (slot first + lane + 32 s), sum their 27 x 4
-// contributions in registers, reduce-scatter them across the warp (five
-// shuffle steps, each halving the 128 padded sums, so lane l ends with node
-// l's totals) and add them to global memory.
-__global__ void __launch_bounds__(32, kP2GWarpsPerSM) p2g_crowd_kernel(SceneTable sc, const float* __restrict__ P,
-                                                                        const int32_t* __restrict__ gidx,
-                                                                        const int4* __restrict__ crowd, int crowd_cap,
-                                                                        uint32_t* __restrict__ work,
-                                                                        float4* __restrict__ accum_all,
-                                                                        uint32_t* __restrict__ status) {
+    __syncwarp();
     pdl_wait();
-    __shared__ __align__(16) float4 s_ring[kRing][6][32];
-    const int lane = threadIdx.x;
-    const int total = (int)min(*reinterpret_cast<volatile const uint32_t*>(work + 2), (uint32_t)crowd_cap);
-    for (;;) {
-        int item = 0;
-        if (lane == 0) item = (int)atomicAdd(work + 3, 1u);
-        item = __shfl_sync(0xffffffffu, item, 0);
-        if (item >= total) return;
-        const int4 e = crowd[item];
-        const SimParams p = sc.prm[e.x];
-        const int bin = e.y / kBinCells, cell = e.y % kBinCells;
-        const int bxi = bin % p.nbx, byi = (bin / p.nbx) % p.nby, bzi = bin / (p.nbx * p.nby);
-        const int bx = bxi * kBinX - 2 + cell % kBinX, by = byi * kBinY - 2 + (cell / kBinX) % kBinY;
-        const int bz = bzi * kBinZ - 2 + cell / 32;
-        const int first = e.z + lane, cnt = max(0, (e.w - lane + 31) / 32), maxc = (e.w + 31) / 32;
-        float am[27], ax[27], ay[27], az[27];
-#pragma unroll
-        for (int k = 0; k < 27; ++k) am[k] = ax[k] = ay[k] = az[k] = 0.f;
-        auto src_of = [&](int s) -> const float4* {
-            return reinterpret_cast<const float4*>(P + (size_t)__ldg(gidx + first + 32 * s) * kAFloats);
-        };
-#pragma unroll
-        for (int d = 0; d < kRing - 1; ++d) {
-            if (d < cnt) {
-                const float4* src = src_of(d);
-#pragma unroll
-                for (int v = 0; v < 6; ++v) cp_async16(&s_ring[d][v][lane], src + v);
-            }
-            cp_async_commit();
+    const int nl = (int)*reinterpret_cast<volatile const uint32_t*>(set.nlist);
+    const int ncrowd = (int)min(*reinterpret_cast<volatile const uint32_t*>(ctl.crowded), (uint32_t)crowd_cap);
+    const int total = ncrowd + nl * kBinZ;
+    SimParams p = sc.prm[0];
+    // The first unit of a warp is its own index, the next ones come from the
+    // counter: one round trip less where a launch has about a unit per warp.
+    for (int unit = blockIdx.x; unit < total;) {
+        // This lane's particles: slots first + stride * s, s < cnt.
+        int scene, bin, cell, first, cnt, stride;
+        const bool packed = unit < ncrowd;  // a chunk of a crowded cell, for all lanes
+        if (packed) {
+            const int4 e = __ldg(crowd + unit);
+            scene = e.x, bin = e.y / kBinCells, cell = e.y % kBinCells;
+            first = e.z + lane, stride = 32, cnt = max(0, (e.w - lane + 31) / 32);
+        } else {
+            // Group-major: every listed bin's group 0 (its most crowded
+            // cells) comes before any group 1, so the long items start first.
+            const int local = unit - ncrowd;
+            const int2 e = __ldg(set.blist + local % nl);
+            scene = e.x, bin = e.y;
+            const SimParams& ps = sc.prm[sc.count == 1 ? 0 : scene];
+            int2 d = make_int2(0, 0);
+            if (bin < ps.nb)  // the overflow bin reaches no node
+                d = __ldg(desc + (size_t)ps.coff + (size_t)bin * kBinCells + (local / nl) * 32 + lane);
+            cell = d.y & 0xFF, first = d.x, stride = 1, cnt = d.y >> 8;
         }
-        for (int s = 0; s < maxc; ++s) {
-            const int pf = s + kRing - 1;
-            if (pf < cnt) {
-                const float4* src = src_of(pf);
+        const int maxc = (int)__reduce_max_sync(0xffffffffu, (unsigned)cnt);
+        if (maxc > 0) {
+            if (sc.count > 1) p = sc.prm[scene];
+            float4* accum = accum_all + p.goff;
+            const int bxi = bin % p.nbx, byi = (bin / p.nbx) % p.nby, bzi = bin / (p.nbx * p.nby);
+            // Node origin of the footprint = base cell of the bin's first cell.
+            const int ox = bxi * kBinX - 2, oy = byi * kBinY - 2, oz = bzi * kBinZ - 2;
+            const int tx = cell % kBinX, ty = (cell / kBinX) % kBinY, tz = cell / 32;
+            float am[27], ax[27], ay[27], az[27];
 #pragma unroll
-                for (int v = 0; v < 6; ++v) cp_async16(&s_ring[pf % kRing][v][lane], src + v);
+            for (int k = 0; k < 27; ++k) am[k] = ax[k] = ay[k] = az[k] = 0.f;
+            auto fetch = [&](int s) {
+                const float4* src = reinterpret_cast<const float4*>(P + (size_t)__ldg(gidx + first + stride * s) * kAFloats);
+#pragma unroll
+                for (int v = 0; v < 6; ++v) cp_async16(&s_ring[s % kRing][v][lane], src + v);
+            };
+#pragma unroll
+            for (int d = 0; d < kRing - 1; ++d) {
+                if (d < cnt) fetch(d);
+                cp_async_commit();
             }
-            cp_async_commit();
-            cp_async_wait<kRing - 1>();
-            __syncwarp();
-            if (s < cnt) {
-                const int sl = s % kRing;
-                const P2GParticle r = p2g_particle(p, s_ring[sl][0][lane], s_ring[sl][1][lane], s_ring[sl][2][lane],
-                                                   s_ring[sl][3][lane], s_ring[sl][4][lane], s_ring[sl][5][lane]);
-                if (r.bx != bx || r.by != by || r.bz != bz) {
-                    atomicOr(status, kStatusBinning);
-                } else {
-                    p2g_stencil(r, [&](int k, int, int, int, float m, float mx, float my, float mz) {
-                        am[k] += m;
-                        ax[k] += mx;
-                        ay[k] += my;
-                        az[k] += mz;
-                    });
+            for (int s = 0; s < maxc; ++s) {
+                if (s + kRing - 1 < cnt) fetch(s + kRing - 1);
+                cp_async_commit();
+                cp_async_wait<kRing - 1>();
+                __syncwarp();
+                if (s < cnt) {
+                    const int sl = s % kRing;
+                    const P2GParticle r = p2g_particle(p, s_ring[sl][0][lane], s_ring[sl][1][lane], s_ring[sl][2][lane],
+                                                       s_ring[sl][3][lane], s_ring[sl][4][lane], s_ring[sl][5][lane]);
+                    // Filed under this lane's cell by construction; a mismatch
+                    // is recorded, never scattered to a wrong node.
+                    if (r.bx - ox != tx || r.by - oy != ty || r.bz - oz != tz) {
+                        atomicOr(status, kStatusBinning);
+                    } else {
+                        p2g_stencil(r, [&](int k, int, int, int, float m, float mx, float my, float mz) {
+                            am[k] += m;
+                            ax[k] += mx;
+                            ay[k] += my;
+                            az[k] += mz;
+                        });
+                    }
+                }
+                __syncwarp();
+            }
+            cp_async_wait<0>();
+            if (packed) {
+                // One cell on all lanes: a butterfly reduce-scatter (five
+                // shuffle steps, each halving the 128 padded sums) leaves
+                // node l's totals on lane l.
+                float v[128];
+#pragma unroll
+                for (int k = 0; k < 32; ++k) {
+                    v[4 * k + 0] = k < 27 ? am[k < 27 ? k : 0] : 0.f;
+                    v[4 * k + 1] = k < 27 ? ax[k < 27 ? k : 0] : 0.f;
+                    v[4 * k + 2] = k < 27 ? ay[k < 27 ? k : 0] : 0.f;
+                    v[4 * k + 3] = k < 27 ? az[k < 27 ? k : 0] : 0.f;
+                }
+#pragma unroll
+                for (int d = 16, h = 64; d >= 1; d >>= 1, h >>= 1) {
+                    const bool upper = (lane & d) != 0;
+#pragma unroll
+                    for (int i = 0; i < h; ++i) {
+                        const float send = upper ? v[i] : v[i + h];
+                        const float keep = upper ? v[i + h] : v[i];
+                        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
+                    }
+                }
+                if (lane < 27) {
+                    const int x = ox + tx + lane % 3, y = oy + ty + (lane / 3) % 3, z = oz + tz + lane / 9;
+                    if (node_in_grid(p, x, y, z) && (v[0] != 0.f || v[1] != 0.f || v[2] != 0.f || v[3] != 0.f))
+                        red_add_v4(accum + node_index(p, x, y, z), v[0], v[1], v[2], v[3]);
+                }
+            } else {
+                // One lane per cell: distinct nodes for each stencil offset.
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+#pragma unroll
+                    for (int b = 0; b < 3; ++b)
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) {
+                            const int k = (c * 3 + b) * 3 + a;
+                            float4* d = &s_foot[((tz + c) * kTY + ty + b) * kTX + tx + a];
+                            __syncwarp();
+                            if (cnt > 0) {
+                                float4 v = *d;
+                                v.x += am[k];
+                                v.y += ax[k];
+                                v.z += ay[k];
+                                v.w += az[k];
+                                *d = v;
+                            }
+                        }
+                __syncwarp();
+                // The z-planes the group's cells reach: zmin .. zmax + 2.
+                const int zmin = (int)__reduce_min_sync(0xffffffffu, cnt > 0 ? (unsigned)tz : 0xFFu);
+                const int zmax = (int)__reduce_max_sync(0xffffffffu, cnt > 0 ? (unsigned)tz : 0u);
+                for (int q = zmin * kFootPlane + lane; q < (zmax + 3) * kFootPlane; q += 32) {
+                    const int x = ox + q % kTX, y = oy + (q / kTX) % kTY, z = oz + q / kFootPlane;
+                    const float4 v = s_foot[q];
+                    s_foot[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (node_in_grid(p, x, y, z) && (v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f))  // NaN counts
+                        red_add_v4(accum + node_index(p, x, y, z), v.x, v.y, v.z, v.w);
                 }
             }
             __syncwarp();
         }
-        cp_async_wait<0>();
-        __syncwarp();
-        float v[128];
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-            v[4 * k + 0] = k < 27 ? am[k < 27 ? k : 0] : 0.f;
-            v[4 * k + 1] = k < 27 ? ax[k < 27 ? k : 0] : 0.f;
-            v[4 * k + 2] = k < 27 ? ay[k < 27 ? k : 0] : 0.f;
-            v[4 * k + 3] = k < 27 ? az[k < 27 ? k : 0] : 0.f;
-        }
-#pragma unroll
-        for (int d = 16, h = 64; d >= 1; d >>= 1, h >>= 1) {
-            const bool upper = (lane & d) != 0;
-#pragma unroll
-            for (int i = 0; i < h; ++i) {
-                const float send = upper ? v[i] : v[i + h];
-                const float keep = upper ? v[i + h] : v[i];
-                v[i] = keep + __shfl_xor_sync(0xffffffffu, send, d);
-            }
-        }
-        if (lane < 27) {
-            const int x = bx + lane % 3, y = by + (lane / 3) % 3, z = bz + lane / 9;
-            if (node_in_grid(p, x, y, z) && (v[0] != 0.f || v[1] != 0.f || v[2] != 0.f || v[3] != 0.f))
-                red_add_v4(accum_all + p.goff + node_index(p, x, y, z), v[0], v[1], v[2], v[3]);
-        }
-        __syncwarp();
+        unsigned next = 0u;
+        if (lane == 0) next = gridDim.x + atomicAdd(ctl.work, 1u);
+        unit = (int)__shfl_sync(0xffffffffu, next, 0);
     }
 }
 
@@ -553,41 +457,34 @@ __global__ void __launch_bounds__(256) bin_count_kernel(SceneTable sc, long long
     const long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const bool valid = j < n;
     int gcell = -1, gbin = -1, bin = -1, scene = 0;
-    long long boff = 0;
     if (valid) {
         scene = scene_of(sc.poff, sc.count, j);
-        const SimParams p = sc.prm[scene];
+        const SimParams& p = sc.prm[scene];
         const float4 q = __ldg(reinterpret_cast<const float4*>(P + (size_t)j * kAFloats));
-        const int cell = cell_of(p, q.x, q.y, q.z, &bin);
-        gcell = (int)p.coff + cell;
+        gcell = (int)p.coff + cell_of(p, q.x, q.y, q.z, &bin);
         gbin = (int)p.boff + bin;
-        boff = p.boff;
     }
-    file_particle(gcell, gbin, bin, scene, boff, set);
+    file_particle(gcell, gbin, bin, scene, set);
     if (valid) pcell[j] = gcell;
 }
 
-// Bin starts in two launches over (scene, chunk of kScanChunk bins) CTAs, no
-// CTA waiting on another: bin_sum_kernel writes each chunk's count sum to
-// bpart[scene * chunks + chunk]; bin_scan_kernel adds the sums of the
-// scene's earlier chunks to poff and scans its own chunk, so that
-// bstart[i] = poff + sum of bcount[0..i) over the scene's nbins = nb + 1
-// bins and bstart[nbins] = poff + its particle count (global slots).  The
-// scan also zeroes the chunk's bin counters of the other set, and CTA (0, 0)
-// the P2G and G2P work counters and writes the per-scene prefixes of the
-// listed bins (itemoff, in P2G items, for the current set; clroff for the set
-// to clear).  Per chunk: coalesced loads into shared
-// memory, a contiguous run of kScanPer counters per thread, a block scan of
-// the run sums, coalesced stores.
-constexpr int kScanThreads = 256;
+// Bin starts, over (scene, chunk of kScanChunk bins) CTAs, no CTA waiting on
+// another: bstart[i] = poff + sum of bcount[0..i) over the scene's nb + 1
+// bins (global slots).  Up to kScanDirect chunks a CTA adds up the counts of
+// all earlier chunks itself and scans its own; scenes of more get a launch
+// before it, in which bin_sum_kernel writes each chunk's sum to bpart[scene *
+// chunks + chunk].  Measured, one launch against two: 2.1 / 4.0 us at 32^3
+// (405 bins), 4.6 / 5.4 at 97 x 61 x 83 (4,368 bins), 6.2 / 5.8 at 128^3
+// (18,513 bins), 21.4 / 5.9 at 256^3 (141,570 bins).
+constexpr int kScanThreads = 512;
 constexpr int kScanWarps = kScanThreads / 32;
-constexpr int kScanPer = 8;
+constexpr int kScanPer = 4;
 constexpr int kScanChunk = kScanThreads * kScanPer;
+constexpr int kScanDirect = 4;
 
 // Sum of v over the CTA, returned to every thread (s_red: kScanWarps ints).
 __device__ __forceinline__ int scan_block_sum(int v, int* s_red) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    v = (int)__reduce_add_sync(0xffffffffu, (unsigned)v);
     if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
     __syncthreads();
     int total = 0;
@@ -617,56 +514,33 @@ __global__ void __launch_bounds__(kScanThreads) bin_sum_kernel(SceneTable sc, co
 }
 
 __global__ void __launch_bounds__(kScanThreads) bin_scan_kernel(SceneTable sc, const uint32_t* __restrict__ bcount_all,
-                                                                uint32_t* __restrict__ bclear_all,
                                                                 const int32_t* __restrict__ bpart,
-                                                                int32_t* __restrict__ bstart_all,
-                                                                uint32_t* __restrict__ work,
-                                                                const uint32_t* __restrict__ cur_nlist,
-                                                                const uint32_t* __restrict__ clear_nlist,
-                                                                long long* __restrict__ itemoff,
-                                                                long long* __restrict__ clroff,
-                                                                uint32_t* __restrict__ tstamp) {
+                                                                int32_t* __restrict__ bstart_all) {
     pdl_wait();
     __shared__ int s_val[kScanChunk];
     __shared__ int s_red[kScanWarps];
     __shared__ int s_warp[kScanWarps];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int scene = blockIdx.x, chunk = blockIdx.y;
-    if (scene == 0 && chunk == 0 && t == 0) {
-        work[0] = 0u;  // P2G items
-        work[1] = 0u;  // G2P items
-        work[2] = 0u;  // crowded-cell list length
-        work[3] = 0u;  // crowded-cell entries taken
-        if (tstamp) *tstamp += 1u;  // this ordering's tile stamp
-        // Per-scene prefixes: P2G items (kBinZ per listed bin of the current
-        // set) and the listed bins of the set to clear.
-        long long run = 0, runc = 0;
-        for (int s2 = 0; s2 < sc.count; ++s2) {
-            itemoff[s2] = run;
-            clroff[s2] = runc;
-            run += (long long)cur_nlist[s2] * kBinZ;
-            runc += (long long)clear_nlist[s2];
-        }
-        itemoff[sc.count] = run;
-        clroff[sc.count] = runc;
-    }
     const SimParams& p = sc.prm[scene];
     const int nbins = p.nb + 1;
     const int c0 = chunk * kScanChunk;
     if (c0 >= nbins) return;
-    const long long boff = p.boff;
-    const uint32_t* bcount = bcount_all + boff + c0;
-    uint32_t* bclear = bclear_all + boff + c0;
-    int32_t* bstart = bstart_all + boff + c0;
+    const uint32_t* bcount = bcount_all + p.boff;
+    int32_t* bstart = bstart_all + p.boff + c0;
     const int m = min(kScanChunk, nbins - c0);
     // Particles of the scene's earlier chunks.
     int pre = 0;
-    for (int i = t; i < chunk; i += kScanThreads) pre += bpart[(long long)scene * gridDim.y + i];
+    if (bpart) {
+        for (int i = t; i < chunk; i += kScanThreads) pre += bpart[(long long)scene * gridDim.y + i];
+    } else {
+#pragma unroll 16
+        for (int i = t; i < c0; i += kScanThreads) pre += (int)__ldg(bcount + i);
+    }
 #pragma unroll
     for (int k = 0; k < kScanPer; ++k) {
         const int i = k * kScanThreads + t;
-        s_val[i] = i < m ? (int)bcount[i] : 0;
-        if (i < m) bclear[i] = 0u;
+        s_val[i] = i < m ? (int)__ldg(bcount + c0 + i) : 0;
     }
     const int carry = (int)p.poff + scan_block_sum(pre, s_red);  // its barrier also publishes s_val
     int v[kScanPer], sum = 0;
@@ -683,14 +557,9 @@ __global__ void __launch_bounds__(kScanThreads) bin_scan_kernel(SceneTable sc, c
     }
     if (lane == 31) s_warp[warp] = incl;
     __syncthreads();
-    int before = 0, total = 0;
+    int run = carry + incl - sum;
 #pragma unroll
-    for (int w = 0; w < kScanWarps; ++w) {
-        const int x = s_warp[w];
-        before += w < warp ? x : 0;
-        total += x;
-    }
-    int run = carry + before + incl - sum;
+    for (int w = 0; w < kScanWarps; ++w) run += w < warp ? s_warp[w] : 0;
 #pragma unroll
     for (int k = 0; k < kScanPer; ++k) {
         s_val[t * kScanPer + k] = run;
@@ -702,19 +571,18 @@ __global__ void __launch_bounds__(kScanThreads) bin_scan_kernel(SceneTable sc, c
         const int i = k * kScanThreads + t;
         if (i < m) bstart[i] = s_val[i];
     }
-    if (t == 0 && c0 + m == nbins) bstart[m] = carry + total;
 }
 
 // The P2G order of a bin's cells (one warp; lane holds the counts of cells
 // 4 lane .. 4 lane + 3): occupied cells by count class (floor(log2 count),
 // 7 for 128 and more), largest class first, by cell index within a class;
-// order[p] = the cell at position p, 0xFF past the occupied cells.  P2G's
-// item g of the bin takes positions 32 g .. 32 g + 31, so a warp's lanes hold
-// cells of similar counts.  Class counts travel as the bytes of two words
+// order[p] = the cell at position p, for the occupied cells, whose number is
+// returned.  P2G's item g of the bin takes positions 32 g .. 32 g + 31, so a
+// warp's lanes hold cells of similar counts.  Class counts travel as the bytes of two words
 // (classes 0..3 and 4..7; a byte holds at most 128): one warp scan gives the
 // cells of each class in lower lanes, and multiplying the totals by
 // 0x01010101 gives byte-wise running sums, hence each class's first position.
-__device__ __forceinline__ void cell_order(uint4 c, uint8_t* __restrict__ order) {
+__device__ __forceinline__ int cell_order(uint4 c, uint8_t* __restrict__ order) {
     const int lane = threadIdx.x & 31;
     const uint32_t cnt[4] = {c.x, c.y, c.z, c.w};
     int cls[4];
@@ -748,36 +616,45 @@ __device__ __forceinline__ void cell_order(uint4 c, uint8_t* __restrict__ order)
         if (h) seen_hi += 1u << sh;
         else seen_lo += 1u << sh;
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-        if (4 * lane + j >= total) order[4 * lane + j] = 0xFFu;
+    return total;
 }
 
-// One warp per listed bin of each scene: cstart of its 128 cells = bstart of
-// the bin + the exclusive scan of their counts (also written to ccur, the
-// cursors the scatter draws slots from).  Then clears the cell
-// counters of the other set for the bins on that set's lists (the cells it
-// last filled).
-__global__ void __launch_bounds__(128) cell_scan_kernel(SceneTable sc, BinSet set, const int32_t* __restrict__ bstart,
-                                                        int32_t* __restrict__ cstart, int32_t* __restrict__ ccur,
-                                                        uint8_t* __restrict__ corder,
-                                                        BinSet clear, const long long* __restrict__ itemoff,
-                                                        const long long* __restrict__ clroff,
-                                                        const uint32_t* __restrict__ tstamp,
-                                                        uint32_t* __restrict__ tmark) {
+// A warp per listed bin: the bin's 128 cells follow one another from the
+// bin's start; ccur receives every cell's first slot (the cursors the scatter
+// draws from).
+//
+// The warp also lays out P2G's work: desc[p] = (first slot, particles << 8 |
+// cell) of the cell at position p of the bin's order, particles capped per
+// item of 32 positions (item_cap); the rest of a crowded cell goes to the
+// crowded-cell list in chunks of kCrowdChunk particles.  Building the list
+// here instead of inside P2G puts it in front of P2G's own work counter, so
+// that one launch serves both (the second launch cost 4.2 us per substep at
+// 8k particles, 10.7 us at 2M).
+//
+// Then the cells and bins that the other set last filled are cleared.
+constexpr int kCellWarps = 8;
+
+__global__ void __launch_bounds__(kCellWarps * 32) cell_scan_kernel(SceneTable sc, BinSet set, BinSet clear,
+                                                                 OrderCtl ctl, const int32_t* __restrict__ bstart,
+                                                                 int32_t* __restrict__ ccur,
+                                                                 int2* __restrict__ desc, int4* __restrict__ crowd,
+                                                                 int crowd_cap, int cap,
+                                                                 const uint32_t* __restrict__ tstamp,
+                                                                 uint32_t* __restrict__ tmark,
+                                                                 uint32_t* __restrict__ status) {
     pdl_wait();
-    const int lane = threadIdx.x & 31;
-    const uint32_t stamp = tmark ? *tstamp : 0u;
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    // Listed bins of all scenes, one after another (itemoff counts kBinZ items per bin).
-    const long long nbins = itemoff[sc.count] / kBinZ;
-    for (long long it = gw; it < nbins; it += nw) {
-        const int scene = sc.count == 1 ? 0 : scene_of(itemoff, sc.count, it * kBinZ);
-        const long long coff = sc.prm[scene].coff, boff = sc.prm[scene].boff;
-        const int bin = set.blist[boff + it - itemoff[scene] / kBinZ];
-        const size_t c0 = (size_t)coff + (size_t)bin * kBinCells + lane * 4;
-        const uint4 c = *reinterpret_cast<const uint4*>(set.ccount + c0);
+    __shared__ int s_count[kCellWarps][kBinCells];
+    __shared__ int s_start[kCellWarps][kBinCells];
+    __shared__ uint8_t s_order[kCellWarps][kBinCells];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t stamp = tmark ? *tstamp + 1u : 0u;  // this ordering's: the scatter stores it
+    const int nbins = (int)*set.nlist;
+    for (int it = blockIdx.x * kCellWarps + warp; it < nbins; it += gridDim.x * kCellWarps) {
+        const int2 e = set.blist[it];
+        const SimParams& p = sc.prm[sc.count == 1 ? 0 : e.x];
+        const size_t c0 = (size_t)p.coff + (size_t)e.y * kBinCells;
+        const uint4 c = reinterpret_cast<const uint4*>(set.ccount + c0)[lane];
+        const int first = bstart[p.boff + e.y];
         const int sum = (int)(c.x + c.y + c.z + c.w);
         int incl = sum;
 #pragma unroll
@@ -785,31 +662,53 @@ __global__ void __launch_bounds__(128) cell_scan_kernel(SceneTable sc, BinSet se
             const int y = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += y;
         }
-        const int e0 = bstart[boff + bin] + incl - sum;
         int4 st;
-        st.x = e0;
-        st.y = e0 + (int)c.x;
+        st.x = first + incl - sum;
+        st.y = st.x + (int)c.x;
         st.z = st.y + (int)c.y;
         st.w = st.z + (int)c.z;
-        *reinterpret_cast<int4*>(cstart + c0) = st;
-        *reinterpret_cast<int4*>(ccur + c0) = st;  // the scatter's cursors start at the cells' first slots
-        cell_order(c, corder + (size_t)coff + (size_t)bin * kBinCells);
-        // The grid-update tiles this bin's particles reach: tiles bin + (dx,
-        // dy, dz), d in {0, 1}^3, lane d.
-        const SimParams& ps = sc.prm[scene];
-        if (tmark && lane < 8 && bin < ps.nb) {
-            const int tx = bin % ps.nbx + (lane & 1), ty = (bin / ps.nbx) % ps.nby + ((lane >> 1) & 1),
-                      tz = bin / (ps.nbx * ps.nby) + (lane >> 2);
-            if (tx < ps.nbx && ty < ps.nby && tz < ps.nbz) tmark[boff + ((long long)tz * ps.nby + ty) * ps.nbx + tx] = stamp;
+        reinterpret_cast<int4*>(ccur + c0)[lane] = st;
+        if (e.y < p.nb) {  // the overflow bin reaches no node: nothing for P2G
+            reinterpret_cast<uint4*>(s_count[warp])[lane] = c;
+            reinterpret_cast<int4*>(s_start[warp])[lane] = st;
+            const int occupied = cell_order(c, s_order[warp]);
+            __syncwarp();
+#pragma unroll
+            for (int g = 0; g < kBinZ; ++g) {
+                const int pos = g * 32 + lane;
+                const bool own = pos < occupied;
+                const int cell = own ? s_order[warp][pos] : 0;
+                const int full = own ? s_count[warp][cell] : 0;
+                const int slot = s_start[warp][cell];
+                int icap = cap;
+                if (cap <= 0 && g * 32 < occupied) icap = item_cap(full);
+                for (int off = icap; off < full; off += kCrowdChunk) {
+                    const uint32_t q = atomicAdd(ctl.crowded, 1u);
+                    if (q < (uint32_t)crowd_cap)
+                        crowd[q] = make_int4(e.x, e.y * kBinCells + cell, slot + off, min(kCrowdChunk, full - off));
+                    else
+                        atomicOr(status, kStatusCrowdList);
+                }
+                desc[c0 + pos] = make_int2(slot, min(full, icap) << 8 | cell);
+            }
+            // The grid-update tiles this bin's particles reach: tiles bin +
+            // (dx, dy, dz), d in {0, 1}^3, lane d.
+            if (tmark && lane < 8) {
+                const int tx = e.y % p.nbx + (lane & 1), ty = (e.y / p.nbx) % p.nby + ((lane >> 1) & 1),
+                          tz = e.y / (p.nbx * p.nby) + (lane >> 2);
+                if (tx < p.nbx && ty < p.nby && tz < p.nbz)
+                    tmark[p.boff + ((long long)tz * p.nby + ty) * p.nbx + tx] = stamp;
+            }
+            __syncwarp();  // the next pass rewrites the warp's shared rows
         }
     }
-    const long long nclear = clroff[sc.count];
-    for (long long it = gw; it < nclear; it += nw) {
-        const int scene = sc.count == 1 ? 0 : scene_of(clroff, sc.count, it);
-        const long long coff = sc.prm[scene].coff, boff = sc.prm[scene].boff;
-        const int bin = clear.blist[boff + it - clroff[scene]];
-        *reinterpret_cast<uint4*>(clear.ccount + (size_t)coff + (size_t)bin * kBinCells + lane * 4) =
+    const int nclear = (int)*clear.nlist;
+    for (int it = blockIdx.x * kCellWarps + warp; it < nclear; it += gridDim.x * kCellWarps) {
+        const int2 e = clear.blist[it];
+        const SimParams& p = sc.prm[sc.count == 1 ? 0 : e.x];
+        reinterpret_cast<uint4*>(clear.ccount + (size_t)p.coff + (size_t)e.y * kBinCells)[lane] =
             make_uint4(0u, 0u, 0u, 0u);
+        if (lane == 0) clear.bcount[p.boff + e.y] = 0u;
     }
 }
 
@@ -818,17 +717,22 @@ __global__ void __launch_bounds__(128) cell_scan_kernel(SceneTable sc, BinSet se
 // the lanes sharing a cell take consecutive slots in lane order).  A thread
 // files kScatterPer particles (block b: particles b * kScatterPer * blockDim
 // .. + kScatterPer * blockDim, one blockDim-wide slice per pass), so that the
-// cursor atomics of its passes are in flight together.  Thread 0 also resets
-// the other set's lists, which cell_scan_kernel has just cleared.
+// cursor atomics of its passes are in flight together.  The first block also
+// resets the other set's list, which the cell scan has used up, and P2G's work
+// counter, and advances the tile stamp.
 constexpr int kScatterPer = 4;
 
-__global__ void __launch_bounds__(256) bin_scatter_kernel(long long n, int scenes, const int32_t* __restrict__ pcell,
+__global__ void __launch_bounds__(256) bin_scatter_kernel(long long n, const int32_t* __restrict__ pcell,
                                                           int32_t* __restrict__ ccur, int32_t* __restrict__ gidx,
-                                                          uint32_t* __restrict__ clear_nlist) {
+                                                          OrderCtl ctl, uint32_t* __restrict__ clear_nlist,
+                                                          uint32_t* __restrict__ tstamp) {
     pdl_wait();
     const long long j0 = blockIdx.x * (long long)blockDim.x * kScatterPer + threadIdx.x;
-    if (j0 == 0)
-        for (int s2 = 0; s2 < scenes; ++s2) clear_nlist[s2] = 0u;
+    if (j0 == 0) {
+        *clear_nlist = 0u;
+        *ctl.work = 0u;
+        if (tstamp) *tstamp += 1u;
+    }
     const int lane = threadIdx.x & 31;
     int cell[kScatterPer], base[kScatterPer];
     uint32_t peers[kScatterPer];
@@ -1013,8 +917,10 @@ __global__ void __launch_bounds__(256, kWide ? 1 : (kMode == 1 ? 2 : ((kBatch ||
                                                   const int32_t* __restrict__ sig_in, int32_t* __restrict__ sig_out,
                                                   const float4* __restrict__ vgrid_all, const float* __restrict__ sdf_all,
                                                   int32_t* __restrict__ pcell, BinSet next,
-                                                  uint32_t* __restrict__ health, LearnArgs la) {
+                                                  uint32_t* __restrict__ crowded, uint32_t* __restrict__ health,
+                                                  LearnArgs la) {
     pdl_wait();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *crowded = 0u;  // P2G has taken its crowded-cell list
     __shared__ SimParams s_prm[kBatch ? kTableScenes : 1];
     __shared__ long long s_first[kBatch ? kTableScenes + 1 : 1];
     __shared__ int s_range[2];
@@ -1321,7 +1227,7 @@ __global__ void __launch_bounds__(256, kWide ? 1 : (kMode == 1 ? 2 : ((kBatch ||
         gcell = (int)p.coff + cell_of(p, nx, ny, nz, &bin);
         gbin = (int)p.boff + bin;
     }
-    file_particle(gcell, gbin, bin, scene, p.boff, next);
+    file_particle(gcell, gbin, bin, scene, next);
     if (!valid) continue;  // only the last passes of the last block have idle lanes
     float4* o = reinterpret_cast<float4*>(Pout + (size_t)j * kAFloats);
     {
@@ -1513,19 +1419,20 @@ int launch_bin_count(const SceneTable& sc, long long n, const float* P, int32_t*
 int bin_scan_chunks(long long bins) { return (int)std::max(1LL, (bins + kScanChunk - 1) / kScanChunk); }
 
 int launch_bin_order(const SceneTable& sc, long long n, long long bins_total, const BinSet& cur, const BinSet& other,
-                     int32_t* bstart, int32_t* cstart, const int32_t* pcell, int32_t* ccur, int32_t* gidx,
-                     uint8_t* corder, long long* itemoff, long long* clroff, uint32_t* work, int32_t* bpart,
-                     int scan_chunks, const TileMarks& tiles, cudaStream_t st) {
+                     const OrderCtl& ctl, int32_t* bstart, int32_t* bpart, int scan_chunks, const int32_t* pcell,
+                     int32_t* ccur, int32_t* gidx, int2* desc, int4* crowd, int crowd_cap, int cell_cap,
+                     const TileMarks& tiles, uint32_t* status, cudaStream_t st) {
     if (n <= 0) return 0;
     const dim3 scan_grid((unsigned)sc.count, (unsigned)scan_chunks);
-    launch_dep(bin_sum_kernel, scan_grid, kScanThreads, 0, st, sc, cur.bcount, bpart);
-    launch_dep(bin_scan_kernel, scan_grid, kScanThreads, 0, st, sc, cur.bcount, other.bcount, bpart, bstart, work, cur.nlist,
-                                                       other.nlist, itemoff, clroff, tiles.stamp);
-    const int ctas = (int)std::max(1LL, std::min((long long)blocks_for(bins_total * 32, 128), 148LL * 8));
-    launch_dep(cell_scan_kernel, ctas, 128, 0, st, sc, cur, bstart, cstart, ccur, corder, other, itemoff, clroff,
-               tiles.stamp, tiles.mark);
-    launch_dep(bin_scatter_kernel, blocks_for(n, 256 * kScatterPer), 256, 0, st, n, sc.count, pcell, ccur, gidx, other.nlist);
-    return 4;
+    const bool summed = scan_chunks > kScanDirect;
+    if (summed) launch_dep(bin_sum_kernel, scan_grid, kScanThreads, 0, st, sc, cur.bcount, bpart);
+    launch_dep(bin_scan_kernel, scan_grid, kScanThreads, 0, st, sc, cur.bcount, summed ? bpart : nullptr, bstart);
+    const int ctas = (int)std::max(1LL, std::min((long long)blocks_for(bins_total, kCellWarps), 148LL * 4));
+    launch_dep(cell_scan_kernel, ctas, kCellWarps * 32, 0, st, sc, cur, other, ctl, bstart, ccur, desc, crowd,
+               crowd_cap, std::max(cell_cap, 0), tiles.stamp, tiles.mark, status);
+    launch_dep(bin_scatter_kernel, blocks_for(n, 256 * kScatterPer), 256, 0, st, n, pcell, ccur, gidx, ctl,
+               other.nlist, tiles.stamp);
+    return summed ? 4 : 3;
 }
 
 int p2g_max_ctas_per_sm() {
@@ -1538,17 +1445,13 @@ int p2g_max_ctas_per_sm() {
 }
 
 int launch_p2g(const SceneTable& sc, long long n, long long bins_total, const float* P, const int32_t* gidx,
-               const int32_t* cstart, const BinSet& cur, const uint8_t* corder, const long long* itemoff,
-               uint32_t* work, float4* accum, int4* crowd, int crowd_cap, uint32_t* status, cudaStream_t st,
-               int ctas_per_sm, int cell_cap) {
+               const BinSet& cur, const int2* desc, const int4* crowd, int crowd_cap, const OrderCtl& ctl,
+               float4* accum, uint32_t* status, cudaStream_t st, int ctas_per_sm) {
     if (n <= 0) return 0;
     const int per_sm = ctas_per_sm > 0 ? ctas_per_sm : kP2GWarpsPerSM;
-    const int cap = cell_cap > 0 ? cell_cap : 0;
     const int warps = (int)std::min(bins_total * kBinZ, 148LL * per_sm);
-    launch_dep(p2g_kernel, warps, 32, 0, st, sc, P, gidx, cstart, cur, corder, itemoff, work, accum, crowd, crowd_cap, status,
-                                     cap);
-    launch_dep(p2g_crowd_kernel, 148 * kP2GWarpsPerSM, 32, 0, st, sc, P, gidx, crowd, crowd_cap, work, accum, status);
-    return 2;
+    launch_dep(p2g_kernel, warps, 32, 0, st, sc, P, gidx, cur, desc, crowd, crowd_cap, ctl, accum, status);
+    return 1;
 }
 
 int launch_grid_update(const SceneTable& sc, const SimParams& p0, long long g_total, float4* accum, float4* vgrid,
@@ -1573,14 +1476,14 @@ int launch_grid_update(const SceneTable& sc, const SimParams& p0, long long g_to
 
 int launch_g2p(const SceneTable& sc, const SimParams& p0, long long n, const float* Pin, float* Pout,
                const int32_t* gidx, const int32_t* sig_in, int32_t* sig_out, const float4* vgrid, const float* sdf,
-               int32_t* pcell, const BinSet& next, uint32_t* health, cudaStream_t st,
+               int32_t* pcell, const BinSet& next, uint32_t* crowded, uint32_t* health, cudaStream_t st,
                const LearnArgs* learn, int block) {
     if (n <= 0) return 0;
     const LearnArgs la = learn ? *learn : LearnArgs{};
     const unsigned grid = blocks_for(n, 256);
     if (learn && sc.count == 1 && la.mlp_tc) {
         launch_dep(g2p_kernel<false, kG2PLearnedTc>, grid, 256, sizeof(MlpTcSmem), st,
-            sc, p0, n, Pin, Pout, gidx, sig_in, sig_out, vgrid, sdf, pcell, next, health, la);
+            sc, p0, n, Pin, Pout, gidx, sig_in, sig_out, vgrid, sdf, pcell, next, crowded, health, la);
         return 1;
     }
     // Plain G2P: 128- or 256-thread CTAs, or 512 = the register-wide 256-thread
@@ -1589,28 +1492,26 @@ int launch_g2p(const SceneTable& sc, const SimParams& p0, long long n, const flo
     const int pb = wide ? 256 : ((block == 128 || block == 256) ? block : 256);
     if (learn && sc.count == 1 && la.mlp)
         launch_dep(g2p_kernel<false, kG2PLearned>, grid, 256, 0, st, sc, p0, n, Pin, Pout, gidx, sig_in, sig_out, vgrid, sdf,
-                                                             pcell, next, health, la);
+                                                             pcell, next, crowded, health, la);
     else if (learn && sc.count == 1 && la.feat)
         launch_dep(g2p_kernel<false, kG2PCollect>, grid, 256, 0, st, sc, p0, n, Pin, Pout, gidx, sig_in, sig_out, vgrid, sdf,
-                                                             pcell, next, health, la);
+                                                             pcell, next, crowded, health, la);
     else if (learn && sc.count == 1)
         launch_dep(g2p_kernel<false, kG2PLarge>, grid, 256, 0, st, sc, p0, n, Pin, Pout, gidx, sig_in, sig_out, vgrid, sdf,
-                                                           pcell, next, health, la);
+                                                           pcell, next, crowded, health, la);
     else if (sc.count == 1 && wide)
         launch_dep(g2p_kernel<false, kG2PPlain, true>, blocks_for(n, pb), pb, 0, st, sc, p0, n, Pin, Pout, gidx, sig_in,
-                                                                             sig_out, vgrid, sdf, pcell, next,
-                                                                             health, la);
+                                                                             sig_out, vgrid, sdf, pcell, next, crowded, health, la);
     else if (sc.count == 1)
         launch_dep(g2p_kernel<false, kG2PPlain>, blocks_for(n, pb), pb, 0, st, sc, p0, n, Pin, Pout, gidx, sig_in, sig_out,
-                                                                       vgrid, sdf, pcell, next, health, la);
+                                                                       vgrid, sdf, pcell, next, crowded, health, la);
     else if (wide)
         launch_dep(g2p_kernel<true, kG2PPlain, true>, blocks_for(n, pb), pb, 0, st, sc, p0, n, Pin, Pout, gidx, sig_in,
-                                                                            sig_out, vgrid, sdf, pcell, next,
-                                                                            health, la);
+                                                                            sig_out, vgrid, sdf, pcell, next, crowded, health, la);
     else {
         constexpr int k = g2p_per_thread(true, kG2PPlain, false);
         launch_dep(g2p_kernel<true, kG2PPlain>, blocks_for(n, (long long)pb * k), pb, k * 3 * pb * sizeof(float4), st,
-            sc, p0, n, Pin, Pout, gidx, sig_in, sig_out, vgrid, sdf, pcell, next, health, la);
+            sc, p0, n, Pin, Pout, gidx, sig_in, sig_out, vgrid, sdf, pcell, next, crowded, health, la);
     }
     return 1;
 }
