@@ -547,8 +547,7 @@ mpm_status mpm_triangles_normalize(float* triangles9_host, int64_t* t, float nor
  * up to the order of float sums. */
 typedef struct mpm_tuning {
     int32_t p2g_ctas_per_sm;  /* 1 .. the most that fit (default 12) */
-    int32_t g2p_block;        /* 128 or 256 (default 256); 512 = 256-thread CTAs free to use up to
-                               * 255 registers (more loads in flight, fewer warps) */
+    int32_t g2p_block;        /* 128 (default) or 256: threads per CTA; 512 runs as 256 */
     int32_t grid_block;       /* 128 or 256: the update visits every node in CTAs of that size;
                                * 0: only the node tiles this substep's particles reach, plus a
                                * reset of tiles they left (default for one scene of 2^23 nodes

@@ -49,6 +49,7 @@ struct SimParams {
     long long goff;       // first grid node
     long long coff;       // first cell: (nb + 1) * kBinCells cells per scene
     long long boff;       // first bin entry: nb + 2 entries per scene
+    unsigned long long inv_nbx, inv_nby;  // 2^48 / nbx and nby, rounded up: bin / nbx = bin * inv_nbx >> 48
 };
 
 // The scenes of an engine on the device: prm[s], and the prefix arrays
@@ -139,6 +140,19 @@ __device__ __forceinline__ int cell_of(const SimParams& p, float x, float y, flo
     const int b = ((uz / kBinZ) * p.nby + uy / kBinY) * p.nbx + ux / kBinX;
     *bin = b;
     return b * kBinCells + ((uz % kBinZ) * kBinY + uy % kBinY) * kBinX + ux % kBinX;
+}
+
+// Node (0, 0, 0) of the stencil of the bin's first cell.  Bins number below
+// 2^24 (cells below 2^31), so the products stay below 2^64 and the quotients
+// by the reciprocals rounded up are exact: with m = (2^48 + e) / d, 0 <= e < d,
+// n m / 2^48 exceeds n / d by n e / (d 2^48) < 2^-24, less than the 1 / d it
+// would take to reach the next whole number.
+__device__ __forceinline__ void bin_origin(const SimParams& p, int bin, int* x, int* y, int* z) {
+    const int row = (int)((unsigned long long)bin * p.inv_nbx >> 48);
+    const int slab = (int)((unsigned long long)row * p.inv_nby >> 48);
+    *x = (bin - row * p.nbx) * kBinX - 2;
+    *y = (row - slab * p.nby) * kBinY - 2;
+    *z = slab * kBinZ - 2;
 }
 
 __device__ __forceinline__ float det3(const float* A) {

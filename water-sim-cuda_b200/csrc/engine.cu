@@ -80,6 +80,7 @@ struct mpm_engine {
     float* P[2] = {nullptr, nullptr};        // particle-major state, 24 floats per particle
     int32_t* sigma[2] = {nullptr, nullptr};  // slot -> original slot (global)
     int32_t* gidx = nullptr;                 // new slot -> old slot of the current binning
+    int2* edge = nullptr;                    // cells of the first and last of every kEdgeSlots slots
     int4* crowd = nullptr;                   // P2G's crowded-cell list
     int crowd_cap = 0;
     int32_t* pcell = nullptr;                // global cell of each slot of P[parity]
@@ -178,7 +179,7 @@ struct mpm_engine {
     double last_stats[3] = {0.0, 0.0, 0.0};  // the three means of the last checked large step
 
     // Launch shapes of the substep (mpm_autotune / mpm_set_tuning).
-    mpm_tuning tune{12, 256, 256, 0.f, 0.f, 0.f, 0};
+    mpm_tuning tune{12, 128, 256, 0.f, 0.f, 0.f, 0};
 };
 
 namespace {
@@ -240,6 +241,7 @@ void free_particles(mpm_engine* e) {
         e->graph_kernels[k] = 0;
     }
     free_dev(e->gidx);
+    free_dev(e->edge);
     free_dev(e->crowd);
     free_dev(e->pcell);
     free_dev(e->ref_keys);
@@ -298,6 +300,7 @@ mpm_status alloc_particles(mpm_engine* e, long long n, int max_n, size_t sort_by
         CK(e, cudaMalloc(&e->sigma[k], ibytes));
     }
     CK(e, cudaMalloc(&e->gidx, ibytes));
+    CK(e, cudaMalloc(&e->edge, (cap + mpm::kEdgeSlots - 1) / mpm::kEdgeSlots * sizeof(int2)));
     // A crowded-cell entry holds at least one particle beyond a cap of 4 or
     // more (the smallest mpm_set_tuning accepts), and a cell yields one entry
     // per 256 of them: fewer than n / 4 entries.
@@ -367,7 +370,7 @@ mpm::TileMarks active_tiles(const mpm_engine* e) { return e->tune.grid_block == 
 // parameters of `sc`.
 int enqueue_order(mpm_engine* e, int par) {
     return mpm::launch_bin_order(e->table, e->n, e->bins_scan, e->bins[par], e->bins[1 - par], e->order, e->bstart,
-                                 e->bpart, e->scan_chunks, e->pcell, e->ccur, e->gidx, e->desc, e->crowd, e->crowd_cap,
+                                 e->bpart, e->scan_chunks, e->pcell, e->ccur, e->gidx, e->edge, e->desc, e->crowd, e->crowd_cap,
                                  e->tune.p2g_cell_cap, active_tiles(e), e->d_flags + 1, e->stream);
 }
 int enqueue_p2g(mpm_engine* e, const mpm::SceneTable& sc, int par) {
@@ -376,10 +379,10 @@ int enqueue_p2g(mpm_engine* e, const mpm::SceneTable& sc, int par) {
 }
 
 // A substep begun with mpm_substep_partial is given up: its ordering's
-// counters (OrderCtl) are zeroed for the next one.
+// counters (OrderCtl) and list are zeroed for the next one (it has cleared
+// the other set, whose list is empty).
 mpm_status abandon_partial(mpm_engine* e) {
-    if (e->partial_stage != 0)
-        CK(e, cudaMemsetAsync(e->order.work, 0, 2 * sizeof(uint32_t), e->stream));
+    if (e->partial_stage != 0) CK(e, cudaMemsetAsync(e->ctl, 0, kCtlBytes, e->stream));
     e->partial_stage = 0;
     return MPM_OK;
 }
@@ -405,7 +408,7 @@ int enqueue_substep(mpm_engine* e, int par, int from, int upto, const cudaEvent_
                                             e->tune.grid_block);
     mark(3);
     if (from <= MPM_STAGE_G2P && upto >= MPM_STAGE_G2P)
-        launches += mpm::launch_g2p(sc, e->prm[0], e->n, e->P[par], e->P[1 - par], e->gidx, e->sigma[par],
+        launches += mpm::launch_g2p(sc, e->prm[0], e->n, e->P[par], e->P[1 - par], e->gidx, e->edge, e->sigma[par],
                                     e->sigma[1 - par], e->vgrid, e->sdf, e->pcell, e->bins[1 - par],
                                     e->order.crowded, e->d_flags, st, nullptr, e->tune.g2p_block);
     mark(4);
@@ -687,6 +690,8 @@ mpm_status create_engine(const mpm_config* cfgs, int32_t count, int32_t device, 
         p.nby = (cfg->size_y + 2 + mpm::kBinY - 1) / mpm::kBinY;
         p.nbz = (cfg->size_z + 2 + mpm::kBinZ - 1) / mpm::kBinZ;
         p.nb = p.nbx * p.nby * p.nbz;
+        p.inv_nbx = ((1ull << 48) + p.nbx - 1) / p.nbx;
+        p.inv_nby = ((1ull << 48) + p.nby - 1) / p.nby;
         p.poff = 0;
         p.goff = g_total;
         p.coff = cells_total;
@@ -851,7 +856,7 @@ int enqueue_large(mpm_engine* e, int par, const mpm::LearnArgs* learn) {
     launches += enqueue_p2g(e, e->table_large, par);
     launches += mpm::launch_grid_update(e->table_large, big, e->g_total, e->accum, e->vgrid, e->sdf, active_tiles(e), st,
                                         e->tune.grid_block);
-    launches += mpm::launch_g2p(e->table_large, big, e->n, e->P[par], e->P[1 - par], e->gidx, e->sigma[par],
+    launches += mpm::launch_g2p(e->table_large, big, e->n, e->P[par], e->P[1 - par], e->gidx, e->edge, e->sigma[par],
                                 e->sigma[1 - par], e->vgrid, e->sdf, e->pcell, e->bins[1 - par], e->order.crowded,
                                 e->d_flags, st, learn);
     return launches;
@@ -887,7 +892,8 @@ mpm_status plain_substeps(mpm_engine* e, int count) {
 // is even, the result moved to parity 1 - par, where an accepted large step
 // leaves its own: the state, its slot-to-particle map, and the counter set
 // the last substep filled (its slot order and cells stay valid, so the next
-// substep orders by it and clears the other set as usual).
+// substep orders by it; the set it came from, which has no list to be cleared
+// by, is zeroed).
 int enqueue_fallback(mpm_engine* e, int par) {
     cudaStream_t st = e->stream;
     int launches = 0;
@@ -905,7 +911,9 @@ int enqueue_fallback(mpm_engine* e, int par) {
         launches += mpm::launch_copy_words(e->sigma[1 - par], e->sigma[q], e->n, st);
         launches += mpm::launch_copy_words(sets + (size_t)(1 - par) * bins_set_words(e), sets + (size_t)q * bins_set_words(e),
                                            (long long)bins_set_words(e), st);
-        launches += mpm::launch_copy_words(e->bins[1 - par].nlist, e->bins[q].nlist, 1, st);
+        launches += mpm::launch_fill(reinterpret_cast<float*>(sets + (size_t)q * bins_set_words(e)),
+                                     (long long)bins_set_words(e), 0.0f, st);
+        launches += mpm::launch_fill(reinterpret_cast<float*>(e->ctl), 2, 0.0f, st);
     }
     return launches;
 }
@@ -1899,7 +1907,7 @@ extern "C" mpm_status mpm_autotune(mpm_engine* e, int32_t repeats, mpm_tuning* o
     }
     e->tune.grid_block = best.grid_block;
     tbest = 1e30f;
-    for (int k : {128, 256, 512}) {
+    for (int k : {128, 256}) {
         if (s != MPM_OK) break;
         e->tune.g2p_block = k;
         if ((s = median_time(MPM_STAGE_G2P, &ms)) != MPM_OK) break;

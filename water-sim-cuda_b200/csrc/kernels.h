@@ -52,11 +52,12 @@ int launch_radix_sort(const int32_t* keys, int n, const SortScratch& s, int32_t*
 // particle-major state, ordered by cell of the binning that produced it.
 // pcell[j] is the global cell of slot j; ccur holds one slot cursor per
 // cell, which the ordering's scatter draws the cell's slots from.  A counter
-// set holds the cell counts (global cells), the bin counts, and the list of
-// the bins that hold particles, as (scene, bin) in the order they were first
-// reached, with its length *nlist.  Two sets alternate: a substep orders the
-// particles by one and its G2P fills the other, which that substep clears
-// first.
+// set holds the cell counts (global cells) and the bin counts, which a G2P or
+// an import fills, and the list of the bins that hold particles, as (scene,
+// bin), with its length *nlist (zero until then), which the ordering by the
+// set makes.  Two sets alternate: a substep orders the particles by one and
+// its G2P fills the other, which that substep clears first, bin by bin of its
+// list.
 struct BinSet {
     uint32_t* ccount;
     int2* blist;
@@ -66,8 +67,8 @@ struct BinSet {
 
 // Counters of one substep, zero before its ordering: P2G's work units taken
 // and the length of the crowded-cell list.  The scatter resets work, G2P
-// resets crowded; an ordering whose substep is abandoned needs it zeroed by
-// the host.
+// resets crowded; an ordering whose substep is abandoned needs it and its
+// set's list length zeroed by the host.
 struct OrderCtl {
     uint32_t* work;
     uint32_t* crowded;
@@ -90,7 +91,10 @@ struct TileMarks {
 // Files the n particles of P (all scenes, slot order) into an empty set.
 int launch_bin_count(const SceneTable& sc, long long n, const float* P, int32_t* pcell, const BinSet& set,
                      cudaStream_t st);
-// Order by cell from set `cur`: gidx[new slot] = old slot, desc (P2G's items:
+// Slots per entry of the ordering's `edge`: the cells of the first and the
+// last of them.  G2P's CTAs take whole entries.
+constexpr int kEdgeSlots = 128;
+// Order by cell from set `cur`: gidx[new slot] = old slot, edge, desc (P2G's items:
 // kBinZ per listed bin, indexed like the cells), crowd / *ctl.crowded (the
 // crowded-cell list; crowd_cap entries of room, at least n / 4 + 64); clears
 // `other`; with tiles.mark set, advances tiles.stamp and marks the tiles the
@@ -101,7 +105,7 @@ int launch_bin_count(const SceneTable& sc, long long n, const float* P, int32_t*
 // to the list (0 = chosen per work item from its cells' counts).
 int launch_bin_order(const SceneTable& sc, long long n, long long bins_total, const BinSet& cur, const BinSet& other,
                      const OrderCtl& ctl, int32_t* bstart, int32_t* bpart, int scan_chunks, const int32_t* pcell,
-                     int32_t* ccur, int32_t* gidx, int2* desc, int4* crowd, int crowd_cap, int cell_cap,
+                     int32_t* ccur, int32_t* gidx, int2* edge, int2* desc, int4* crowd, int crowd_cap, int cell_cap,
                      const TileMarks& tiles, uint32_t* status, cudaStream_t st);
 // Chunks of the bin scan for a scene of `bins` bins.
 int bin_scan_chunks(long long bins);
@@ -140,9 +144,9 @@ struct LearnArgs {
 // sig_out[j] = sig_in[gidx[j]]; files slot j into `next`; zeroes *crowded
 // (OrderCtl).  learn: a large step of one scene (LearnArgs), else null.
 int launch_g2p(const SceneTable& sc, const SimParams& p0, long long n, const float* Pin, float* Pout,
-               const int32_t* gidx, const int32_t* sig_in, int32_t* sig_out, const float4* vgrid, const float* sdf,
-               int32_t* pcell, const BinSet& next, uint32_t* crowded, uint32_t* health, cudaStream_t st,
-               const LearnArgs* learn = nullptr, int block = 256);
+               const int32_t* gidx, const int2* edge, const int32_t* sig_in, int32_t* sig_out, const float4* vgrid,
+               const float* sdf, int32_t* pcell, const BinSet& next, uint32_t* crowded, uint32_t* health,
+               cudaStream_t st, const LearnArgs* learn = nullptr, int block = 256);
 
 // The kernels below take one scene's SimParams and pointers already offset to
 // that scene's part of the arrays.

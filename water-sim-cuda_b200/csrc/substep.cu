@@ -48,6 +48,11 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
                  "l"(gmem), "l"(pol)
                  : "memory");
 }
+__device__ __forceinline__ void cp_async16_plain(void* smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem))),
+                 "l"(gmem)
+                 : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
@@ -61,22 +66,18 @@ __device__ __forceinline__ void cp_async_wait() {
 // visible (griddepcontrol.wait; a no-op for an ordinary launch).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Files this lane's particle under global cell `gcell` (global bin `gbin`,
-// bin `bin` of scene `scene`) of a counter set: one reduction per distinct
-// cell of the warp (no value comes back, so no lane waits on it) and one
-// atomic per distinct bin, whose leader appends the bin to the set's list when
-// it is the bin's first particle.  The particle's place within its cell is
-// drawn later, by the ordering's scatter.  Every lane of the warp must call
-// it; lanes with gcell < 0 take part without counting.
-__device__ __forceinline__ void file_particle(int gcell, int gbin, int bin, int scene, const BinSet& set) {
+// Files this lane's particle under global cell `gcell` (global bin `gbin`) of
+// a counter set: one reduction per distinct cell of the warp and one per
+// distinct bin.  No value comes back, so no lane waits on them: which bins
+// hold particles is for the bin scan to see, and the particle's place within
+// its cell is drawn by the ordering's scatter.  Every lane of the warp must
+// call it; lanes with gcell < 0 take part without counting.
+__device__ __forceinline__ void file_particle(int gcell, int gbin, const BinSet& set) {
     const int lane = threadIdx.x & 31;
     const uint32_t peers = __match_any_sync(0xffffffffu, gcell);
     if (gcell >= 0 && lane == __ffs(peers) - 1) atomicAdd(set.ccount + gcell, (uint32_t)__popc(peers));
     const uint32_t bpeers = __match_any_sync(0xffffffffu, gbin);
-    if (gbin >= 0 && lane == __ffs(bpeers) - 1) {
-        if (atomicAdd(set.bcount + gbin, (uint32_t)__popc(bpeers)) == 0u)
-            set.blist[atomicAdd(set.nlist, 1u)] = make_int2(scene, bin);
-    }
+    if (gbin >= 0 && lane == __ffs(bpeers) - 1) atomicAdd(set.bcount + gbin, (uint32_t)__popc(bpeers));
 }
 
 // Scene lookup for the per-particle and per-node kernels.  With one scene
@@ -472,21 +473,22 @@ __global__ void __launch_bounds__(256) bin_count_kernel(SceneTable sc, long long
                                                         int32_t* __restrict__ pcell, BinSet set) {
     const long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const bool valid = j < n;
-    int gcell = -1, gbin = -1, bin = -1, scene = 0;
+    int gcell = -1, gbin = -1;
     if (valid) {
-        scene = scene_of(sc.poff, sc.count, j);
-        const SimParams& p = sc.prm[scene];
+        int bin;
+        const SimParams& p = sc.prm[scene_of(sc.poff, sc.count, j)];
         const float4 q = __ldg(reinterpret_cast<const float4*>(P + (size_t)j * kAFloats));
         gcell = (int)p.coff + cell_of(p, q.x, q.y, q.z, &bin);
         gbin = (int)p.boff + bin;
     }
-    file_particle(gcell, gbin, bin, scene, set);
+    file_particle(gcell, gbin, set);
     if (valid) pcell[j] = gcell;
 }
 
 // Bin starts, over (scene, chunk of kScanChunk bins) CTAs, no CTA waiting on
 // another: bstart[i] = poff + sum of bcount[0..i) over the scene's nb + 1
-// bins (global slots).  Up to kScanDirect chunks a CTA adds up the counts of
+// bins (global slots); and the list of the bins that hold particles, each CTA
+// appending its own in index order.  Up to kScanDirect chunks a CTA adds up the counts of
 // all earlier chunks itself and scans its own; scenes of more get a launch
 // before it, in which bin_sum_kernel writes each chunk's sum to bpart[scene *
 // chunks + chunk].  Measured, one launch against two: 2.1 / 4.0 us at 32^3
@@ -529,20 +531,21 @@ __global__ void __launch_bounds__(kScanThreads) bin_sum_kernel(SceneTable sc, co
     if (threadIdx.x == 0) bpart[(long long)scene * gridDim.y + chunk] = sum;
 }
 
-__global__ void __launch_bounds__(kScanThreads) bin_scan_kernel(SceneTable sc, const uint32_t* __restrict__ bcount_all,
+__global__ void __launch_bounds__(kScanThreads) bin_scan_kernel(SceneTable sc, BinSet set,
                                                                 const int32_t* __restrict__ bpart,
                                                                 int32_t* __restrict__ bstart_all) {
     pdl_wait();
     __shared__ int s_val[kScanChunk];
     __shared__ int s_red[kScanWarps];
-    __shared__ int s_warp[kScanWarps];
+    __shared__ int2 s_warp[kScanWarps];
+    __shared__ uint32_t s_list;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int scene = blockIdx.x, chunk = blockIdx.y;
     const SimParams& p = sc.prm[scene];
     const int nbins = p.nb + 1;
     const int c0 = chunk * kScanChunk;
     if (c0 >= nbins) return;
-    const uint32_t* bcount = bcount_all + p.boff;
+    const uint32_t* bcount = set.bcount + p.boff;
     int32_t* bstart = bstart_all + p.boff + c0;
     const int m = min(kScanChunk, nbins - c0);
     // Particles of the scene's earlier chunks.
@@ -559,23 +562,31 @@ __global__ void __launch_bounds__(kScanThreads) bin_scan_kernel(SceneTable sc, c
         s_val[i] = i < m ? (int)__ldg(bcount + c0 + i) : 0;
     }
     const int carry = (int)p.poff + scan_block_sum(pre, s_red);  // its barrier also publishes s_val
-    int v[kScanPer], sum = 0;
+    int v[kScanPer];
+    int2 sum = make_int2(0, 0);  // particles, occupied bins
 #pragma unroll
     for (int k = 0; k < kScanPer; ++k) {
         v[k] = s_val[t * kScanPer + k];
-        sum += v[k];
+        sum.x += v[k];
+        sum.y += v[k] != 0;
     }
-    int incl = sum;
+    int2 incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
+        const int x = __shfl_up_sync(0xffffffffu, incl.x, o), y = __shfl_up_sync(0xffffffffu, incl.y, o);
+        if (lane >= o) incl.x += x, incl.y += y;
     }
     if (lane == 31) s_warp[warp] = incl;
     __syncthreads();
-    int run = carry + incl - sum;
+    int run = carry + incl.x - sum.x, at = incl.y - sum.y, occupied = 0;
 #pragma unroll
-    for (int w = 0; w < kScanWarps; ++w) run += w < warp ? s_warp[w] : 0;
+    for (int w = 0; w < kScanWarps; ++w) {
+        const int2 x = s_warp[w];
+        run += w < warp ? x.x : 0;
+        at += w < warp ? x.y : 0;
+        occupied += x.y;
+    }
+    if (t == 0) s_list = atomicAdd(set.nlist, (uint32_t)occupied);
 #pragma unroll
     for (int k = 0; k < kScanPer; ++k) {
         s_val[t * kScanPer + k] = run;
@@ -587,6 +598,9 @@ __global__ void __launch_bounds__(kScanThreads) bin_scan_kernel(SceneTable sc, c
         const int i = k * kScanThreads + t;
         if (i < m) bstart[i] = s_val[i];
     }
+#pragma unroll
+    for (int k = 0; k < kScanPer; ++k)
+        if (v[k] != 0) set.blist[s_list + at++] = make_int2(scene, c0 + t * kScanPer + k);
 }
 
 // The P2G order of a bin's cells (one warp; lane holds the counts of cells
@@ -733,14 +747,16 @@ __global__ void __launch_bounds__(kCellWarps * 32) cell_scan_kernel(SceneTable s
 // the lanes sharing a cell take consecutive slots in lane order).  A thread
 // files kScatterPer particles (block b: particles b * kScatterPer * blockDim
 // .. + kScatterPer * blockDim, one blockDim-wide slice per pass), so that the
-// cursor atomics of its passes are in flight together.  The first block also
-// resets the other set's list, which the cell scan has used up, and P2G's work
+// cursor atomics of its passes are in flight together.  edge[b] receives the
+// cells of the first and the last slot of every kEdgeSlots slots (G2P's
+// footprints).  The first block also resets the other set's list, which the cell scan has used up, and P2G's work
 // counter, and advances the tile stamp.
 constexpr int kScatterPer = 4;
 
 __global__ void __launch_bounds__(256) bin_scatter_kernel(long long n, const int32_t* __restrict__ pcell,
                                                           int32_t* __restrict__ ccur, int32_t* __restrict__ gidx,
-                                                          OrderCtl ctl, uint32_t* __restrict__ clear_nlist,
+                                                          int2* __restrict__ edge, OrderCtl ctl,
+                                                          uint32_t* __restrict__ clear_nlist,
                                                           uint32_t* __restrict__ tstamp) {
     pdl_wait();
     const long long j0 = blockIdx.x * (long long)blockDim.x * kScatterPer + threadIdx.x;
@@ -766,7 +782,11 @@ __global__ void __launch_bounds__(256) bin_scatter_kernel(long long n, const int
 #pragma unroll
     for (int k = 0; k < kScatterPer; ++k) {
         const int b = __shfl_sync(0xffffffffu, base[k], __ffs(peers[k]) - 1);
-        if (cell[k] >= 0) gidx[b + __popc(peers[k] & lanemask_lt())] = (int32_t)(j0 + (long long)k * blockDim.x);
+        if (cell[k] < 0) continue;
+        const int slot = b + __popc(peers[k] & lanemask_lt());
+        gidx[slot] = (int32_t)(j0 + (long long)k * blockDim.x);
+        if (slot % kEdgeSlots == 0) edge[slot / kEdgeSlots].x = cell[k];
+        if (slot % kEdgeSlots == kEdgeSlots - 1 || slot == n - 1) edge[slot / kEdgeSlots].y = cell[k];
     }
 }
 
@@ -911,30 +931,39 @@ __global__ void __launch_bounds__(256) grid_tiles_kernel(SceneTable sc, SimParam
 // R substeps under a constant acceleration move a particle by exactly that.
 enum G2PMode : int { kG2PPlain = 0, kG2PLearned = 1, kG2PCollect = 2, kG2PLarge = 3, kG2PLearnedTc = 4 };
 
-// Particles per thread of a G2P instantiation: two for the batched plain
-// mode (records staged in dynamic shared memory, kPer x 3 x blockDim float4),
-// one otherwise.  Measured per substep on the 64-scene batch, two per thread
-// cut G2P by 5-8 %; on one scene (fewer registers, more warps per SM) two
-// per thread cost 5 % and four 20 %.
-__host__ __device__ constexpr int g2p_per_thread(bool batch, int mode, bool wide) {
-    return (mode == 0 && !wide && batch) ? 2 : 1;
-}
+// The nodes a CTA's particles gather from, staged in shared memory.  Slots
+// are ordered by cell, so a CTA's particles fill a run of cells: with
+// particles to fill them, some z-layers of one bin, or the last layers of one
+// and the first of another, whose stencils reach 10 x 6 nodes per plane and
+// two planes more than there are layers.  The ordering leaves the cells of a
+// run's first and last slot in `edge`, so the CTA copies those planes in while
+// its threads still follow gidx to their records; the 27 node reads of a
+// particle then hit shared memory.  (Straight from global memory every row of
+// three nodes is an L1 or L2 round trip of its own, about ten in a row per
+// particle at 64 registers: 12.5 long-scoreboard stalls per issue.)  A
+// particle of neither region (a run that crosses a third bin, as in sparse
+// fluid) reads the grid.  Nodes outside the grid are staged as zeros whose
+// mass has its sign bit set, like a node inside an obstacle: either way the
+// SDF test below must not be skipped.
+//
+// G2P per substep before / after (with 128-thread CTAs, whose barrier waits for
+// fewer warps: 94 us at 256; and with reductions instead of returning atomics
+// in the filing): 650k particles 37.6 / 30.4 us, 2M 104 / 83 us, 6.9M in 256^3
+// 325 / 258 us, the 64-scene batch 362 / 291 us.  DRAM then carries 3.9 of the
+// 6.5 TB/s; issue (57 % of slots) and the chain gidx - record - stores bound it.
+constexpr int kStagePlanes = 9;  // planes of 60 nodes: 8.6 KB per CTA
 
 // CTAs per SM: the learned tcgen05 mode fits four (64 registers, 128 TMEM
 // columns and about 45 KB of shared memory each), so one CTA's MMA waits
 // overlap the other three's work; mma.sync learned, collect and batched
 // modes need more registers.
-// kWide: 256-thread CTAs free to use up to 255 registers (one CTA per SM,
-// every node load of a particle in flight at once) instead of 64 registers
-// and four CTAs per SM; chosen by the autotuner.
-template <bool kBatch, int kMode, bool kWide = false>
-__global__ void __launch_bounds__(256, kWide ? 1 : (kMode == 1 ? 2 : ((kBatch || kMode == 2) ? 3 : 4))) g2p_kernel(SceneTable sc, SimParams p0, long long n_total, const float* __restrict__ Pin,
-                                                  float* __restrict__ Pout, const int32_t* __restrict__ gidx,
-                                                  const int32_t* __restrict__ sig_in, int32_t* __restrict__ sig_out,
-                                                  const float4* __restrict__ vgrid_all, const float* __restrict__ sdf_all,
-                                                  int32_t* __restrict__ pcell, BinSet next,
-                                                  uint32_t* __restrict__ crowded, uint32_t* __restrict__ health,
-                                                  LearnArgs la) {
+template <bool kBatch, int kMode>
+__global__ void __launch_bounds__(256, kMode == 1 ? 2 : ((kBatch || kMode == 2) ? 3 : 4)) g2p_kernel(
+    SceneTable sc, SimParams p0, long long n_total, const float* __restrict__ Pin, float* __restrict__ Pout,
+    const int32_t* __restrict__ gidx, const int2* __restrict__ edge, const int32_t* __restrict__ sig_in,
+    int32_t* __restrict__ sig_out, const float4* __restrict__ vgrid_all, const float* __restrict__ sdf_all,
+    int32_t* __restrict__ pcell, BinSet next, uint32_t* __restrict__ crowded, uint32_t* __restrict__ health,
+    LearnArgs la) {
     pdl_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) *crowded = 0u;  // P2G has taken its crowded-cell list
     __shared__ SimParams s_prm[kBatch ? kTableScenes : 1];
@@ -942,69 +971,78 @@ __global__ void __launch_bounds__(256, kWide ? 1 : (kMode == 1 ? 2 : ((kBatch ||
     __shared__ int s_range[2];
     __shared__ __align__(16) unsigned char s_mlp_raw[kMode == kG2PLearned ? sizeof(MlpPacked) : 16];
     __shared__ uint32_t s_stage[kMode == kG2PLearned ? 8 * 32 * kMlpStageStride : 1];
+    __shared__ float4 s_node_own[kMode == kG2PLearnedTc ? 1 : kStagePlanes * kFootPlane];
     extern __shared__ __align__(1024) unsigned char s_dyn[];  // MlpTcSmem in the tcgen05 mode
     if constexpr (kMode == kG2PLearned) {
         const uint4* src = reinterpret_cast<const uint4*>(la.mlp);
         uint4* dst = reinterpret_cast<uint4*>(s_mlp_raw);
         for (int i = threadIdx.x; i < (int)(sizeof(MlpPacked) / 16); i += blockDim.x) dst[i] = __ldg(src + i);
-        __syncthreads();
     }
+    float4* s_node = s_node_own;
     if constexpr (kMode == kG2PLearnedTc) {
         MlpTcSmem& ts = *reinterpret_cast<MlpTcSmem*>(s_dyn);
+        // The layer-input buffer holds the nodes until the MLP starts.
+        static_assert(sizeof(ts.a) >= kStagePlanes * kFootPlane * sizeof(float4), "staged nodes fit the MLP input");
+        s_node = reinterpret_cast<float4*>(ts.a);
         const uint4* src = reinterpret_cast<const uint4*>(la.mlp_tc);
         uint4* dst = reinterpret_cast<uint4*>(&ts.w);
         for (int i = threadIdx.x; i < (int)(sizeof(MlpTc) / 16); i += blockDim.x) dst[i] = __ldg(src + i);
         mlp_tc_begin(ts, la.wait_test);  // TMEM columns and the mbarrier; synchronises the CTA
     }
-    constexpr int kPer = g2p_per_thread(kBatch, kMode, kWide);
-    const long long cta0 = (long long)blockIdx.x * kPer * blockDim.x;  // this CTA's particles: [cta0, cta1)
-    const SceneLookup<kBatch> look(sc, sc.poff, s_prm, s_first, s_range, cta0,
-                                   min(cta0 + (long long)kPer * blockDim.x, n_total));
-    // The plain mode takes kPer particles per thread (block b: particles
-    // b * kPer * blockDim .. + kPer * blockDim, one blockDim-wide slice per
-    // pass) and requests all their positions and F up front, into shared
-    // memory with cp.async, so that a record's load overlaps the passes
-    // before it.  Every lane makes all kPer passes: filing is warp-wide.
-    float4* s_rec = reinterpret_cast<float4*>(s_dyn);  // [kPer][3][blockDim] when kPer > 1
-    if constexpr (kPer > 1) {
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            const long long jk = ((long long)blockIdx.x * kPer + k) * blockDim.x + threadIdx.x;
-            if (jk < n_total) {
-                const float4* qk = reinterpret_cast<const float4*>(Pin + (size_t)__ldg(gidx + jk) * kAFloats);
-#pragma unroll
-                for (int v = 0; v < 3; ++v) cp_async16(s_rec + (k * 3 + v) * blockDim.x + threadIdx.x, qk + v);
-            }
-        }
-        cp_async_commit();
-    }
-#pragma unroll 1
-    for (int k = 0; k < kPer; ++k) {
-    const long long jj = ((long long)blockIdx.x * kPer + k) * blockDim.x + threadIdx.x;
-    const bool valid = jj < n_total;
-    const long long j = valid ? jj : n_total - 1;  // idle lanes redo the last particle and store nothing
+    const long long cta0 = (long long)blockIdx.x * blockDim.x;  // this CTA's particles: [cta0, cta1)
+    const long long cta1 = min(cta0 + (long long)blockDim.x, n_total);
+    const SceneLookup<kBatch> look(sc, sc.poff, s_prm, s_first, s_range, cta0, cta1);
+    const bool valid = cta0 + threadIdx.x < n_total;
+    const long long j = valid ? cta0 + threadIdx.x : n_total - 1;  // idle lanes redo the last particle and store nothing
     const int scene = look.scene(j);
     const SimParams& p = kBatch ? look.params(scene) : p0;
     const float4* vgrid = vgrid_all + p.goff;
     const float* sdf = sdf_all + p.goff;
     const int src = __ldg(gidx + j);
-    const float4* q = reinterpret_cast<const float4*>(Pin + (size_t)src * kAFloats);
-    float4 q0, q1, q2;
-    if constexpr (kPer > 1) {
-        if (k == 0) cp_async_wait<0>();  // every record of this thread has arrived
-        const float4* r = s_rec + (k * 3) * blockDim.x + threadIdx.x;
-        q0 = valid ? r[0] : make_float4(0.f, 0.f, 0.f, 0.f);
-        q1 = valid ? r[blockDim.x] : make_float4(0.f, 0.f, 0.f, 0.f);
-        q2 = valid ? r[2 * blockDim.x] : make_float4(0.f, 0.f, 0.f, 0.f);
-    } else {
-        // Records are 96 bytes from a cudaMalloc'd base, so each starts on a
-        // 32-byte boundary: one 32-byte load (sm_100 ld.global.v8) for the
-        // position and F00..F04, one 16-byte load for F05..F08.
-        asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-            : "=f"(q0.x), "=f"(q0.y), "=f"(q0.z), "=f"(q0.w), "=f"(q1.x), "=f"(q1.y), "=f"(q1.z), "=f"(q1.w)
-            : "l"(q));
-        q2 = __ldg(q + 2);
+    // The CTA's two regions: node origin (o*) of the first staged plane, and
+    // planes (nz*).
+    int ox0, oy0, oz0, nz0, ox1, oy1, oz1, nz1;
+    const int scene0 = look.scene(cta0), scene1 = look.scene(cta1 - 1);
+    {
+        const SimParams& pa = kBatch ? look.params(scene0) : p0;
+        const SimParams& pb = kBatch ? look.params(scene1) : p0;
+        const int l0 = __ldg(&edge[cta0 / kEdgeSlots].x) - (int)pa.coff;
+        const int l1 = __ldg(&edge[(cta1 - 1) / kEdgeSlots].y) - (int)pb.coff;
+        const int bin0 = l0 / kBinCells, bin1 = l1 / kBinCells;
+        const int z0 = l0 % kBinCells / 32, z1 = l1 % kBinCells / 32;
+        const bool one = bin0 == bin1 && scene0 == scene1;
+        nz0 = bin0 >= pa.nb ? 0 : (one ? z1 : kBinZ - 1) - z0 + 3;  // the overflow bin reaches no node
+        nz1 = one || bin1 >= pb.nb ? 0 : z1 + 3;
+        if (nz0 + nz1 > kStagePlanes) nz1 = 0;
+        bin_origin(pa, bin0, &ox0, &oy0, &oz0);
+        bin_origin(pb, bin1, &ox1, &oy1, &oz1);
+        oz0 += z0;
+        // 60 threads copy a plane, the CTA two or four at a time.
+        const int t = threadIdx.x, sub = t / kFootPlane, step = blockDim.x / kFootPlane;
+        const int tx = t % kTX, ty = t % kFootPlane / kTX;
+        for (int plane = sub < step ? sub : nz0 + nz1; plane < nz0 + nz1; plane += step) {
+            const bool second = plane >= nz0;
+            const SimParams& pr = second ? pb : pa;
+            const int x = (second ? ox1 : ox0) + tx, y = (second ? oy1 : oy0) + ty,
+                      z = second ? oz1 + plane - nz0 : oz0 + plane;
+            float4* dst = s_node + plane * kFootPlane + ty * kTX + tx;
+            if (node_in_grid(pr, x, y, z))
+                cp_async16_plain(dst, vgrid_all + pr.goff + node_index(pr, x, y, z));
+            else
+                *dst = make_float4(-0.0f, 0.f, 0.f, 0.f);
+        }
+        cp_async_commit();
     }
+    const int sig = __ldg(sig_in + src);  // early: its round trip overlaps the record's
+    const float4* q = reinterpret_cast<const float4*>(Pin + (size_t)src * kAFloats);
+    // Records are 96 bytes from a cudaMalloc'd base, so each starts on a
+    // 32-byte boundary: one 32-byte load (sm_100 ld.global.v8) for the
+    // position and F00..F04, one 16-byte load for F05..F08.
+    float4 q0, q1;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(q0.x), "=f"(q0.y), "=f"(q0.z), "=f"(q0.w), "=f"(q1.x), "=f"(q1.y), "=f"(q1.z), "=f"(q1.w)
+        : "l"(q));
+    const float4 q2 = __ldg(q + 2);
     float4 qv = make_float4(0.f, 0.f, 0.f, 0.f);
     if constexpr (kMode != kG2PPlain) qv = __ldg(q + 3);  // old velocity
     const float pos[3] = {q0.x, q0.y, q0.z};
@@ -1029,57 +1067,67 @@ __global__ void __launch_bounds__(256, kWide ? 1 : (kMode == 1 ? 2 : ((kBatch ||
     // row form made the tcgen05 learned G2P spill three times as much and run
     // 7 % slower.
     float tv[3] = {0.f, 0.f, 0.f}, tc[9], tm = 0.f;
+    // This particle's first node in the staged planes, -1 if it is in neither
+    // region.
+    int at = -1;
+    if ((!kBatch || scene == scene1) && (unsigned)(bx - ox1) < kBinX && (unsigned)(by - oy1) < kBinY && bz >= oz1 &&
+        bz - oz1 + 3 <= nz1)
+        at = ((nz0 + bz - oz1) * kTY + by - oy1) * kTX + bx - ox1;
+    if ((!kBatch || scene == scene0) && (unsigned)(bx - ox0) < kBinX && (unsigned)(by - oy0) < kBinY && bz >= oz0 &&
+        bz - oz0 + 3 <= nz0)
+        at = ((bz - oz0) * kTY + by - oy0) * kTX + bx - ox0;
+    cp_async_wait<0>();
+    __syncthreads();
     // Set when a stencil node lies outside the grid or inside an obstacle:
     // only then can the SDF at the new position be negative (see below).
     uint32_t sdf_risk = 0u;
     const int plane = p.sx * p.sy;
-    // Whole stencil inside the grid (almost every particle): no per-node
-    // bounds tests.  Nodes outside the grid add nothing.
-    const bool inside = p.sx >= 3 && p.sy >= 3 && p.sz >= 3 && (unsigned)bx <= (unsigned)(p.sx - 3) &&
-                        (unsigned)by <= (unsigned)(p.sy - 3) && (unsigned)bz <= (unsigned)(p.sz - 3);
     constexpr bool kRowSums = kMode != kG2PLearned && kMode != kG2PLearnedTc;
     if constexpr (kRowSums) {
         float M[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) M[k] = 0.f;
+        // One row of three nodes along x, at offsets (b, c).
+        auto add_row = [&](int b, int c, const float4* g) {
+            sdf_risk |= (__float_as_uint(g[0].x) | __float_as_uint(g[1].x) | __float_as_uint(g[2].x)) >> 31;
+            const float s0[3] = {wx[0] * g[0].y + wx[1] * g[1].y + wx[2] * g[2].y,
+                                 wx[0] * g[0].z + wx[1] * g[1].z + wx[2] * g[2].z,
+                                 wx[0] * g[0].w + wx[1] * g[1].w + wx[2] * g[2].w};
+            const float s1[3] = {wx[2] * g[2].y - wx[0] * g[0].y, wx[2] * g[2].z - wx[0] * g[0].z,
+                                 wx[2] * g[2].w - wx[0] * g[0].w};
+            const float wyz = wy[b] * wz[c];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
+            for (int k = 0; k < 3; ++k) {
+                tv[k] += wyz * s0[k];
+                M[3 * k + 0] += wyz * s1[k];
+                if (b == 0) M[3 * k + 1] -= wyz * s0[k];
+                if (b == 2) M[3 * k + 1] += wyz * s0[k];
+                if (c == 0) M[3 * k + 2] -= wyz * s0[k];
+                if (c == 2) M[3 * k + 2] += wyz * s0[k];
+            }
+            if constexpr (kMode != kG2PPlain)
+                tm += wyz * (wx[0] * fabsf(g[0].x) + wx[1] * fabsf(g[1].x) + wx[2] * fabsf(g[2].x));
+        };
+        if (at >= 0) {
+            const float4* base = s_node + at;
 #pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                const int z = bz + c, y = by + b;
-                float4 g[3];
-                if (inside) {
-                    const float4* row = vgrid + ((size_t)z * plane + (size_t)y * p.sx + bx);
+            for (int c = 0; c < 3; ++c)
 #pragma unroll
-                    for (int a = 0; a < 3; ++a) g[a] = __ldg(row + a);
-                } else {
+                for (int b = 0; b < 3; ++b) add_row(b, c, base + (c * kTY + b) * kTX);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    const int z = bz + c, y = by + b;
                     const bool zy = (unsigned)z < (unsigned)p.sz && (unsigned)y < (unsigned)p.sy;
+                    const float4* row = vgrid + ((long long)z * plane + (long long)y * p.sx + bx);
+                    float4 g[3];
 #pragma unroll
-                    for (int a = 0; a < 3; ++a) {
-                        const bool ok = zy && (unsigned)(bx + a) < (unsigned)p.sx;
-                        g[a] = ok ? __ldg(vgrid + ((size_t)z * plane + (size_t)y * p.sx + bx + a))
-                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (!ok) sdf_risk = 1u;
-                    }
+                    for (int a = 0; a < 3; ++a)
+                        g[a] = zy && (unsigned)(bx + a) < (unsigned)p.sx ? __ldg(row + a) : make_float4(-0.0f, 0.f, 0.f, 0.f);
+                    add_row(b, c, g);
                 }
-                sdf_risk |= (__float_as_uint(g[0].x) | __float_as_uint(g[1].x) | __float_as_uint(g[2].x)) >> 31;
-                const float s0[3] = {wx[0] * g[0].y + wx[1] * g[1].y + wx[2] * g[2].y,
-                                     wx[0] * g[0].z + wx[1] * g[1].z + wx[2] * g[2].z,
-                                     wx[0] * g[0].w + wx[1] * g[1].w + wx[2] * g[2].w};
-                const float s1[3] = {wx[2] * g[2].y - wx[0] * g[0].y, wx[2] * g[2].z - wx[0] * g[0].z,
-                                     wx[2] * g[2].w - wx[0] * g[0].w};
-                const float wyz = wy[b] * wz[c];
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    tv[k] += wyz * s0[k];
-                    M[3 * k + 0] += wyz * s1[k];
-                    if (b == 0) M[3 * k + 1] -= wyz * s0[k];
-                    if (b == 2) M[3 * k + 1] += wyz * s0[k];
-                    if (c == 0) M[3 * k + 2] -= wyz * s0[k];
-                    if (c == 2) M[3 * k + 2] += wyz * s0[k];
-                }
-                if constexpr (kMode != kG2PPlain)
-                    tm += wyz * (wx[0] * fabsf(g[0].x) + wx[1] * fabsf(g[1].x) + wx[2] * fabsf(g[2].x));
             }
         }
         const float gx = fx - 1.0f, gy = fy - 1.0f, gz = fz - 1.0f;  // exact
@@ -1092,10 +1140,9 @@ __global__ void __launch_bounds__(256, kWide ? 1 : (kMode == 1 ? 2 : ((kBatch ||
     } else {
 #pragma unroll
         for (int k = 0; k < 9; ++k) tc[k] = 0.f;
-        // One node of the stencil, offsets (a, b, c), `row` = node (base x, y, z).
-        auto gather = [&](int a, int b, int c, const float4* row) {
+        // One node of the stencil, offsets (a, b, c).
+        auto gather = [&](int a, int b, int c, float4 g) {
             const float dxv = -(fx - (float)a), dyv = -(fy - (float)b), dzv = -(fz - (float)c);
-            const float4 g = __ldg(row + a);
             sdf_risk |= __float_as_uint(g.x) >> 31;
             const float w = wx[a] * wy[b] * wz[c];
             tv[0] += w * g.y;
@@ -1113,28 +1160,27 @@ __global__ void __launch_bounds__(256, kWide ? 1 : (kMode == 1 ? 2 : ((kBatch ||
             tc[7] += term * g.w * dyv;
             tc[8] += term * g.w * dzv;
         };
+        if (at >= 0) {
+            const float4* base = s_node + at;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const int z = bz + c;
-            if (!inside && (unsigned)z >= (unsigned)p.sz) {
-                sdf_risk = 1u;
-                continue;
-            }
+            for (int c = 0; c < 3; ++c)
 #pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                const int y = by + b;
-                if (!inside && (unsigned)y >= (unsigned)p.sy) {
-                    sdf_risk = 1u;
-                    continue;
-                }
-                const float4* row = vgrid + ((size_t)z * plane + (size_t)y * p.sx + bx);
+                for (int b = 0; b < 3; ++b)
 #pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    if (!inside && (unsigned)(bx + a) >= (unsigned)p.sx) {
-                        sdf_risk = 1u;
-                        continue;
-                    }
-                    gather(a, b, c, row);
+                    for (int a = 0; a < 3; ++a) gather(a, b, c, base[(c * kTY + b) * kTX + a]);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const int z = bz + c;
+#pragma unroll
+                for (int b = 0; b < 3; ++b) {
+                    const int y = by + b;
+                    const bool zy = (unsigned)z < (unsigned)p.sz && (unsigned)y < (unsigned)p.sy;
+                    const float4* row = vgrid + ((long long)z * plane + (long long)y * p.sx + bx);
+#pragma unroll
+                    for (int a = 0; a < 3; ++a)
+                        gather(a, b, c, zy && (unsigned)(bx + a) < (unsigned)p.sx ? __ldg(row + a)
+                                                                               : make_float4(-0.0f, 0.f, 0.f, 0.f));
                 }
             }
         }
@@ -1159,6 +1205,7 @@ __global__ void __launch_bounds__(256, kWide ? 1 : (kMode == 1 ? 2 : ((kBatch ||
                                  s_stage + (threadIdx.x >> 5) * 32 * kMlpStageStride, f, dv);
             } else {
                 MlpTcSmem& ts = *reinterpret_cast<MlpTcSmem*>(s_dyn);
+                __syncthreads();  // every thread has read its nodes: the input buffer is the MLP's now
                 mlp_forward_tc(ts, f, dv);
                 mlp_tc_end(ts);  // TMEM freed before the rest of the particle update
                 if (ts.failed && threadIdx.x == 0) atomicOr(la.status, kStatusTimeout);
@@ -1189,7 +1236,7 @@ __global__ void __launch_bounds__(256, kWide ? 1 : (kMode == 1 ? 2 : ((kBatch ||
                 atomicAdd(la.stat + 2, dev[2]);
             }
         } else if (valid) {  // collection probe: la.feat holds n rows
-            float* fo = la.feat + (size_t)__ldg(sig_in + src) * kMlpIn;
+            float* fo = la.feat + (size_t)sig * kMlpIn;
 #pragma unroll
             for (int k = 0; k < kMlpIn; k += 4) *reinterpret_cast<float4*>(fo + k) = make_float4(f[k], f[k + 1], f[k + 2], f[k + 3]);
         }
@@ -1238,13 +1285,14 @@ __global__ void __launch_bounds__(256, kWide ? 1 : (kMode == 1 ? 2 : ((kBatch ||
             tv[2] -= nrm.z * vdn;
         }
     }
-    int bin = -1, gcell = -1, gbin = -1;
+    int gcell = -1, gbin = -1;
     if (valid) {
+        int bin;
         gcell = (int)p.coff + cell_of(p, nx, ny, nz, &bin);
         gbin = (int)p.boff + bin;
     }
-    file_particle(gcell, gbin, bin, scene, next);
-    if (!valid) continue;  // only the last passes of the last block have idle lanes
+    file_particle(gcell, gbin, next);
+    if (!valid) return;  // only the last block has idle lanes
     float4* o = reinterpret_cast<float4*>(Pout + (size_t)j * kAFloats);
     {
         // Three 32-byte stores (st.global.v8) of the 96-byte record: half the
@@ -1258,10 +1306,10 @@ __global__ void __launch_bounds__(256, kWide ? 1 : (kMode == 1 ? 2 : ((kBatch ||
                          "f"(w[8 * h + 4]), "f"(w[8 * h + 5]), "f"(w[8 * h + 6]), "f"(w[8 * h + 7])
                          : "memory");
     }
-    sig_out[j] = __ldg(sig_in + src);
+    sig_out[j] = sig;
     pcell[j] = gcell;
     if constexpr (kMode == kG2PCollect) {
-        float* vo = la.vel + (size_t)__ldg(sig_in + src) * 3;
+        float* vo = la.vel + (size_t)sig * 3;
         vo[0] = tv[0], vo[1] = tv[1], vo[2] = tv[2];
     }
 
@@ -1271,7 +1319,6 @@ __global__ void __launch_bounds__(256, kWide ? 1 : (kMode == 1 ? 2 : ((kBatch ||
     if (!(nx >= 0.f && nx < (float)p.sx && ny >= 0.f && ny < (float)p.sy && nz >= 0.f && nz < (float)p.sz))
         flags |= 2u;
     if (flags) atomicOr(health, flags);
-    }
 }
 
 // ------------------------------------------------------- state transfer ----
@@ -1436,17 +1483,17 @@ int bin_scan_chunks(long long bins) { return (int)std::max(1LL, (bins + kScanChu
 
 int launch_bin_order(const SceneTable& sc, long long n, long long bins_total, const BinSet& cur, const BinSet& other,
                      const OrderCtl& ctl, int32_t* bstart, int32_t* bpart, int scan_chunks, const int32_t* pcell,
-                     int32_t* ccur, int32_t* gidx, int2* desc, int4* crowd, int crowd_cap, int cell_cap,
+                     int32_t* ccur, int32_t* gidx, int2* edge, int2* desc, int4* crowd, int crowd_cap, int cell_cap,
                      const TileMarks& tiles, uint32_t* status, cudaStream_t st) {
     if (n <= 0) return 0;
     const dim3 scan_grid((unsigned)sc.count, (unsigned)scan_chunks);
     const bool summed = scan_chunks > kScanDirect;
     if (summed) launch_dep(bin_sum_kernel, scan_grid, kScanThreads, 0, st, sc, cur.bcount, bpart);
-    launch_dep(bin_scan_kernel, scan_grid, kScanThreads, 0, st, sc, cur.bcount, summed ? bpart : nullptr, bstart);
+    launch_dep(bin_scan_kernel, scan_grid, kScanThreads, 0, st, sc, cur, summed ? bpart : nullptr, bstart);
     const int ctas = (int)std::max(1LL, std::min((long long)blocks_for(bins_total, kCellWarps), 148LL * 4));
     launch_dep(cell_scan_kernel, ctas, kCellWarps * 32, 0, st, sc, cur, other, ctl, bstart, ccur, desc, crowd,
                crowd_cap, std::max(cell_cap, 0), tiles.stamp, tiles.mark, status);
-    launch_dep(bin_scatter_kernel, blocks_for(n, 256 * kScatterPer), 256, 0, st, n, pcell, ccur, gidx, ctl,
+    launch_dep(bin_scatter_kernel, blocks_for(n, 256 * kScatterPer), 256, 0, st, n, pcell, ccur, gidx, edge, ctl,
                other.nlist, tiles.stamp);
     return summed ? 4 : 3;
 }
@@ -1491,44 +1538,23 @@ int launch_grid_update(const SceneTable& sc, const SimParams& p0, long long g_to
 }
 
 int launch_g2p(const SceneTable& sc, const SimParams& p0, long long n, const float* Pin, float* Pout,
-               const int32_t* gidx, const int32_t* sig_in, int32_t* sig_out, const float4* vgrid, const float* sdf,
-               int32_t* pcell, const BinSet& next, uint32_t* crowded, uint32_t* health, cudaStream_t st,
-               const LearnArgs* learn, int block) {
+               const int32_t* gidx, const int2* edge, const int32_t* sig_in, int32_t* sig_out, const float4* vgrid,
+               const float* sdf, int32_t* pcell, const BinSet& next, uint32_t* crowded, uint32_t* health,
+               cudaStream_t st, const LearnArgs* learn, int block) {
     if (n <= 0) return 0;
     const LearnArgs la = learn ? *learn : LearnArgs{};
-    const unsigned grid = blocks_for(n, 256);
-    if (learn && sc.count == 1 && la.mlp_tc) {
-        launch_dep(g2p_kernel<false, kG2PLearnedTc>, grid, 256, sizeof(MlpTcSmem), st,
-            sc, p0, n, Pin, Pout, gidx, sig_in, sig_out, vgrid, sdf, pcell, next, crowded, health, la);
-        return 1;
-    }
-    // Plain G2P: 128- or 256-thread CTAs, or 512 = the register-wide 256-thread
-    // variant (the learned modes stage 8 warps of MLP inputs and always run 256).
-    const bool wide = block == 512;
-    const int pb = wide ? 256 : ((block == 128 || block == 256) ? block : 256);
-    if (learn && sc.count == 1 && la.mlp)
-        launch_dep(g2p_kernel<false, kG2PLearned>, grid, 256, 0, st, sc, p0, n, Pin, Pout, gidx, sig_in, sig_out, vgrid, sdf,
-                                                             pcell, next, crowded, health, la);
-    else if (learn && sc.count == 1 && la.feat)
-        launch_dep(g2p_kernel<false, kG2PCollect>, grid, 256, 0, st, sc, p0, n, Pin, Pout, gidx, sig_in, sig_out, vgrid, sdf,
-                                                             pcell, next, crowded, health, la);
-    else if (learn && sc.count == 1)
-        launch_dep(g2p_kernel<false, kG2PLarge>, grid, 256, 0, st, sc, p0, n, Pin, Pout, gidx, sig_in, sig_out, vgrid, sdf,
-                                                           pcell, next, crowded, health, la);
-    else if (sc.count == 1 && wide)
-        launch_dep(g2p_kernel<false, kG2PPlain, true>, blocks_for(n, pb), pb, 0, st, sc, p0, n, Pin, Pout, gidx, sig_in,
-                                                                             sig_out, vgrid, sdf, pcell, next, crowded, health, la);
-    else if (sc.count == 1)
-        launch_dep(g2p_kernel<false, kG2PPlain>, blocks_for(n, pb), pb, 0, st, sc, p0, n, Pin, Pout, gidx, sig_in, sig_out,
-                                                                       vgrid, sdf, pcell, next, crowded, health, la);
-    else if (wide)
-        launch_dep(g2p_kernel<true, kG2PPlain, true>, blocks_for(n, pb), pb, 0, st, sc, p0, n, Pin, Pout, gidx, sig_in,
-                                                                            sig_out, vgrid, sdf, pcell, next, crowded, health, la);
-    else {
-        constexpr int k = g2p_per_thread(true, kG2PPlain, false);
-        launch_dep(g2p_kernel<true, kG2PPlain>, blocks_for(n, (long long)pb * k), pb, k * 3 * pb * sizeof(float4), st,
-            sc, p0, n, Pin, Pout, gidx, sig_in, sig_out, vgrid, sdf, pcell, next, crowded, health, la);
-    }
+    // The learned modes work on 256 particles per CTA; the others take 128 too.
+    auto go = [&](auto kernel, int threads, size_t smem) {
+        launch_dep(kernel, blocks_for(n, threads), threads, smem, st, sc, p0, n, Pin, Pout, gidx, edge, sig_in, sig_out,
+                   vgrid, sdf, pcell, next, crowded, health, la);
+    };
+    const int plain = block == 128 ? 128 : 256;
+    if (learn && sc.count == 1 && la.mlp_tc) go(g2p_kernel<false, kG2PLearnedTc>, 256, sizeof(MlpTcSmem));
+    else if (learn && sc.count == 1 && la.mlp) go(g2p_kernel<false, kG2PLearned>, 256, 0);
+    else if (learn && sc.count == 1 && la.feat) go(g2p_kernel<false, kG2PCollect>, 256, 0);
+    else if (learn && sc.count == 1) go(g2p_kernel<false, kG2PLarge>, 256, 0);
+    else if (sc.count == 1) go(g2p_kernel<false, kG2PPlain>, plain, 0);
+    else go(g2p_kernel<true, kG2PPlain>, plain, 0);
     return 1;
 }
 
