@@ -367,8 +367,10 @@ mpm_status mpm_scene_get_sort(mpm_engine* engine, int32_t scene, int32_t* keys_h
  * permutation of those keys (thrust::sequence + thrust::sort_by_key).
  * Positions are three device arrays of n floats.  Work is enqueued on
  * `stream` (a cudaStream_t, NULL = legacy default stream); scratch memory is
- * taken with cudaMallocAsync on that stream and released before return, as
- * the reference allocates its key buffer each call (engine.cu:95,101).
+ * taken in stream order on it and released before return (the reference
+ * allocates its key buffer each call, engine.cu:95,101), from a pool of the
+ * library's that keeps at most 256 MiB between calls and gives it back when an
+ * engine on the device is destroyed.
  * Returns after enqueueing; synchronize the stream before reading. */
 mpm_status mpm_sort_particles_device(const float* d_pos_x, const float* d_pos_y, const float* d_pos_z,
                                      int64_t n, int32_t* d_keys, int32_t* d_perm, void* stream);

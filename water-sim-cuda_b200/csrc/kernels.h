@@ -25,6 +25,8 @@ struct SortScratch {
     int32_t* val_b = nullptr;
     uint32_t* hist = nullptr;    // [256][nb] per-CTA digit counts, scanned in place
     uint32_t* totals = nullptr;  // [256] digit totals of the pass
+    uint32_t* diff = nullptr;    // [nb] bits in which a CTA's keys differ from key 0
+    uint32_t* active = nullptr;  // bit k: pass k runs
     int n = 0;
     int nb = 0;       // CTAs per pass
     int per_cta = 0;  // keys per CTA (multiple of the 2048-key tile)
@@ -35,8 +37,10 @@ size_t sort_scratch_bytes(int n);
 // Points the scratch sub-buffers into `base` (sort_scratch_bytes(n) bytes).
 void sort_scratch_carve(void* base, int n, SortScratch* s);
 
-// keys[i] = Morton key of (px[i], py[i], pz[i]) (setKeys, kernels.cu:361-371).
-int launch_morton_keys(const float* px, const float* py, const float* pz, int n, int32_t* keys, cudaStream_t st);
+// keys[i] = Morton key of (px[i], py[i], pz[i]) (setKeys, kernels.cu:361-371),
+// i < s.n, and their sort permutation as launch_radix_sort writes it.
+int launch_morton_sort(const float* px, const float* py, const float* pz, int32_t* keys, const SortScratch& s,
+                       int32_t* sigma, cudaStream_t st);
 
 // Sorts `keys` (n signed ints, left unchanged) with values 0..n-1, stable, and
 // writes the permutation sigma[j] = index of the j-th smallest key, the

@@ -1,7 +1,7 @@
 // Morton keys + stable sort for callers that cannot allocate device memory.
 //
 // mpm_sort_particles_device takes its radix-sort scratch (ping-pong key and
-// value buffers, per-CTA digit histograms) with cudaMallocAsync on every
+// value buffers, per-CTA digit histograms) from a stream-ordered pool on every
 // call.  Some hosts cannot do that: a process whose device memory is owned
 // by another allocator (a game engine's or a framework's pool that has
 // reserved the memory up front), a real-time frame loop that must not take
@@ -87,14 +87,13 @@ extern "C" mpm_status mpm_sort_particles_device_static(const float* px, const fl
     void* scratch = nullptr;
     mpm_status s = scratch_on_current_device(&scratch);
     if (s != MPM_OK) return s;
-    // Every histogram entry and digit total is written by its pass before it
-    // is read, and the key/value buffers are written before they are read, so
-    // nothing left in the array by an earlier call needs clearing.
+    // Every histogram entry, digit total and pass flag is written by its pass
+    // before it is read, and the key/value buffers are written before they are
+    // read, so nothing left in the array by an earlier call needs clearing.
     mpm::SortScratch plan;
     mpm::sort_scratch_carve(scratch, ni, &plan);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    mpm::launch_morton_keys(px, py, pz, ni, d_keys, st);
-    mpm::launch_radix_sort(d_keys, ni, plan, d_perm, nullptr, nullptr, nullptr, st);
+    mpm::launch_morton_sort(px, py, pz, d_keys, plan, d_perm, st);
     const cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return cuda_fail(err, "static sort launch");
     return MPM_OK;

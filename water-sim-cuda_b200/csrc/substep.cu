@@ -21,6 +21,7 @@
 #include <cstdint>
 
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace mpm {
 namespace {
@@ -58,13 +59,6 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
-
-// Programmatic dependent launch: the substep's kernels are launched with
-// programmatic stream serialisation (launch_dep), so that a kernel's CTAs are
-// scheduled while its predecessor drains; each such kernel waits here, before
-// touching memory, until its predecessor has completed and its writes are
-// visible (griddepcontrol.wait; a no-op for an ordinary launch).
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Files this lane's particle under global cell `gcell` (global bin `gbin`) of
 // a counter set: one reduction per distinct cell of the warp and one per
@@ -1452,23 +1446,6 @@ __global__ void __launch_bounds__(256) copy_words_kernel(uint32_t* __restrict__ 
 }
 
 inline int blocks_for(long long n, int t) { return (int)((n + t - 1) / t); }
-
-// Launches a substep kernel (one that starts with pdl_wait) with programmatic
-// stream serialisation.
-template <typename... P, typename... A>
-void launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-}
 
 }  // namespace
 
