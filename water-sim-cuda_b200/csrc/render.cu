@@ -71,10 +71,14 @@ __device__ __forceinline__ float ord_dec(unsigned u) {
     return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
-// One thread per particle: the pixels of its sprite.
-__global__ void splat_kernel(const float* __restrict__ xyz, long long n, Cam c, unsigned* __restrict__ zbuf) {
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// One thread per particle: the pixels of its sprite.  Most fragments lie behind
+// one that is there already: a plain load (through L1; a stale value is only
+// smaller) drops those before the atomic.  Particles go last to first, since
+// scenes are seeded with z ascending and the default camera looks down -z, so
+// that near ones mostly come first.  2M particles, 1920 x 1600: 1064 -> 401 us.
+__global__ void splat_kernel(const float* __restrict__ xyz, long long n, Cam c, unsigned* zbuf) {
+    const long long i = n - 1 - (blockIdx.x * (long long)blockDim.x + threadIdx.x);
+    if (i < 0) return;
     const float x = xyz[i * 3], y = xyz[i * 3 + 1], z = xyz[i * 3 + 2];
     const float vx = c.m[0] * x + c.m[4] * y + c.m[8] * z + c.m[12];
     const float vy = c.m[1] * x + c.m[5] * y + c.m[9] * z + c.m[13];
@@ -97,8 +101,9 @@ __global__ void splat_kernel(const float* __restrict__ xyz, long long n, Cam c, 
             const float nx2 = s * 2.0f - 1.0f;
             const float r2 = nx2 * nx2 + ny2 * ny2;
             if (r2 > 1.0f) continue;
-            const float zz = vz + sqrtf(1.0f - r2) * c.radius;
-            atomicMax(zbuf + (size_t)py * c.w + px, ord_enc(zz));
+            const unsigned zz = ord_enc(vz + sqrtf(1.0f - r2) * c.radius);
+            unsigned* at = zbuf + (size_t)py * c.w + px;
+            if (*at < zz) atomicMax(at, zz);
         }
     }
 }
@@ -244,9 +249,24 @@ __global__ void obstacle_resolve_kernel(const unsigned long long* __restrict__ k
     odepth[i] = __uint_as_float((unsigned)(k >> 32));
 }
 
+// A colour component as the 8-bit framebuffer stores it (the same single
+// roundings on host and device; NaN gives 0 on both).
+__host__ __device__ inline unsigned char unorm8(float f) {
+    f = f < 0.0f ? 0.0f : (f > 1.0f ? 1.0f : f);
+    return f == f ? (unsigned char)floorf(f * 255.0f + 0.5f) : (unsigned char)0;
+}
+
+// The float image and its 8-bit copy: converting 9.2M components of a 1920 x
+// 1600 image on the host took 17 ms of a read-back.
+__device__ __forceinline__ void store_pixel(float* __restrict__ rgb, unsigned char* __restrict__ rgb8, size_t i, float v) {
+    rgb[i] = v;
+    rgb8[i] = unorm8(v);
+}
+
 __global__ void composite_kernel(const float* __restrict__ depth, const unsigned char* __restrict__ bg, int w, int h,
                                  float p00, float p11, float p22, float p32, float lx, float ly, float lz,
-                                 const float* __restrict__ odepth, float* __restrict__ rgb) {
+                                 const float* __restrict__ odepth, float* __restrict__ rgb,
+                                 unsigned char* __restrict__ rgb8) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= w || y >= h) return;
     const size_t o = ((size_t)y * w + x) * 3;
@@ -256,7 +276,7 @@ __global__ void composite_kernel(const float* __restrict__ depth, const unsigned
     // keeps the background
     const bool hidden = odepth && !(((p22 * d + p32) / -d) * 0.5f + 0.5f < odepth[(size_t)y * w + x]);
     if (d > 5000.0f || hidden) {
-        for (int c = 0; c < 3; ++c) rgb[o + c] = bg[o + c] / 255.0f;
+        for (int c = 0; c < 3; ++c) store_pixel(rgb, rgb8, o + c, bg[o + c] / 255.0f);
         return;
     }
     const float3 pc = view_pos(depth, w, h, x, y, p00, p11);
@@ -277,12 +297,7 @@ __global__ void composite_kernel(const float* __restrict__ depth, const unsigned
     const float a = 0.3f + fres * 0.5f;
     const float wc[3] = {0.1f, 0.5f, 0.8f};
     const float bc[3] = {b.x, b.y, b.z};
-    for (int c = 0; c < 3; ++c) rgb[o + c] = bc[c] * (1.0f - a) + wc[c] * a + spec;
-}
-
-inline unsigned char unorm8(float f) {
-    f = f < 0.0f ? 0.0f : (f > 1.0f ? 1.0f : f);
-    return (unsigned char)std::floor(f * 255.0f + 0.5f);
+    for (int c = 0; c < 3; ++c) store_pixel(rgb, rgb8, o + c, bc[c] * (1.0f - a) + wc[c] * a + spec);
 }
 
 // glm::lookAt / perspective / translate / rotate restated (column-major).
@@ -327,6 +342,7 @@ struct mpm_renderer {
     float* tmp = nullptr;    // after the horizontal blur
     float* fin = nullptr;    // after the vertical blur
     float* rgb = nullptr;
+    unsigned char* rgb8 = nullptr;     // rgb as the framebuffer's 8 bits
     unsigned char* bg = nullptr;       // the background texture: base + obstacles
     unsigned char* base = nullptr;     // clear colour or the caller's image
     float* odepth = nullptr;           // obstacles' window depth; null without obstacles
@@ -449,6 +465,7 @@ mpm_status mpm_renderer_create(const mpm_render_params* params, int32_t device, 
     if (err == cudaSuccess) err = cudaMalloc(&r->tmp, npix * sizeof(float));
     if (err == cudaSuccess) err = cudaMalloc(&r->fin, npix * sizeof(float));
     if (err == cudaSuccess) err = cudaMalloc(&r->rgb, npix * 3 * sizeof(float));
+    if (err == cudaSuccess) err = cudaMalloc(&r->rgb8, npix * 3);
     if (err == cudaSuccess) err = cudaMalloc(&r->bg, npix * 3);
     if (err == cudaSuccess) err = cudaMalloc(&r->base, npix * 3);
     if (err != cudaSuccess) {
@@ -468,7 +485,7 @@ mpm_status mpm_renderer_create(const mpm_render_params* params, int32_t device, 
 void mpm_renderer_destroy(mpm_renderer* r) {
     if (!r) return;
     cudaSetDevice(r->device);
-    for (void* p : {(void*)r->zbuf, (void*)r->depth, (void*)r->tmp, (void*)r->fin, (void*)r->rgb, (void*)r->bg,
+    for (void* p : {(void*)r->zbuf, (void*)r->depth, (void*)r->tmp, (void*)r->fin, (void*)r->rgb, (void*)r->rgb8, (void*)r->bg,
                     (void*)r->base, (void*)r->odepth, (void*)r->okey, (void*)r->otris, (void*)r->ocolor})
         if (p) cudaFree(p);
     delete r;
@@ -589,7 +606,7 @@ mpm_status mpm_render_points(mpm_renderer* r, const float* xyz_device, int64_t n
     blur_kernel<<<grd, blk, 0, st>>>(r->depth, r->tmp, w, h, 1, 0, r->prm.filter_size, r->prm.depth_falloff);
     blur_kernel<<<grd, blk, 0, st>>>(r->tmp, r->fin, w, h, 0, 1, r->prm.filter_size, r->prm.depth_falloff);
     composite_kernel<<<grd, blk, 0, st>>>(r->fin, r->bg, w, h, r->cam.p00, r->cam.p11, r->cam.p22, r->cam.p32,
-                                          r->light[0], r->light[1], r->light[2], r->odepth, r->rgb);
+                                          r->light[0], r->light[1], r->light[2], r->odepth, r->rgb, r->rgb8);
     RK(r, cudaGetLastError());
     return MPM_OK;
 }
@@ -617,15 +634,8 @@ mpm_status mpm_renderer_get_image(mpm_renderer* r, float* rgb_host, uint8_t* rgb
     RK(r, cudaSetDevice(r->device));
     RK(r, cudaDeviceSynchronize());
     const size_t npix = (size_t)r->prm.width * r->prm.height;
-    std::vector<float> tmp;
-    float* dst = rgb_host;
-    if (!dst) {
-        tmp.resize(npix * 3);
-        dst = tmp.data();
-    }
-    RK(r, cudaMemcpy(dst, r->rgb, npix * 3 * sizeof(float), cudaMemcpyDeviceToHost));
-    if (rgb8_host)
-        for (size_t i = 0; i < npix * 3; ++i) rgb8_host[i] = unorm8(dst[i]);
+    if (rgb_host) RK(r, cudaMemcpy(rgb_host, r->rgb, npix * 3 * sizeof(float), cudaMemcpyDeviceToHost));
+    if (rgb8_host) RK(r, cudaMemcpy(rgb8_host, r->rgb8, npix * 3, cudaMemcpyDeviceToHost));
     return MPM_OK;
 }
 
