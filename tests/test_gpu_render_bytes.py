@@ -15,7 +15,7 @@ def test_bytes_and_order(gpu_ok, mpm, size, n):
     pos = (np.array([10.0, 8.0, 4.0]) + rng.random((n, 3)) * np.array([24.0, 20.0, 30.0])).astype(np.float32)
     seen = []
     for order in (slice(None), slice(None, None, -1), rng.permutation(n)):
-        d = torch.from_numpy(np.ascontiguousarray(pos[order])).cuda()
+        d = torch.from_numpy(pos[order].copy()).cuda()
         with mpm.Renderer((48, 40, 44), *size, light_dir=(0.1, 0.2, 1.0)) as r:
             r.render_device(d.data_ptr() if n else 0, n)
             f, b = r.image()
