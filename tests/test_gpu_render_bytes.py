@@ -21,6 +21,9 @@ def test_bytes_and_order(gpu_ok, mpm, size, n):
             f, b = r.image()
             seen.append((r.depth(0), f, b))
     for depth, f, b in seen:
-        assert np.array_equal(depth, seen[0][0]) and np.array_equal(f, seen[0][1]) and np.array_equal(b, seen[0][2])
+        # (a 1 x 1 image has no neighbour to take a normal from: NaN, byte 0)
+        assert np.array_equal(depth, seen[0][0]) and np.array_equal(f, seen[0][1], equal_nan=True)
+        assert np.array_equal(b, seen[0][2])
+    f = np.where(np.isnan(f), np.float32(0), f)
     want = np.floor(np.clip(f, np.float32(0), np.float32(1)) * np.float32(255) + np.float32(0.5)).astype(np.uint8)
     assert np.array_equal(b, want)

@@ -16,6 +16,7 @@
 
 #include "../../include/mpm_b200.h"
 #include "corrector_tc_train.cuh"
+#include "launch.cuh"
 #include "kernels.h"
 
 namespace mpm {
@@ -385,10 +386,42 @@ __global__ void __launch_bounds__(kTrainThreads) mlp_train_kernel(
     if ((tid & 31) == 0) atomicAdd(loss, lsum * inv_count);
 }
 
-// Adam on the trained parameters; zeroes the gradient.
+// Trained parameter i (value v) into its places of the packed weights.
+__device__ __forceinline__ void train_pack_one(MlpTrainW* __restrict__ t, int i, float v) {
+    const __nv_bfloat16 b = __float2bfloat16_rn(v);
+    if (i < kPB1) {
+        t->w1[canon_index((i - kPW1) / 16, (i - kPW1) % 16, 16)] = b;
+    } else if (i < kPW2) {
+        t->b1[i - kPB1] = v;
+    } else if (i < kPB2) {
+        const int u = (i - kPW2) / 64, k = (i - kPW2) % 64;
+        t->w2[canon_index(u, k, 64)] = b;
+        t->w2t[canon_index(k, u, 64)] = b;
+    } else if (i < kPW3) {
+        t->b2[i - kPB2] = v;
+    } else if (i < kPB3) {
+        const int o = (i - kPW3) / 64, k = (i - kPW3) % 64;
+        t->w3[canon_index(o, k, 64)] = b;
+        t->w3t[canon_index(k, o, 16)] = b;
+    } else {
+        t->b3[i - kPB3] = v;
+    }
+}
+
+// All packed weights (their padding is zeroed once, when they are allocated).
+__global__ void train_pack_kernel(const float* __restrict__ w, MlpTrainW* __restrict__ t) {
+    const int i = kPTrainFirst + blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < kPCount) train_pack_one(t, i, w[i]);
+}
+
+// Adam on the trained parameters; zeroes the gradient and packs the new
+// weights for the next step.  Its trigger lets that step's CTAs start on what
+// does not depend on them.
 __global__ void adam_kernel(float* __restrict__ w, float* __restrict__ grad, float* __restrict__ m1,
-                            float* __restrict__ m2, float lr, float beta1, float beta2, float eps, float bc1,
-                            float bc2) {
+                            float* __restrict__ m2, MlpTrainW* __restrict__ packed, float lr, float beta1, float beta2,
+                            float eps, float bc1, float bc2) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    pdl_wait();
     const int i = kPTrainFirst + blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= kPCount) return;
     const float g = grad[i];
@@ -397,41 +430,44 @@ __global__ void adam_kernel(float* __restrict__ w, float* __restrict__ grad, flo
     const float b = beta2 * m2[i] + (1.0f - beta2) * g * g;
     m1[i] = a;
     m2[i] = b;
-    w[i] -= lr * (a / bc1) / (sqrtf(b / bc2) + eps);
+    const float v = w[i] - lr * (a / bc1) / (sqrtf(b / bc2) + eps);
+    w[i] = v;
+    train_pack_one(packed, i, v);
+}
+
+// Four consecutive gradient entries at once (16-byte aligned: kGradPad).
+__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
 // The training gradient on tcgen05 (corrector_tc_train.cuh): the loss and
 // batch of mlp_train_kernel, tiles of 128 samples, rows at or beyond `batch`
 // masked by dY = 0.  A bounded wait that gives up sets kStatusTimeout in
 // *status and the CTA adds nothing to the gradient.
-__global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(
-    const float* __restrict__ w, const float* __restrict__ feat, const float* __restrict__ targ, long long size,
-    const long long* __restrict__ idx_list, int batch, unsigned long long seed, int step, float* __restrict__ grad,
-    float* __restrict__ loss, uint32_t* __restrict__ status) {
+__global__ void __launch_bounds__(kTrThreads, 2) mlp_train_tc_kernel(
+    const float* __restrict__ w, const MlpTrainW* __restrict__ packed, const float* __restrict__ feat,
+    const float* __restrict__ targ, long long size, const long long* __restrict__ idx_list, int batch,
+    unsigned long long seed, int step, float* __restrict__ grad, float* __restrict__ loss, uint32_t* __restrict__ status) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     MlpTrainSmem& s = *reinterpret_cast<MlpTrainSmem*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, wq = (tid >> 5) & 3, ch = 32 * (tid >> 7);
     const int srow = 32 * wq + lane;  // this thread's sample row in the epilogues
-    // Weights, their transposed copies, and the zero padding of dY and dZ^T.
-    for (int i = tid; i < 64 * 16; i += kTrThreads)
-        s.w.w1[canon_index(i / 16, i % 16, 16)] = __float2bfloat16_rn(w[kPW1 + i]);
-    for (int i = tid; i < 64 * 64; i += kTrThreads) {
-        const int u = i / 64, k = i % 64;
-        const __nv_bfloat16 v = __float2bfloat16_rn(w[kPW2 + i]);
-        s.w.w2[canon_index(u, k, 64)] = v;
-        s.w.w2t[canon_index(k, u, 64)] = v;
-    }
-    for (int i = tid; i < 16 * 64; i += kTrThreads) {
-        const int o = i / 64, k = i % 64;
-        const __nv_bfloat16 v = __float2bfloat16_rn(o < kMlpOut ? w[kPW3 + o * 64 + k] : 0.f);
-        s.w.w3[canon_index(o, k, 64)] = v;
-        s.w.w3t[canon_index(k, o, 16)] = v;
-    }
-    if (tid < 64) s.w.b1[tid] = w[kPB1 + tid], s.w.b2[tid] = w[kPB2 + tid];
-    if (tid < 4) s.w.b3[tid] = tid < kMlpOut ? w[kPB3 + tid] : 0.f;
+    const int ntiles = (batch + kTrTile - 1) / kTrTile;
+    // Loading a tile: two threads per sample, eight features each.
+    const int lrow = tid >> 1, lk = (tid & 1) * 8;
+    auto sample = [&](int tile) {
+        const long long i = (long long)tile * kTrTile + lrow;
+        return i >= batch ? 0ll : (idx_list ? idx_list[i] : sample_index(seed, 0x7A11ull + (unsigned long long)step, i, size));
+    };
+    // Before the wait for the weights: the zero padding of dY, TMEM, and the
+    // CTA's samples on their way into L2 (the indices are drawn at random from
+    // a dataset of gigabytes).
     for (int i = tid; i < (int)(sizeof(s.dy) / 16); i += kTrThreads) reinterpret_cast<uint4*>(s.dy)[i] = uint4{0, 0, 0, 0};
-    for (int i = tid; i < (int)(sizeof(s.dzt) / 16); i += kTrThreads)
-        reinterpret_cast<uint4*>(s.dzt)[i] = uint4{0, 0, 0, 0};
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const long long j = sample(tile);
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(feat + j * kMlpIn + lk));
+        if (lk == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(targ + j * kMlpOut));
+    }
     if (tid < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s.tmem)),
                      "r"(kTrTmemCols)
@@ -443,6 +479,9 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(
         s.failed = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    pdl_wait();
+    for (int i = tid; i < (int)(sizeof(MlpTrainW) / 16); i += kTrThreads)
+        reinterpret_cast<uint4*>(&s.w)[i] = __ldg(reinterpret_cast<const uint4*>(packed) + i);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -452,25 +491,23 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(
     float gW3 = 0.f, gB3 = 0.f, gB2 = 0.f, gB1 = 0.f, lsum = 0.f;
     uint32_t phase = 0;
     bool any = false;
-    const int ntiles = (batch + kTrTile - 1) / kTrTile;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        if (tid < kTrTile) {
-            const long long i = (long long)tile * kTrTile + tid;
-            long long j = 0;
-            if (i < batch) j = idx_list ? idx_list[i] : sample_index(seed, 0x7A11ull + (unsigned long long)step, i, size);
-            s.sidx[tid] = j;
-        }
-        __syncthreads();
-        for (int e = tid; e < kTrTile * kMlpIn; e += kTrThreads) {
-            const int r = e >> 4, k = e & 15;
-            const __nv_bfloat16 v =
-                __float2bfloat16_rn((feat[s.sidx[r] * kMlpIn + k] - w[kPInMean + k]) * w[kPInInvStd + k]);
-            s.x[canon_index(r, k, 16)] = v;
-            s.xt[canon_index(k, r, kTrTile)] = v;
-        }
-        for (int e = tid; e < kTrTile * kMlpOut; e += kTrThreads) {
-            const int r = e / kMlpOut, o = e % kMlpOut;
-            s.dyf[r * 4 + o] = targ[s.sidx[r] * kMlpOut + o] / w[kPOutStd + o];
+        {
+            const long long j = sample(tile);
+            const float4* row = reinterpret_cast<const float4*>(feat + j * kMlpIn + lk);
+            const float4 fa = __ldg(row), fb = __ldg(row + 1);
+            const float fv[8] = {fa.x, fa.y, fa.z, fa.w, fb.x, fb.y, fb.z, fb.w};
+            uint4 packed_row;
+            __nv_bfloat16* v = reinterpret_cast<__nv_bfloat16*>(&packed_row);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                v[k] = __float2bfloat16_rn((fv[k] - __ldg(w + kPInMean + lk + k)) * __ldg(w + kPInInvStd + lk + k));
+                s.xt[canon_index(lk + k, lrow, kTrTile)] = v[k];
+            }
+            *reinterpret_cast<uint4*>(s.x + canon_index(lrow, lk, 16)) = packed_row;
+            if (lk == 0)
+#pragma unroll
+                for (int o = 0; o < kMlpOut; ++o) s.dyf[lrow * 4 + o] = __ldg(targ + j * kMlpOut + o) / __ldg(w + kPOutStd + o);
         }
         // Z1 = X W1^T.
         mlp_tr_publish();
@@ -563,7 +600,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(
                 v[j] *= g2[j];
                 v[j + 1] *= g2[j + 1];
                 const __nv_bfloat162 d = __floats2bfloat162_rn(v[j], v[j + 1]);
-                *reinterpret_cast<__nv_bfloat162*>(s.dz + canon_index(srow, u, 64)) = d;
+                *reinterpret_cast<__nv_bfloat162*>(s.h2 + canon_index(srow, u, 64)) = d;  // dZ2
                 s.dzt[canon_index(u, srow, kTrTile)] = d.x;
                 s.dzt[canon_index(u + 1, srow, kTrTile)] = d.y;
             }
@@ -572,7 +609,7 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(
         // dH1 = dZ2 W2 and dW2 += dZ2^T H1.
         mlp_tr_publish();
         if (tid == 0) {
-            mlp_tr_mma(tm + kTrColZ2, s.dz, s.w.w2t, 64, 64, false);
+            mlp_tr_mma(tm + kTrColZ2, s.h2, s.w.w2t, 64, 64, false);
             mlp_tr_mma(tm + kTrColDW2, s.dzt, s.h1t, 64, kTrTile, any);
             umma_commit(&s.mbar);
         }
@@ -608,12 +645,13 @@ __global__ void __launch_bounds__(kTrThreads, 1) mlp_train_tc_kernel(
             float v[32];
             tmem_ld32(trow + kTrColDW2 + (uint32_t)ch, v);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) atomicAdd(grad + kPW2 + u * 64 + ch + j, v[j]);
+            for (int j = 0; j < 32; j += 4) red_add_v4(grad + kPW2 + u * 64 + ch + j, v[j], v[j + 1], v[j + 2], v[j + 3]);
             if (ch == 0) {
                 float v16[16];
                 tmem_ld16(trow + kTrColDW1, v16);
 #pragma unroll
-                for (int i = 0; i < kMlpIn; ++i) atomicAdd(grad + kPW1 + u * kMlpIn + i, v16[i]);
+                for (int i = 0; i < kMlpIn; i += 4)
+                    red_add_v4(grad + kPW1 + u * kMlpIn + i, v16[i], v16[i + 1], v16[i + 2], v16[i + 3]);
             }
         }
         atomicAdd(grad + kPB2 + ch + lane, gB2);
@@ -675,7 +713,9 @@ struct mpm_corrector {
     float* feat = nullptr;   // [capacity][16]
     float* targ = nullptr;   // [capacity][3]
     float* w = nullptr;      // [kPCount] master parameters
+    float* grad_mem = nullptr;  // grad starts kGradPad floats in
     float* grad = nullptr;   // [kPCount]
+    mpm::MlpTrainW* train_w = nullptr;  // packed weights of the tcgen05 training step
     float* m1 = nullptr;     // Adam moments
     float* m2 = nullptr;
     float* loss = nullptr;   // [1]
@@ -778,7 +818,10 @@ mpm_status mpm_corrector_create(int32_t device, int64_t capacity, mpm_corrector*
     CA(cudaMalloc(&c->feat, cap * mpm::kMlpIn * sizeof(float)));
     CA(cudaMalloc(&c->targ, cap * mpm::kMlpOut * sizeof(float)));
     CA(cudaMalloc(&c->w, mpm::kPCount * sizeof(float)));
-    CA(cudaMalloc(&c->grad, mpm::kPCount * sizeof(float)));
+    CA(cudaMalloc(&c->grad_mem, (mpm::kPCount + mpm::kGradPad) * sizeof(float)));
+    c->grad = c->grad_mem + mpm::kGradPad;
+    CA(cudaMalloc(&c->train_w, sizeof(mpm::MlpTrainW)));
+    CA(cudaMemsetAsync(c->train_w, 0, sizeof(mpm::MlpTrainW), c->stream));
     CA(cudaMalloc(&c->m1, mpm::kPCount * sizeof(float)));
     CA(cudaMalloc(&c->m2, mpm::kPCount * sizeof(float)));
     CA(cudaMalloc(&c->loss, sizeof(float)));
@@ -805,7 +848,7 @@ void mpm_corrector_destroy(mpm_corrector* c) {
     if (!c) return;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    for (void* p : {(void*)c->feat, (void*)c->targ, (void*)c->w, (void*)c->grad, (void*)c->m1, (void*)c->m2,
+    for (void* p : {(void*)c->feat, (void*)c->targ, (void*)c->w, (void*)c->grad_mem, (void*)c->train_w, (void*)c->m1, (void*)c->m2,
                     (void*)c->loss, (void*)c->mom, (void*)c->idx, (void*)c->packed, (void*)c->io,
                     (void*)c->packed_tc, (void*)c->status})
         if (p) cudaFree(p);
@@ -923,9 +966,9 @@ mpm_status launch_train(mpm_corrector* c, int batch, const long long* idx, unsig
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
     if (c->train_kind == MPM_TRAIN_TCGEN05) {
         const int tiles = (batch + mpm::kTrTile - 1) / mpm::kTrTile;
-        const int grid = std::max(1, std::min(tiles, sms));
-        mpm::mlp_train_tc_kernel<<<grid, mpm::kTrThreads, sizeof(mpm::MlpTrainSmem), c->stream>>>(
-            c->w, c->feat, c->targ, c->size, idx, batch, seed, step, c->grad, c->loss, c->status);
+        const int grid = std::max(1, std::min(tiles, 2 * sms));
+        mpm::launch_dep(mpm::mlp_train_tc_kernel, grid, mpm::kTrThreads, sizeof(mpm::MlpTrainSmem), c->stream, c->w,
+                        c->train_w, c->feat, c->targ, c->size, idx, batch, seed, step, c->grad, c->loss, c->status);
         CC(c, cudaGetLastError());
         return MPM_OK;
     }
@@ -960,14 +1003,15 @@ mpm_status mpm_corrector_train(mpm_corrector* c, int32_t steps, int32_t batch, f
     CC(c, cudaMemsetAsync(c->status, 0, sizeof(uint32_t), c->stream));
     const float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
     const int ntrain = mpm::kPCount - mpm::kPTrainFirst;
+    mpm::train_pack_kernel<<<mpm::blocks_of(ntrain, 256), 256, 0, c->stream>>>(c->w, c->train_w);
     for (int i = 0; i < steps; ++i) {
         st = launch_train(c, batch, nullptr, seed, c->adam_t);
         if (st != MPM_OK) return st;
         ++c->adam_t;
         const float bc1 = 1.0f - (float)std::pow((double)beta1, c->adam_t);
         const float bc2 = 1.0f - (float)std::pow((double)beta2, c->adam_t);
-        mpm::adam_kernel<<<mpm::blocks_of(ntrain, 256), 256, 0, c->stream>>>(c->w, c->grad, c->m1, c->m2, lr, beta1,
-                                                                         beta2, eps, bc1, bc2);
+        mpm::launch_dep(mpm::adam_kernel, mpm::blocks_of(ntrain, 256), 256, 0, c->stream, c->w, c->grad, c->m1, c->m2,
+                        c->train_w, lr, beta1, beta2, eps, bc1, bc2);
         CC(c, cudaGetLastError());
     }
     float loss = 0.f;
@@ -997,6 +1041,7 @@ mpm_status mpm_corrector_gradient(mpm_corrector* c, int64_t count, const int64_t
     CC(c, cudaMemsetAsync(c->grad, 0, mpm::kPCount * sizeof(float), c->stream));
     CC(c, cudaMemsetAsync(c->loss, 0, sizeof(float), c->stream));
     CC(c, cudaMemsetAsync(c->status, 0, sizeof(uint32_t), c->stream));
+    mpm::train_pack_kernel<<<mpm::blocks_of(mpm::kPCount - mpm::kPTrainFirst, 256), 256, 0, c->stream>>>(c->w, c->train_w);
     st = launch_train(c, (int)count, c->idx, 0, 0);
     if (st != MPM_OK) return st;
     if (grad_host)

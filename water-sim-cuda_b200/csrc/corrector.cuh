@@ -40,6 +40,10 @@ enum MlpParam : int {
     kPCount = kPB3 + kMlpOut,                  // 5478
     kPTrainFirst = kPW1                        // parameters trained: [kPW1, kPCount)
 };
+// Floats before the device gradient: its W1 and W2 then start on 16-byte
+// boundaries.
+constexpr int kGradPad = 1;
+static_assert((kPW1 + kGradPad) % 4 == 0 && (kPW2 + kGradPad) % 4 == 0, "vector reductions into W1 and W2");
 
 // Inference copy: weights as bf16 mma.m16n8k16 B fragments in lane order (one
 // 8-byte load per lane and fragment, conflict-free from shared memory), fp32

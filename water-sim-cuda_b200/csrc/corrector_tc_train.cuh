@@ -1,6 +1,12 @@
 // Training step of the corrector MLP on the 5th-generation tensor cores.
 //
-// A persistent CTA of 256 threads takes tiles of 128 samples.  Per tile,
+// Persistent CTAs of 256 threads, two per SM, take tiles of 128 samples.  A
+// tile is a chain of six MMA rounds with an epilogue after each, so a CTA alone
+// leaves the SM waiting; the second one fills those gaps (registers, 102 KB of
+// shared memory and 256 TMEM columns each allow two).  Measured at 65,536
+// samples: 60.6 us per gradient with one CTA per SM that also packed the
+// weights and added its sums entry by entry, 37.8 us now; the chain of a tile
+// (about 12 us) still bounds it, 1.73 tiles per CTA.  Per tile,
 // every GEMM is a tcgen05.mma with bf16 operands in shared memory in the
 // canonical K-major layout of corrector_tc.cuh and fp32 accumulators in TMEM:
 //
@@ -27,9 +33,10 @@
 
 namespace mpm {
 
-// Weights of a training step in the canonical layout, staged by each CTA
-// from the fp32 master parameters.
-struct MlpTrainW {
+// Weights of a training step in the canonical layout: rounded from the fp32
+// master parameters once per step (by the Adam kernel that updates them) and
+// copied in by each CTA.
+struct alignas(16) MlpTrainW {
     __nv_bfloat16 w1[64 * 16];   // [u][i]   Z1 = X W1^T
     __nv_bfloat16 w2[64 * 64];   // [u][k]   Z2 = H1 W2^T
     __nv_bfloat16 w3[16 * 64];   // [o][k]   Y = H2 W3^T (rows 3..15 zero)
@@ -43,26 +50,30 @@ struct MlpTrainW {
 constexpr int kTrTile = 128;
 constexpr int kTrThreads = 256;
 // TMEM columns: Z1, then dH2 [0, 64); Z2, then dH1 [64, 128); Y [128, 144);
-// dW2 [256, 320); dW1 [320, 336).
-constexpr int kTrTmemCols = 512;
-constexpr uint32_t kTrColZ1 = 0, kTrColZ2 = 64, kTrColY = 128, kTrColDW2 = 256, kTrColDW1 = 320;
+// dW1 [144, 160); dW2 [160, 224).
+constexpr int kTrTmemCols = 256;
+constexpr uint32_t kTrColZ1 = 0, kTrColZ2 = 64, kTrColY = 128, kTrColDW1 = 144, kTrColDW2 = 160;
 
 struct MlpTrainSmem {
     MlpTrainW w;
     __nv_bfloat16 x[kTrTile * 16];     // [s][i]
     __nv_bfloat16 xt[16 * kTrTile];    // [i][s]
+    // H2 [s][k]; dZ2 [s][u] takes its place once dH2 has been waited for (the
+    // output layer's gradients have been summed by then).
+    __nv_bfloat16 h2[kTrTile * 64];
+    __nv_bfloat16 dy[kTrTile * 16];    // [s][o], columns 3..15 zero
+    // dZ2^T, then dZ1^T: [u][s].  The MMAs that read it take 128 rows, the 64
+    // units and whatever follows (h1): accumulator rows 64..127 are not read.
+    __nv_bfloat16 dzt[64 * kTrTile];
     __nv_bfloat16 h1[kTrTile * 64];    // [s][k]
     __nv_bfloat16 h1t[64 * kTrTile];   // [k][s]
-    __nv_bfloat16 h2[kTrTile * 64];    // [s][k]
-    __nv_bfloat16 dy[kTrTile * 16];    // [s][o], columns 3..15 zero
-    __nv_bfloat16 dz[kTrTile * 64];    // dZ2 [s][u]
-    __nv_bfloat16 dzt[128 * kTrTile];  // dZ2^T, then dZ1^T: [u][s], rows 64..127 zero
     float dyf[kTrTile * 4];            // targets, then dY (fp32)
-    long long sidx[kTrTile];
     unsigned long long mbar;
     uint32_t tmem;
     uint32_t failed;
 };
+
+static_assert(sizeof(MlpTrainW) % 16 == 0 && sizeof(MlpTrainSmem) <= 112 * 1024, "two CTAs per SM");
 
 #if defined(__CUDACC__)
 
