@@ -240,10 +240,17 @@ __device__ __forceinline__ void mlp_tc_hidden(MlpTcSmem& s, const float* bias) {
     for (int c0 = 0; c0 < 64; c0 += 16) {
         float v[16];
         tmem_ld16(taddr + (uint32_t)c0, v);
+        // Eight values make one 16-byte row of a core matrix.
 #pragma unroll
-        for (int i = 0; i < 16; i += 2) {
-            const float g0 = gelu_tanh(v[i] + bias[c0 + i]), g1 = gelu_tanh(v[i + 1] + bias[c0 + i + 1]);
-            *reinterpret_cast<__nv_bfloat162*>(a + canon_index(r, c0 + i, 64)) = __floats2bfloat162_rn(g0, g1);
+        for (int i = 0; i < 16; i += 8) {
+            uint32_t h[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float2 g = gelu_tanh2(make_float2(v[i + 2 * q], v[i + 2 * q + 1]),
+                                            *reinterpret_cast<const float2*>(bias + c0 + i + 2 * q));
+                h[q] = pack_bf16x2(g.x, g.y);
+            }
+            *reinterpret_cast<uint4*>(a + canon_index(r, c0 + i, 64)) = make_uint4(h[0], h[1], h[2], h[3]);
         }
     }
 }

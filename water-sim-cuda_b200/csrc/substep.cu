@@ -950,7 +950,9 @@ constexpr int kStagePlanes = 9;  // planes of 60 nodes: 8.6 KB per CTA
 // CTAs per SM: the learned tcgen05 mode fits four (64 registers, 128 TMEM
 // columns and about 45 KB of shared memory each), so one CTA's MMA waits
 // overlap the other three's work; mma.sync learned, collect and batched
-// modes need more registers.
+// modes need more registers.  The tcgen05 mode at 2M particles: 330 us with
+// per-warp statistics, node-by-node sums and scalar GELU, 225 us now (three
+// CTAs of 80 registers without spills: 254 against 243 us before the row sums).
 template <bool kBatch, int kMode>
 __global__ void __launch_bounds__(256, kMode == 1 ? 2 : ((kBatch || kMode == 2) ? 3 : 4)) g2p_kernel(
     SceneTable sc, SimParams p0, long long n_total, const float* __restrict__ Pin, float* __restrict__ Pout,
@@ -966,6 +968,7 @@ __global__ void __launch_bounds__(256, kMode == 1 ? 2 : ((kBatch || kMode == 2) 
     __shared__ __align__(16) unsigned char s_mlp_raw[kMode == kG2PLearned ? sizeof(MlpPacked) : 16];
     __shared__ uint32_t s_stage[kMode == kG2PLearned ? 8 * 32 * kMlpStageStride : 1];
     __shared__ float4 s_node_own[kMode == kG2PLearnedTc ? 1 : kStagePlanes * kFootPlane];
+    __shared__ float s_dev[kMode == kG2PLearned || kMode == kG2PLearnedTc ? 3 : 1][8];  // the warps' statistic sums
     extern __shared__ __align__(1024) unsigned char s_dyn[];  // MlpTcSmem in the tcgen05 mode
     if constexpr (kMode == kG2PLearned) {
         const uint4* src = reinterpret_cast<const uint4*>(la.mlp);
@@ -1050,16 +1053,12 @@ __global__ void __launch_bounds__(256, kMode == 1 ? 2 : ((kBatch || kMode == 2) 
     axis_weights(fx, 1.0f, wx);
     axis_weights(fy, 1.0f, wy);
     axis_weights(fz, 1.0f, wz);
-    // Interpolation sums (g2PTransfer's loop, kernels.cu:214-235).  The plain,
-    // large and collection modes take them separably per axis: with o =
-    // (a, b, c) the node offset and x_node - x_p = (o - 1) - (f - 1),
+    // Interpolation sums (g2PTransfer's loop, kernels.cu:214-235), separably
+    // per axis: with o = (a, b, c) the node offset and x_node - x_p = (o - 1) - (f - 1),
     //   v' = sum w v,   C' = 4 (M - v' (f - 1)^T),   M[k][d] = sum w v_k (o_d - 1),
     // each row of three nodes along x reduced first (S0 = sum_a wx v, S1 =
     // sum_a wx (a - 1) v) before its weight wy wz is applied: a quarter fewer
-    // instructions.  The learned modes sum node by node (the reference's
-    // form), which holds fewer values live next to the MLP's registers: the
-    // row form made the tcgen05 learned G2P spill three times as much and run
-    // 7 % slower.
+    // instructions than node by node.
     float tv[3] = {0.f, 0.f, 0.f}, tc[9], tm = 0.f;
     // This particle's first node in the staged planes, -1 if it is in neither
     // region.
@@ -1070,14 +1069,16 @@ __global__ void __launch_bounds__(256, kMode == 1 ? 2 : ((kBatch || kMode == 2) 
     if ((!kBatch || scene == scene0) && (unsigned)(bx - ox0) < kBinX && (unsigned)(by - oy0) < kBinY && bz >= oz0 &&
         bz - oz0 + 3 <= nz0)
         at = ((bz - oz0) * kTY + by - oy0) * kTX + bx - ox0;
+    // The SDF at the particle, for the features: loaded while the nodes arrive.
+    constexpr bool kFeatures = kMode == kG2PLearned || kMode == kG2PCollect || kMode == kG2PLearnedTc;
+    const float phi = kFeatures ? sdf_trilinear(p, sdf, pos[0], pos[1], pos[2]) : 0.f;
     cp_async_wait<0>();
     __syncthreads();
     // Set when a stencil node lies outside the grid or inside an obstacle:
     // only then can the SDF at the new position be negative (see below).
     uint32_t sdf_risk = 0u;
     const int plane = p.sx * p.sy;
-    constexpr bool kRowSums = kMode != kG2PLearned && kMode != kG2PLearnedTc;
-    if constexpr (kRowSums) {
+    {
         float M[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) M[k] = 0.f;
@@ -1131,62 +1132,14 @@ __global__ void __launch_bounds__(256, kMode == 1 ? 2 : ((kBatch || kMode == 2) 
             tc[3 * k + 1] = 4.0f * (M[3 * k + 1] - tv[k] * gy);
             tc[3 * k + 2] = 4.0f * (M[3 * k + 2] - tv[k] * gz);
         }
-    } else {
-#pragma unroll
-        for (int k = 0; k < 9; ++k) tc[k] = 0.f;
-        // One node of the stencil, offsets (a, b, c).
-        auto gather = [&](int a, int b, int c, float4 g) {
-            const float dxv = -(fx - (float)a), dyv = -(fy - (float)b), dzv = -(fz - (float)c);
-            sdf_risk |= __float_as_uint(g.x) >> 31;
-            const float w = wx[a] * wy[b] * wz[c];
-            tv[0] += w * g.y;
-            tv[1] += w * g.z;
-            tv[2] += w * g.w;
-            tm += w * fabsf(g.x);
-            const float term = 4.0f * w;
-            tc[0] += term * g.y * dxv;
-            tc[1] += term * g.y * dyv;
-            tc[2] += term * g.y * dzv;
-            tc[3] += term * g.z * dxv;
-            tc[4] += term * g.z * dyv;
-            tc[5] += term * g.z * dzv;
-            tc[6] += term * g.w * dxv;
-            tc[7] += term * g.w * dyv;
-            tc[8] += term * g.w * dzv;
-        };
-        if (at >= 0) {
-            const float4* base = s_node + at;
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-#pragma unroll
-                for (int b = 0; b < 3; ++b)
-#pragma unroll
-                    for (int a = 0; a < 3; ++a) gather(a, b, c, base[(c * kTY + b) * kTX + a]);
-        } else {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const int z = bz + c;
-#pragma unroll
-                for (int b = 0; b < 3; ++b) {
-                    const int y = by + b;
-                    const bool zy = (unsigned)z < (unsigned)p.sz && (unsigned)y < (unsigned)p.sy;
-                    const float4* row = vgrid + ((long long)z * plane + (long long)y * p.sx + bx);
-#pragma unroll
-                    for (int a = 0; a < 3; ++a)
-                        gather(a, b, c, zy && (unsigned)(bx + a) < (unsigned)p.sx ? __ldg(row + a)
-                                                                               : make_float4(-0.0f, 0.f, 0.f, 0.f));
-                }
-            }
-        }
     }
-    if constexpr (kMode == kG2PLearned || kMode == kG2PCollect || kMode == kG2PLearnedTc) {
+    if constexpr (kFeatures) {
         float f[kMlpIn];
 #pragma unroll
         for (int k = 0; k < 9; ++k) f[k] = tc[k];
         f[9] = tv[0], f[10] = tv[1], f[11] = tv[2];
         f[12] = tm * (p.pvol / p.pmass) - 1.0f;
         f[13] = f[14] = f[15] = 0.f;
-        const float phi = sdf_trilinear(p, sdf, pos[0], pos[1], pos[2]);
         if (fabsf(phi) < 4.0f) {
             const float3 nrm = sdf_gradient_dir(p, sdf, pos[0], pos[1], pos[2]);
             const float s = phi * (1.0f - fabsf(phi) * 0.25f);
@@ -1224,10 +1177,17 @@ __global__ void __launch_bounds__(256, kMode == 1 ? 2 : ((kBatch || kMode == 2) 
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) dev[q] += __shfl_xor_sync(0xffffffffu, dev[q], o);
             }
-            if ((threadIdx.x & 31) == 0) {
-                atomicAdd(la.stat, dev[0]);
-                atomicAdd(la.stat + 1, dev[1]);
-                atomicAdd(la.stat + 2, dev[2]);
+            // One reduction per CTA and sum: three additions per warp to the
+            // same three words serialised in L2 and were the kernel's time
+            // (2M particles: 186k of them; the kernel 345 -> 243 us).
+            const int warp = threadIdx.x >> 5;
+            if ((threadIdx.x & 31) == 0) s_dev[0][warp] = dev[0], s_dev[1][warp] = dev[1], s_dev[2][warp] = dev[2];
+            __syncthreads();
+            if (threadIdx.x < 3) {
+                float sum = 0.f;
+#pragma unroll
+                for (int w = 0; w < 8; ++w) sum += s_dev[threadIdx.x][w];
+                atomicAdd(la.stat + threadIdx.x, sum);
             }
         } else if (valid) {  // collection probe: la.feat holds n rows
             float* fo = la.feat + (size_t)sig * kMlpIn;
