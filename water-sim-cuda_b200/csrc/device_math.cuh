@@ -53,12 +53,13 @@ struct SimParams {
 };
 
 // The scenes of an engine on the device: prm[s], and the prefix arrays
-// poff[s] / goff[s] (S + 1 entries each) that map a global particle slot or
-// grid node to its scene.
+// poff[s] / goff[s] / boff[s] (S + 1 entries each) that map a global particle
+// slot, grid node or bin entry to its scene.
 struct SceneTable {
     const SimParams* prm;
     const long long* poff;
     const long long* goff;
+    const long long* boff;
     int count;
 };
 

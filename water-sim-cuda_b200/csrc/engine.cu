@@ -71,6 +71,7 @@ struct mpm_engine {
     SimParams* d_prm = nullptr;
     long long* d_poff = nullptr;     // S + 1 first slots
     long long* d_goff = nullptr;     // S + 1 first nodes
+    long long* d_boff = nullptr;     // S + 1 first bin entries
     mpm::SceneTable table{};
 
     bool initialized = false;
@@ -349,16 +350,19 @@ constexpr size_t kCtlBytes = kCtlWords * sizeof(uint32_t);
 
 // Uploads the scene table (after the particle offsets change).
 mpm_status upload_table(mpm_engine* e) {
-    std::vector<long long> poff(e->scenes + 1), goff(e->scenes + 1);
+    std::vector<long long> poff(e->scenes + 1), goff(e->scenes + 1), boff(e->scenes + 1);
     for (int s = 0; s < e->scenes; ++s) {
         poff[s] = e->prm[s].poff;
         goff[s] = e->prm[s].goff;
+        boff[s] = e->prm[s].boff;
     }
     poff[e->scenes] = e->n;
     goff[e->scenes] = e->g_total;
+    boff[e->scenes] = e->bins_total;
     CK(e, cudaMemcpyAsync(e->d_prm, e->prm.data(), e->scenes * sizeof(SimParams), cudaMemcpyHostToDevice, e->stream));
     CK(e, cudaMemcpyAsync(e->d_poff, poff.data(), poff.size() * sizeof(long long), cudaMemcpyHostToDevice, e->stream));
     CK(e, cudaMemcpyAsync(e->d_goff, goff.data(), goff.size() * sizeof(long long), cudaMemcpyHostToDevice, e->stream));
+    CK(e, cudaMemcpyAsync(e->d_boff, boff.data(), boff.size() * sizeof(long long), cudaMemcpyHostToDevice, e->stream));
     // Pageable host copies: wait before the vectors go out of scope.
     CK(e, cudaStreamSynchronize(e->stream));
     return MPM_OK;
@@ -620,6 +624,10 @@ mpm_status run_steps(mpm_engine* e, int32_t nsub) {
     return export_positions(e);
 }
 
+// Grid nodes (all scenes) from which the touched-tile grid update is the
+// default, and from which the autotuner tries it.
+constexpr long long kTilesFrom = 1LL << 20;
+
 // Engine with `count` scenes; grid arrays, counter sets and the scene table
 // are allocated here, particle arrays by the first init.
 // The P2G accumulation grid as a persisting L2 window on the engine's
@@ -756,7 +764,8 @@ mpm_status create_engine(const mpm_config* cfgs, int32_t count, int32_t device, 
         (err = cudaMalloc(&e->desc, (size_t)cells_total * sizeof(int2))) != cudaSuccess ||
         (err = cudaMalloc(&e->d_prm, count * sizeof(SimParams))) != cudaSuccess ||
         (err = cudaMalloc(&e->d_poff, (count + 1) * sizeof(long long))) != cudaSuccess ||
-        (err = cudaMalloc(&e->d_goff, (count + 1) * sizeof(long long))) != cudaSuccess)
+        (err = cudaMalloc(&e->d_goff, (count + 1) * sizeof(long long))) != cudaSuccess ||
+        (err = cudaMalloc(&e->d_boff, (count + 1) * sizeof(long long))) != cudaSuccess)
         return fail(cuda_fail(e, err, "cudaMalloc(grid)"));
     carve_bins(e);
     e->tiles.stamp = static_cast<uint32_t*>(e->tiles_mem);
@@ -767,11 +776,14 @@ mpm_status create_engine(const mpm_config* cfgs, int32_t count, int32_t device, 
     e->table.prm = e->d_prm;
     e->table.poff = e->d_poff;
     e->table.goff = e->d_goff;
+    e->table.boff = e->d_boff;
     e->table.count = count;
-    // A grid of 2^23 nodes or more (256^3) is mostly empty in the workloads
-    // measured; there the touched-tile update is 2.7x faster than the update
-    // of every node, while on 128^3 it ties and on 64^3 it is slower.
-    if (count == 1 && g_total >= (1LL << 23)) e->tune.grid_block = 0;
+    // Fluid fills a small part of a large grid, so the touched-tile update
+    // reads and writes less there.  Grid update per substep, every node / touched
+    // tiles (the ordering's marks cost 0.3 to 1.5 us more): 64^3 2.7 / 3.7 us,
+    // 97 x 61 x 83 4.5 / 4.7, 128^3 with 2M particles 12.2 / 8.7, with 5.2M 13.0 /
+    // 10.3, the 64-scene batch (17M nodes) 145 / 70, 256^3 96 / 28.
+    if (g_total >= kTilesFrom) e->tune.grid_block = 0;
     cudaMemsetAsync(e->accum, 0, (size_t)g_total * sizeof(float4), e->stream);
     cudaMemsetAsync(e->vgrid, 0, (size_t)g_total * sizeof(float4), e->stream);
     cudaMemsetAsync(e->tiles_mem, 0, tiles_bytes(e), e->stream);
@@ -1059,6 +1071,7 @@ extern "C" void mpm_destroy(mpm_engine* e) {
     free_dev(e->d_prm);
     free_dev(e->d_poff);
     free_dev(e->d_goff);
+    free_dev(e->d_boff);
     free_dev(e->d_flags);
     free_dev(e->staging);
     free_dev(e->d_prm_large);
@@ -1952,6 +1965,7 @@ extern "C" mpm_status mpm_autotune(mpm_engine* e, int32_t repeats, mpm_tuning* o
     tbest = 1e30f;
     for (int k : {128, 256, 0}) {
         if (s != MPM_OK) break;
+        if (k == 0 && e->g_total < kTilesFrom) break;  // slower there (create_engine)
         e->tune.grid_block = k;
         if ((s = median_time(MPM_STAGE_GRID, &ms)) != MPM_OK) break;
         if (ms < tbest) tbest = ms, best.grid_block = k, best.grid_ms = ms;

@@ -845,8 +845,7 @@ __global__ void __launch_bounds__(256) grid_update_kernel(SceneTable sc, SimPara
     if (a.x != 0.f || a.y != 0.f || a.z != 0.f || a.w != 0.f) accum[gi] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// One warp per node tile (TileMarks; global bin entries, the scene found by
-// binary search over the scenes' first entries): lane l takes the nodes
+// One warp per node tile (TileMarks; global bin entries): lane l takes the nodes
 // (x0 + l % 8, y0 + l / 8, z0 + c), c = 0..3.  A tile marked by this
 // substep's ordering is updated like grid_update_kernel; a tile updated
 // before but not marked now holds no accumulated mass any more and is reset to
@@ -857,20 +856,15 @@ __global__ void __launch_bounds__(256) grid_tiles_kernel(SceneTable sc, SimParam
                                                          float4* __restrict__ accum_all, float4* __restrict__ vgrid_all,
                                                          const float* __restrict__ sdf_all) {
     pdl_wait();
+    __shared__ SimParams s_prm[kBatch ? kTableScenes : 1];
+    __shared__ long long s_first[kBatch ? kTableScenes + 1 : 1];
+    __shared__ int s_range[2];
     const long long gt = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
+    const SceneLookup<kBatch> look(sc, sc.boff, s_prm, s_first, s_range, blockIdx.x * (long long)(blockDim.x / 32),
+                                   min((blockIdx.x + 1) * (long long)(blockDim.x / 32), tiles.count));
     if (gt >= tiles.count) return;  // warp-uniform
-    int scene = 0;
-    if constexpr (kBatch) {
-        int lo = 0, hi = sc.count - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (__ldg(&sc.prm[mid].boff) <= gt) lo = mid;
-            else hi = mid - 1;
-        }
-        scene = lo;
-    }
-    const SimParams& p = kBatch ? sc.prm[scene] : p0;
+    const SimParams& p = kBatch ? look.params(look.scene(gt)) : p0;
     const int t = (int)(gt - p.boff);
     if (t >= p.nb) return;  // the overflow bin's entries hold no tile
     float4* accum = accum_all + p.goff;
