@@ -584,12 +584,8 @@ mpm_status enter_scene(mpm_engine* e, int32_t scene) {
 mpm_status export_positions(mpm_engine* e) {
     const int b = 1 - e->pos_cur;
     CK(e, cudaStreamWaitEvent(e->stream, e->copy_done[b], 0));
-    for (int sc = 0; sc < e->scenes; ++sc) {
-        const SimParams& p = e->prm[sc];
-        e->kernel_launches += mpm::launch_positions_export(p, e->P[e->parity] + p.poff * mpm::kAFloats,
-                                                           e->sigma[e->parity] + p.poff, e->pos_buf[b] + p.poff * 3,
-                                                           e->stream);
-    }
+    e->kernel_launches +=
+        mpm::launch_positions_export(e->n, e->P[e->parity], e->sigma[e->parity], e->pos_buf[b], e->stream);
     CK(e, cudaGetLastError());
     CK(e, cudaEventRecord(e->pos_ready[b], e->stream));
     e->pos_cur = b;
