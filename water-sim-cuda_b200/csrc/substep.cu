@@ -43,7 +43,7 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
 // on measured 5 % off P2G on the 2M dam break (early and late states).
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     uint64_t pol;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
     asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(
                      static_cast<uint32_t>(__cvta_generic_to_shared(smem))),
                  "l"(gmem), "l"(pol)
@@ -51,6 +51,11 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 }
 __device__ __forceinline__ void cp_async16_plain(void* smem, const void* gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem))),
+                 "l"(gmem)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem))),
                  "l"(gmem)
                  : "memory");
 }
@@ -145,12 +150,18 @@ struct SceneLookup {
 // out every bin's item 0 before any item 1, and so on, so the longest items
 // start first.  Lane = cell: all particles of a cell scatter to the same 27
 // nodes, so the lane sums them in registers, reading them through a ring of
-// kRing particles fetched ahead with 16-byte cp.async copies (the gather
-// through gidx costs no registers).  The lane then adds its 27 sums to the
-// warp's footprint, the bin's 10 x 6 x 6 nodes in shared memory: the lanes'
-// cells are distinct, so for one stencil offset their nodes differ and a plain
-// read-add-write per offset is race-free.  The footprint's z-planes that the
-// item reached go to global memory with one vector reduction per touched node.
+// kRing particles fetched ahead with 16-byte cp.async copies, at indices that
+// are copied to shared memory kIdxWindow at a time (neither costs registers;
+// the indices loaded one by one as they are needed: 88.1 / 86.7 us on the 2M
+// dam break; a ring of 3 or 4: 3 and 5 % slower).  A record's six vectors are
+// read and written by its own lane only, so the ring needs no warp barrier
+// (copied with neighbouring lanes on neighbouring vectors, 15 % slower: the
+// shuffles cost more than the 32 separate lines of a copy).  The lane then adds
+// its 27 sums to the warp's footprint, the bin's 10 x 6 x 6 nodes in shared
+// memory: the lanes' cells are distinct, so for one stencil offset their nodes
+// differ and a plain read-add-write per offset is race-free.  The footprint's
+// z-planes that the item reached go to global memory with one vector reduction
+// per touched node.
 // A lane sums at most `cap` particles of its cell; the rest of a crowded cell
 // (this Tait law resists only expansion, so compressed fluid piles up) is on
 // the list in chunks of kCrowdChunk particles: there the 32 lanes share one
@@ -159,8 +170,15 @@ struct SceneLookup {
 // of their particles would hold up the kernel.)  The ordering lays out both
 // (cell_scan_kernel).  Unlike the reference, no partial sum is dropped (it
 // drops shared-tile cells whose partial mass is <= 1e-9, kernels.cu:132).
+// What bounds it: the 108 sums leave room for 12 warps per SM, whose
+// instructions (about 510 per 32 particles) and waits take turns: 47 % of the
+// issue slots, DRAM at 2.5 TB/s.  2M particles 86.7 us (29 us for the records
+// alone), 6.1M in 64 scenes 253 us.  Taking the next unit while one is summed
+// or written out, to hide the unit's three dependent loads, made the last
+// units uneven: 93.1 and 88.7 us.
 constexpr int kP2GWarpsPerSM = 12;
 constexpr int kRing = 2;
+constexpr int kIdxWindow = 32;
 // Where a launch has fewer items than half its warps, each item's particles are
 // shared out over 2, 4 or 8 warps (parts): the lanes of a part take an equal
 // share of their cells' particles, and the parts' sums meet in the global
@@ -168,22 +186,25 @@ constexpr int kRing = 2;
 // and up to 32 rounds per lane, and warps without an item are free; with more
 // items than that a further part only adds another flush (parts until there
 // are two or four units per warp: the 113k sphere drop 4 and 12 % slower).
-// P2G per substep, before / after: 8k particles (16 bins) 18.1 / 8.5 us, 113k
-// (about 200 bins) 19.3 / 14.5 us.
+// P2G per substep, one warp an item / parts: 8k particles (16 bins) 18.1 / 8.5
+// us, 113k (about 200 bins) 19.3 / 14.5 us.
 constexpr int kMaxParts = 8;
 constexpr int kCellCap = 12;      // particles of a cell its own lane sums; the rest: the crowded-cell list
 constexpr int kCrowdChunk = 256;  // particles of a crowded cell per list entry
 constexpr int kTX = kBinX + 2, kTY = kBinY + 2;
 constexpr int kFootPlane = kTX * kTY;              // 60 nodes of one z-plane
 constexpr int kFootNodes = kFootPlane * (kBinZ + 2);  // 360: a bin's stencil footprint
+constexpr int kFlushRows = 3;  // rows of a footprint plane that a warp flushes at once
+static_assert(kFlushRows * kTX <= 32 && 2 * kFlushRows == kTY, "two passes per plane");
 static_assert(kBinX * kBinY == 32 && kBinZ == 4, "a bin is 128 cells: four items of 32");
 
 // Spline weights of nodes 0, 1, 2 of one axis at fractional offset f = pos -
-// base, times m.  For f in [0.5, 1.5) (every particle at pos >= 0.5) the
-// branch of bspline_weight is known per node and the same roundings are
+// base, times m.  For f in [0.5, 1.5) (kInner; every particle at pos >= 0.5)
+// the branch of bspline_weight is known per node and the same roundings are
 // written out; otherwise the general form.
+template <bool kInner>
 __device__ __forceinline__ void axis_weights(float f, float m, float* w) {
-    if (f >= 0.5f && f < 1.5f) {
+    if constexpr (kInner) {
         const float t0 = __fsub_rn(1.5f, f);
         const float x1 = __fsub_rn(f, 1.0f);
         const float t2 = __fsub_rn(1.5f, __fsub_rn(2.0f, f));
@@ -196,6 +217,40 @@ __device__ __forceinline__ void axis_weights(float f, float m, float* w) {
     }
 }
 
+// All three axes, wx times m, with one branch instead of three (P2G on the 2M
+// dam break 90.6 / 89.2 us).
+__device__ __forceinline__ void stencil_weights(float fx, float fy, float fz, float m, float* wx, float* wy,
+                                                float* wz) {
+    if (fx >= 0.5f && fx < 1.5f && fy >= 0.5f && fy < 1.5f && fz >= 0.5f && fz < 1.5f) {
+        axis_weights<true>(fx, m, wx);
+        axis_weights<true>(fy, 1.0f, wy);
+        axis_weights<true>(fz, 1.0f, wz);
+    } else {
+        axis_weights<false>(fx, m, wx);
+        axis_weights<false>(fy, 1.0f, wy);
+        axis_weights<false>(fz, 1.0f, wz);
+    }
+}
+
+// The Tait law's constants of a scene.  Where gamma is a whole number of at
+// most kTaitPower in magnitude, J^|gamma| - 1 is |gamma| steps of p' = p J +
+// (J - 1) from p = 0: no branch, no powf and no cancellation against 1 (J - 1
+// is exact for J in [0.9, 1.1]); a negative gamma's is -p / (1 + p).  n is 0
+// for every other gamma, and where k = 4 DT V / m is not an ordinary number:
+// those go through powf and the division.  P2G per substep, powf / steps: 2M
+// particles 97.2 / 90.6 us, 650k at gamma -2 40.3 / 36.1 us.
+constexpr int kTaitPower = 8;
+struct Tait {
+    int n;
+    float k;
+    __device__ __forceinline__ explicit Tait(const SimParams& p) {
+        const float g = fabsf(p.gamma);
+        k = 4.0f * p.dt * p.pvol / p.pmass;
+        const bool plain = k == 0.0f || (fabsf(k) > 1e-30f && fabsf(k) < 1e30f);
+        n = plain && g >= 1.0f && g <= (float)kTaitPower && g == truncf(g) ? (int)p.gamma : 0;
+    }
+};
+
 // Per-particle part of P2G from the particle's 96-byte record: the spline
 // weights (mass folded into wx) and the affine momentum at stencil node
 // (0,0,0), u = v - C' f, with C' the stress-augmented affine matrix.  Node
@@ -207,8 +262,8 @@ struct P2GParticle {
     int bx, by, bz;  // stencil base cell
 };
 
-__device__ __forceinline__ P2GParticle p2g_particle(const SimParams& p, float4 q0, float4 q1, float4 q2, float4 q3,
-                                                    float4 q4, float4 q5) {
+__device__ __forceinline__ P2GParticle p2g_particle(const SimParams& p, const Tait& tait, float4 q0, float4 q1,
+                                                    float4 q2, float4 q3, float4 q4, float4 q5) {
     P2GParticle r;
     const float px = q0.x, py = q0.y, pz = q0.z;
     const float F[9] = {q0.w, q1.x, q1.y, q1.z, q1.w, q2.x, q2.y, q2.z, q2.w};
@@ -226,13 +281,25 @@ __device__ __forceinline__ P2GParticle p2g_particle(const SimParams& p, float4 q
     // matrix C' = C + (4 DT V p / m) I (kernels.cu:20-35).
     float J = det3(F);
     J = fmaxf(0.9f, fminf(J, 1.1f));
-    // J^gamma - 1 > 0 only for J > 1 (gamma > 0) or J < 1 (gamma < 0); the
-    // clamp below zeroes every other case, so powf runs only where it counts.
-    float pressure = 0.0f;
-    if ((p.gamma > 0.0f && J > 1.0f) || (p.gamma < 0.0f && J < 1.0f))
-        pressure = p.compression * (powf(J, p.gamma) - 1.0f);
-    if (pressure < 0.0f) pressure = 0.0f;
-    const float multi = 4.0f * p.dt * (p.pvol * J) * pressure / p.pmass;
+    float multi;
+    if (tait.n != 0) {
+        const float e = J - 1.0f;
+        float t = e;
+#pragma unroll
+        for (int k = 1; k < kTaitPower; ++k)
+            if (k < abs(tait.n)) t = fmaf(t, J, e);
+        if (tait.n < 0) t = -t / (1.0f + t);
+        const bool expands = tait.n > 0 ? J > 1.0f : J < 1.0f;
+        multi = tait.k * J * (expands ? fmaxf(p.compression * t, 0.0f) : 0.0f);
+    } else {
+        // J^gamma - 1 > 0 only for J > 1 (gamma > 0) or J < 1 (gamma < 0); the
+        // clamp below zeroes every other case, so powf runs only where it counts.
+        float pressure = 0.0f;
+        if ((p.gamma > 0.0f && J > 1.0f) || (p.gamma < 0.0f && J < 1.0f))
+            pressure = p.compression * (powf(J, p.gamma) - 1.0f);
+        if (pressure < 0.0f) pressure = 0.0f;
+        multi = 4.0f * p.dt * (p.pvol * J) * pressure / p.pmass;
+    }
     C[0] += multi;
     C[4] += multi;
     C[8] += multi;
@@ -242,9 +309,7 @@ __device__ __forceinline__ P2GParticle p2g_particle(const SimParams& p, float4 q
     r.by = stencil_base(py);
     r.bz = stencil_base(pz);
     const float fx = px - (float)r.bx, fy = py - (float)r.by, fz = pz - (float)r.bz;
-    axis_weights(fx, p.pmass, r.wx);
-    axis_weights(fy, 1.0f, r.wy);
-    axis_weights(fz, 1.0f, r.wz);
+    stencil_weights(fx, fy, fz, p.pmass, r.wx, r.wy, r.wz);
     r.u0 = q3.x - (C[0] * fx + C[1] * fy + C[2] * fz);
     r.u1 = q3.y - (C[3] * fx + C[4] * fy + C[5] * fz);
     r.u2 = q3.z - (C[6] * fx + C[7] * fy + C[8] * fz);
@@ -312,6 +377,7 @@ __global__ void __launch_bounds__(32, kP2GWarpsPerSM) p2g_kernel(SceneTable sc, 
                                                                   uint32_t* __restrict__ status) {
     __shared__ __align__(16) float4 s_ring[kRing][6][32];
     __shared__ float4 s_foot[kFootNodes];
+    __shared__ int s_idx[kIdxWindow][32];
     const int lane = threadIdx.x;
     for (int q = lane; q < kFootNodes; q += 32) s_foot[q] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncwarp();
@@ -323,6 +389,7 @@ __global__ void __launch_bounds__(32, kP2GWarpsPerSM) p2g_kernel(SceneTable sc, 
     while (parts < kMaxParts && items * parts * 2 <= (int)gridDim.x) parts *= 2;
     const int total = ncrowd + items * parts;
     SimParams p = sc.prm[0];
+    Tait tait(p);
     // The first unit of a warp is its own index, the next ones come from the
     // counter: one round trip less where a launch has about a unit per warp.
     for (int unit = blockIdx.x; unit < total;) {
@@ -350,7 +417,10 @@ __global__ void __launch_bounds__(32, kP2GWarpsPerSM) p2g_kernel(SceneTable sc, 
         }
         const int maxc = (int)__reduce_max_sync(0xffffffffu, (unsigned)cnt);
         if (maxc > 0) {
-            if (sc.count > 1) p = sc.prm[scene];
+            if (sc.count > 1) {
+                p = sc.prm[scene];
+                tait = Tait(p);
+            }
             float4* accum = accum_all + p.goff;
             const int bxi = bin % p.nbx, byi = (bin / p.nbx) % p.nby, bzi = bin / (p.nbx * p.nby);
             // Node origin of the footprint = base cell of the bin's first cell.
@@ -359,25 +429,37 @@ __global__ void __launch_bounds__(32, kP2GWarpsPerSM) p2g_kernel(SceneTable sc, 
             float am[27], ax[27], ay[27], az[27];
 #pragma unroll
             for (int k = 0; k < 27; ++k) am[k] = ax[k] = ay[k] = az[k] = 0.f;
+            // Particle numbers of the lane's next kIdxWindow slots from s on,
+            // all in flight together.
+            auto fetch_indices = [&](int s) {
+#pragma unroll 1
+                for (int k = s; k < min(cnt, s + kIdxWindow); ++k)
+                    cp_async4(&s_idx[k % kIdxWindow][lane], gidx + first + stride * k);
+                cp_async_commit();
+                cp_async_wait<0>();
+            };
             auto fetch = [&](int s) {
-                const float4* src = reinterpret_cast<const float4*>(P + (size_t)__ldg(gidx + first + stride * s) * kAFloats);
+                const float4* src =
+                    reinterpret_cast<const float4*>(P + (size_t)s_idx[s % kIdxWindow][lane] * kAFloats);
 #pragma unroll
                 for (int v = 0; v < 6; ++v) cp_async16(&s_ring[s % kRing][v][lane], src + v);
             };
+            fetch_indices(0);
 #pragma unroll
             for (int d = 0; d < kRing - 1; ++d) {
                 if (d < cnt) fetch(d);
                 cp_async_commit();
             }
             for (int s = 0; s < maxc; ++s) {
+                if ((s + kRing - 1) % kIdxWindow == 0) fetch_indices(s + kRing - 1);
                 if (s + kRing - 1 < cnt) fetch(s + kRing - 1);
                 cp_async_commit();
                 cp_async_wait<kRing - 1>();
-                __syncwarp();
                 if (s < cnt) {
                     const int sl = s % kRing;
-                    const P2GParticle r = p2g_particle(p, s_ring[sl][0][lane], s_ring[sl][1][lane], s_ring[sl][2][lane],
-                                                       s_ring[sl][3][lane], s_ring[sl][4][lane], s_ring[sl][5][lane]);
+                    const P2GParticle r = p2g_particle(p, tait, s_ring[sl][0][lane], s_ring[sl][1][lane],
+                                                       s_ring[sl][2][lane], s_ring[sl][3][lane], s_ring[sl][4][lane],
+                                                       s_ring[sl][5][lane]);
                     // Filed under this lane's cell by construction; a mismatch
                     // is recorded, never scattered to a wrong node.
                     if (r.bx - ox != tx || r.by - oy != ty || r.bz - oz != tz) {
@@ -391,9 +473,9 @@ __global__ void __launch_bounds__(32, kP2GWarpsPerSM) p2g_kernel(SceneTable sc, 
                         });
                     }
                 }
-                __syncwarp();
             }
             cp_async_wait<0>();
+            __syncwarp();
             if (packed) {
                 // One cell on all lanes: a butterfly reduce-scatter (five
                 // shuffle steps, each halving the 128 padded sums) leaves
@@ -445,12 +527,30 @@ __global__ void __launch_bounds__(32, kP2GWarpsPerSM) p2g_kernel(SceneTable sc, 
                 // The z-planes the group's cells reach: zmin .. zmax + 2.
                 const int zmin = (int)__reduce_min_sync(0xffffffffu, cnt > 0 ? (unsigned)tz : 0xFFu);
                 const int zmax = (int)__reduce_max_sync(0xffffffffu, cnt > 0 ? (unsigned)tz : 0u);
-                for (int q = zmin * kFootPlane + lane; q < (zmax + 3) * kFootPlane; q += 32) {
-                    const int x = ox + q % kTX, y = oy + (q / kTX) % kTY, z = oz + q / kFootPlane;
-                    const float4 v = s_foot[q];
-                    s_foot[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (node_in_grid(p, x, y, z) && (v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f))  // NaN counts
-                        red_add_v4(accum + node_index(p, x, y, z), v.x, v.y, v.z, v.w);
+                // Half a plane at a time, three rows of ten nodes on thirty lanes, so
+                // that a lane's x stays and its addresses advance by constants (a
+                // node per lane and division, 2M dam break: 89.7 / 88.1 us).
+                if (lane < kFlushRows * kTX) {
+                    const int lx = lane % kTX, ly = lane / kTX;
+                    const int x = ox + lx, y = oy + ly;
+                    const bool in_x = (unsigned)x < (unsigned)p.sx;
+                    const bool in_y0 = in_x && (unsigned)y < (unsigned)p.sy;
+                    const bool in_y1 = in_x && (unsigned)(y + kFlushRows) < (unsigned)p.sy;
+                    float4* s = s_foot + zmin * kFootPlane + lane;
+                    float4* d = accum + ((long long)(oz + zmin) * p.sy + y) * p.sx + x;
+                    const int half = kFlushRows * p.sx;
+                    for (int z = oz + zmin; z < oz + zmax + 3; ++z) {
+                        const bool in_z = (unsigned)z < (unsigned)p.sz;
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const float4 v = s[h * kFlushRows * kTX];
+                            s[h * kFlushRows * kTX] = make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (in_z && (h ? in_y1 : in_y0) && (v.x != 0.f || v.y != 0.f || v.z != 0.f || v.w != 0.f))
+                                red_add_v4(d + h * half, v.x, v.y, v.z, v.w);  // NaN counts
+                        }
+                        s += kFootPlane;
+                        d += (long long)p.sx * p.sy;
+                    }
                 }
             }
             __syncwarp();
@@ -1044,9 +1144,7 @@ __global__ void __launch_bounds__(256, kMode == 1 ? 2 : ((kBatch || kMode == 2) 
     // and axis_weights gives bspline_weight's values.
     const float fx = pos[0] - (float)bx, fy = pos[1] - (float)by, fz = pos[2] - (float)bz;
     float wx[3], wy[3], wz[3];
-    axis_weights(fx, 1.0f, wx);
-    axis_weights(fy, 1.0f, wy);
-    axis_weights(fz, 1.0f, wz);
+    stencil_weights(fx, fy, fz, 1.0f, wx, wy, wz);
     // Interpolation sums (g2PTransfer's loop, kernels.cu:214-235), separably
     // per axis: with o = (a, b, c) the node offset and x_node - x_p = (o - 1) - (f - 1),
     //   v' = sum w v,   C' = 4 (M - v' (f - 1)^T),   M[k][d] = sum w v_k (o_d - 1),
