@@ -39,6 +39,7 @@
 
 #include "kernels.h"
 #include "mpm_b200.h"
+#include "readback.h"
 
 using mpm::SimParams;
 
@@ -58,6 +59,7 @@ struct mpm_engine {
     int device = 0;
     cudaStream_t stream = nullptr;
     std::string last_error;
+    mpm::Readback readback;  // large results to pageable memory
     uint32_t checks = 0;
 
     // Scenes: config, constants and offsets (host copy of the device table).
@@ -1259,8 +1261,7 @@ extern "C" mpm_status mpm_scene_get_state(mpm_engine* e, int32_t scene, float* o
     e->kernel_launches += mpm::launch_state_export(p, e->P[e->parity] + p.poff * mpm::kAFloats,
                                                    e->sigma[e->parity] + p.poff, e->staging, e->stream);
     CK(e, cudaGetLastError());
-    CK(e, cudaMemcpyAsync(out, e->staging, bytes, cudaMemcpyDeviceToHost, e->stream));
-    CK(e, cudaStreamSynchronize(e->stream));
+    CK(e, e->readback.read(out, e->staging, bytes, e->stream));
     return MPM_OK;
 }
 
@@ -1272,16 +1273,14 @@ extern "C" const float* mpm_scene_positions_device(mpm_engine* e, int32_t scene)
 }
 
 namespace {
-// Enqueues the read-back of the current positions of `scene` (-1: all
-// scenes) on the copy stream, after the export that wrote them.
-mpm_status enqueue_positions_copy(mpm_engine* e, int32_t scene, float* xyz) {
+// Enqueues the read-back of all scenes' current positions on the copy stream,
+// after the export that wrote them.
+mpm_status enqueue_positions_copy(mpm_engine* e, float* xyz) {
     const int b = e->pos_cur;
-    const long long first = scene < 0 ? 0 : e->prm[scene].poff;
-    const long long count = scene < 0 ? e->n : e->prm[scene].n;
     CK(e, cudaStreamWaitEvent(e->copy_stream, e->pos_ready[b], 0));
-    if (count > 0)
-        CK(e, cudaMemcpyAsync(xyz, e->pos_buf[b] + first * 3, (size_t)count * 3 * sizeof(float),
-                              cudaMemcpyDeviceToHost, e->copy_stream));
+    if (e->n > 0)
+        CK(e, cudaMemcpyAsync(xyz, e->pos_buf[b], (size_t)e->n * 3 * sizeof(float), cudaMemcpyDeviceToHost,
+                              e->copy_stream));
     CK(e, cudaEventRecord(e->copy_done[b], e->copy_stream));
     return MPM_OK;
 }
@@ -1292,7 +1291,7 @@ extern "C" mpm_status mpm_get_positions_async(mpm_engine* e, float* xyz) {
     if (s != MPM_OK) return s;
     if (!e->initialized) return record(e, MPM_ERR_NOT_INITIALIZED, "mpm_init_particles has not been called");
     if (e->n > 0 && !xyz) return record(e, MPM_ERR_INVALID_ARGUMENT, "xyz_host is NULL");
-    return enqueue_positions_copy(e, -1, xyz);
+    return enqueue_positions_copy(e, xyz);
 }
 
 extern "C" mpm_status mpm_positions_wait(mpm_engine* e) {
@@ -1311,8 +1310,10 @@ extern "C" mpm_status mpm_scene_get_positions(mpm_engine* e, int32_t scene, floa
     const SimParams& p = e->prm[scene];
     if (p.n == 0) return MPM_OK;
     if (!xyz) return record(e, MPM_ERR_INVALID_ARGUMENT, "xyz_host is NULL");
-    if ((s = enqueue_positions_copy(e, scene, xyz)) != MPM_OK) return s;
-    CK(e, cudaStreamSynchronize(e->copy_stream));
+    const int b = e->pos_cur;
+    CK(e, cudaStreamWaitEvent(e->copy_stream, e->pos_ready[b], 0));
+    CK(e, e->readback.read(xyz, e->pos_buf[b] + p.poff * 3, (size_t)p.n * 3 * sizeof(float), e->copy_stream));
+    CK(e, cudaEventRecord(e->copy_done[b], e->copy_stream));
     return MPM_OK;
 }
 
@@ -1328,8 +1329,7 @@ extern "C" mpm_status mpm_scene_get_grid(mpm_engine* e, int32_t scene, float* ou
     const float4* src = (e->grid_view == GridView::kAccum ? e->accum : e->vgrid) + p.goff;
     e->kernel_launches += mpm::launch_grid_export(p, src, e->staging, e->stream);
     CK(e, cudaGetLastError());
-    CK(e, cudaMemcpyAsync(out, e->staging, bytes, cudaMemcpyDeviceToHost, e->stream));
-    CK(e, cudaStreamSynchronize(e->stream));
+    CK(e, e->readback.read(out, e->staging, bytes, e->stream));
     return MPM_OK;
 }
 
@@ -1340,8 +1340,7 @@ extern "C" mpm_status mpm_scene_get_sdf(mpm_engine* e, int32_t scene, float* out
     if (s != MPM_OK) return s;
     if (!out) return record(e, MPM_ERR_INVALID_ARGUMENT, "sdf_host is NULL");
     const SimParams& p = e->prm[scene];
-    CK(e, cudaMemcpyAsync(out, e->sdf + p.goff, (size_t)p.g * sizeof(float), cudaMemcpyDeviceToHost, e->stream));
-    CK(e, cudaStreamSynchronize(e->stream));
+    CK(e, e->readback.read(out, e->sdf + p.goff, (size_t)p.g * sizeof(float), e->stream));
     return MPM_OK;
 }
 
@@ -1369,8 +1368,8 @@ extern "C" mpm_status mpm_scene_get_sort(mpm_engine* e, int32_t scene, int32_t* 
         e->sort_passes += 4;
     }
     CK(e, cudaGetLastError());
-    if (keys_host) CK(e, cudaMemcpyAsync(keys_host, e->ref_keys, bytes, cudaMemcpyDeviceToHost, e->stream));
-    if (perm_host) CK(e, cudaMemcpyAsync(perm_host, e->ref_perm, bytes, cudaMemcpyDeviceToHost, e->stream));
+    if (keys_host) CK(e, e->readback.read(keys_host, e->ref_keys, bytes, e->stream));
+    if (perm_host) CK(e, e->readback.read(perm_host, e->ref_perm, bytes, e->stream));
     CK(e, cudaStreamSynchronize(e->stream));
     return MPM_OK;
 }

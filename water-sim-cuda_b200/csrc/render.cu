@@ -53,6 +53,7 @@
 
 #include "../../include/mpm_b200.h"
 #include "kernels.h"
+#include "readback.h"
 
 namespace {
 
@@ -351,6 +352,8 @@ struct mpm_renderer {
     unsigned char* ocolor = nullptr;   // their flat colours, 8 bits
     int ntris = 0;
     std::string last_error;
+    mpm::Readback readback;
+    cudaStream_t read_stream = nullptr;
 };
 
 namespace {
@@ -468,6 +471,7 @@ mpm_status mpm_renderer_create(const mpm_render_params* params, int32_t device, 
     if (err == cudaSuccess) err = cudaMalloc(&r->rgb8, npix * 3);
     if (err == cudaSuccess) err = cudaMalloc(&r->bg, npix * 3);
     if (err == cudaSuccess) err = cudaMalloc(&r->base, npix * 3);
+    if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&r->read_stream, cudaStreamNonBlocking);
     if (err != cudaSuccess) {
         cudaGetLastError();
         return bad(rfail(nullptr, MPM_ERR_OUT_OF_MEMORY, std::string("renderer allocation: ") + cudaGetErrorString(err)));
@@ -488,6 +492,7 @@ void mpm_renderer_destroy(mpm_renderer* r) {
     for (void* p : {(void*)r->zbuf, (void*)r->depth, (void*)r->tmp, (void*)r->fin, (void*)r->rgb, (void*)r->rgb8, (void*)r->bg,
                     (void*)r->base, (void*)r->odepth, (void*)r->okey, (void*)r->otris, (void*)r->ocolor})
         if (p) cudaFree(p);
+    if (r->read_stream) cudaStreamDestroy(r->read_stream);
     delete r;
 }
 
@@ -582,10 +587,10 @@ mpm_status mpm_renderer_get_background(mpm_renderer* r, uint8_t* rgb8_host, floa
     RK(r, cudaSetDevice(r->device));
     RK(r, cudaDeviceSynchronize());
     const size_t npix = (size_t)r->prm.width * r->prm.height;
-    if (rgb8_host) RK(r, cudaMemcpy(rgb8_host, r->bg, npix * 3, cudaMemcpyDeviceToHost));
+    if (rgb8_host) RK(r, r->readback.read(rgb8_host, r->bg, npix * 3, r->read_stream));
     if (depth_host) {
         if (r->odepth) {
-            RK(r, cudaMemcpy(depth_host, r->odepth, npix * sizeof(float), cudaMemcpyDeviceToHost));
+            RK(r, r->readback.read(depth_host, r->odepth, npix * sizeof(float), r->read_stream));
         } else {
             for (size_t i = 0; i < npix; ++i) depth_host[i] = 1.0f;
         }
@@ -625,7 +630,7 @@ mpm_status mpm_renderer_get_depth(mpm_renderer* r, int32_t which, float* host) {
     RK(r, cudaDeviceSynchronize());
     const size_t npix = (size_t)r->prm.width * r->prm.height;
     const float* src = which == 0 ? r->depth : (which == 1 ? r->tmp : r->fin);
-    RK(r, cudaMemcpy(host, src, npix * sizeof(float), cudaMemcpyDeviceToHost));
+    RK(r, r->readback.read(host, src, npix * sizeof(float), r->read_stream));
     return MPM_OK;
 }
 
@@ -634,8 +639,8 @@ mpm_status mpm_renderer_get_image(mpm_renderer* r, float* rgb_host, uint8_t* rgb
     RK(r, cudaSetDevice(r->device));
     RK(r, cudaDeviceSynchronize());
     const size_t npix = (size_t)r->prm.width * r->prm.height;
-    if (rgb_host) RK(r, cudaMemcpy(rgb_host, r->rgb, npix * 3 * sizeof(float), cudaMemcpyDeviceToHost));
-    if (rgb8_host) RK(r, cudaMemcpy(rgb8_host, r->rgb8, npix * 3, cudaMemcpyDeviceToHost));
+    if (rgb_host) RK(r, r->readback.read(rgb_host, r->rgb, npix * 3 * sizeof(float), r->read_stream));
+    if (rgb8_host) RK(r, r->readback.read(rgb8_host, r->rgb8, npix * 3, r->read_stream));
     return MPM_OK;
 }
 
