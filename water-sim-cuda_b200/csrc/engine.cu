@@ -135,6 +135,14 @@ struct mpm_engine {
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     cudaGraph_t graph_src[2] = {nullptr, nullptr};
     int graph_kernels[2] = {0, 0};
+    cudaGraphExec_t chain[2] = {nullptr, nullptr};  // kChain substeps from parity 0 / 1, captured when first needed
+    int chain_kernels[2] = {0, 0};
+    bool chain_off = false;  // the chains could not be captured
+    // What the graphs embed beside addresses that change with the particle
+    // buffers only (free_particles): a new state of the same sizes keeps them.
+    std::vector<SimParams> graph_prm;
+    mpm_tuning graph_tune{};
+    int graph_timing = -1;
 
     // Stage timing: kTimingMarks event-record nodes per substep graph, pointed
     // at a fresh slot of `tev` before each launch (scratch events once full).
@@ -234,16 +242,26 @@ void free_learned_buffers(mpm_engine* e) {
     free_dev(e->vplain);
 }
 
+void destroy_graphs(mpm_engine* e) {
+    for (int k = 0; k < 2; ++k) {
+        if (e->graph[k]) cudaGraphExecDestroy(e->graph[k]);
+        if (e->graph_src[k]) cudaGraphDestroy(e->graph_src[k]);
+        if (e->chain[k]) cudaGraphExecDestroy(e->chain[k]);
+        e->graph[k] = nullptr;
+        e->graph_src[k] = nullptr;
+        e->chain[k] = nullptr;
+        e->graph_kernels[k] = e->chain_kernels[k] = 0;
+    }
+    e->chain_off = false;
+    e->graph_prm.clear();
+}
+
 void free_particles(mpm_engine* e) {
     destroy_learned_graphs(e);
+    destroy_graphs(e);
     for (int k = 0; k < 2; ++k) {
         free_dev(e->P[k]);
         free_dev(e->sigma[k]);
-        if (e->graph[k]) cudaGraphExecDestroy(e->graph[k]);
-        if (e->graph_src[k]) cudaGraphDestroy(e->graph_src[k]);
-        e->graph[k] = nullptr;
-        e->graph_src[k] = nullptr;
-        e->graph_kernels[k] = 0;
     }
     free_dev(e->gidx);
     free_dev(e->edge);
@@ -275,20 +293,13 @@ mpm_status alloc_particles(mpm_engine* e, long long n, int max_n, size_t sort_by
     if (e->cap_n > 0 && n <= e->cap_n && max_n <= e->cap_max_n && sort_bytes <= e->cap_sort) {
         // The buffers of an earlier init are large enough: keep them (freeing
         // and allocating half a gigabyte takes from a few to hundreds of
-        // milliseconds).  The substep graphs are captured again by the caller;
-        // the learned-step buffers, sized by the earlier n, are allocated
-        // again when next needed.  Work of the earlier state (an asynchronous
+        // milliseconds).  The caller captures the substep graphs again where
+        // they no longer fit; the learned-step buffers, sized by the earlier
+        // n, are allocated again when next needed.  Work of the earlier state (an asynchronous
         // positions read-back on the copy stream included) ends first.
         CK(e, cudaStreamSynchronize(e->stream));
         CK(e, cudaStreamSynchronize(e->copy_stream));
         destroy_learned_graphs(e);
-        for (int k = 0; k < 2; ++k) {
-            if (e->graph[k]) cudaGraphExecDestroy(e->graph[k]);
-            if (e->graph_src[k]) cudaGraphDestroy(e->graph_src[k]);
-            e->graph[k] = nullptr;
-            e->graph_src[k] = nullptr;
-            e->graph_kernels[k] = 0;
-        }
         free_learned_buffers(e);
         e->n = n;
         e->max_n = max_n;
@@ -429,11 +440,8 @@ mpm_status capture_graphs(mpm_engine* e) {
     // velocities, so the first tile update resets every tile not marked.
     if (active_tiles(e).mark) CK(e, cudaMemsetAsync(e->tiles.dirty, 1, (size_t)e->bins_total, e->stream));
     const bool timed = e->timing_cap > 0;
+    destroy_graphs(e);
     for (int par = 0; par < 2; ++par) {
-        if (e->graph[par]) cudaGraphExecDestroy(e->graph[par]);
-        if (e->graph_src[par]) cudaGraphDestroy(e->graph_src[par]);
-        e->graph[par] = nullptr;
-        e->graph_src[par] = nullptr;
         cudaGraph_t g = nullptr;
         CK(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
         const int launches = enqueue_substep(e, par, MPM_STAGE_SORT, MPM_STAGE_G2P, timed ? e->tscratch : nullptr);
@@ -467,7 +475,55 @@ mpm_status capture_graphs(mpm_engine* e) {
         CK(e, cudaGraphInstantiate(&e->graph[par], g, 0));
         e->graph_kernels[par] = launches;
     }
+    e->graph_prm = e->prm;
+    e->graph_tune = e->tune;
+    e->graph_timing = e->timing_cap;
     return MPM_OK;
+}
+
+// Whether the captured graphs fit the current state.  Capturing them for every
+// new state took most of a small one's init: 8k particles 333 / 92 us.
+bool graphs_fit(const mpm_engine* e) {
+    const mpm_tuning &a = e->graph_tune, &b = e->tune;
+    return e->graph[0] && e->graph[1] && e->graph_timing == e->timing_cap && a.p2g_ctas_per_sm == b.p2g_ctas_per_sm &&
+           a.g2p_block == b.g2p_block && a.grid_block == b.grid_block && a.p2g_cell_cap == b.p2g_cell_cap &&
+           e->graph_prm.size() == e->prm.size() &&
+           std::memcmp(e->graph_prm.data(), e->prm.data(), e->prm.size() * sizeof(SimParams)) == 0;
+}
+
+// kChain substeps as one graph: three launches and the gaps of about 3 us
+// before their first kernels fewer.  A chain ends at the parity it began with.
+// Captured when first needed.  A frame of 4 substeps at 8k particles, single
+// graphs / a chain: 118 / 108 us; 113k 159 / 156; no difference from 2M on.
+constexpr int kChain = 4;
+
+// The chain from the current parity, or null: single substeps instead.
+cudaGraphExec_t chain_graph(mpm_engine* e) {
+    const int par = e->parity;
+    if (e->chain[par] || e->chain_off || e->timing_cap > 0) return e->timing_cap > 0 ? nullptr : e->chain[par];
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(e->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return nullptr;  // the caller's own capture
+    }
+    e->chain_off = true;
+    if (cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    int launches = 0;
+    for (int k = 0; k < kChain; ++k) launches += enqueue_substep(e, par ^ (k & 1), MPM_STAGE_SORT, MPM_STAGE_G2P);
+    const bool launched = cudaGetLastError() == cudaSuccess;
+    cudaGraph_t g = nullptr;
+    const bool ended = cudaStreamEndCapture(e->stream, &g) == cudaSuccess;
+    e->chain_off = !(launched && ended && cudaGraphInstantiate(&e->chain[par], g, 0) == cudaSuccess);
+    if (g) cudaGraphDestroy(g);
+    if (e->chain_off) {
+        cudaGetLastError();
+        e->chain[par] = nullptr;
+    }
+    e->chain_kernels[par] = launches;
+    return e->chain[par];
 }
 
 void free_timing(mpm_engine* e) {
@@ -561,8 +617,8 @@ mpm_status load_states(mpm_engine* e, const float* const* soa26_host, bool init_
     e->health = 0;
     mpm_status st = export_positions(e);
     if (st != MPM_OK) return st;
-    st = capture_graphs(e);
-    if (st != MPM_OK) return st;
+    if (graphs_fit(e)) destroy_learned_graphs(e);
+    else if ((st = capture_graphs(e)) != MPM_OK) return st;
     e->initialized = true;
     return sync_and_collect(e);
 }
@@ -604,6 +660,16 @@ mpm_status run_steps(mpm_engine* e, int32_t nsub) {
         e->accum_dirty = false;
     }
     for (int s = 0; s < nsub; ++s) {
+        while (nsub - s >= kChain) {
+            const cudaGraphExec_t chain = chain_graph(e);
+            if (!chain) break;
+            CK(e, cudaGraphLaunch(chain, e->stream));
+            e->kernel_launches += e->chain_kernels[e->parity];
+            e->sort_src = e->parity ^ 1;
+            e->substeps += kChain;
+            s += kChain;
+        }
+        if (s == nsub) break;
         if (e->timing_cap > 0) {
             const int par = e->parity;
             const bool slot = e->timing_used < e->timing_cap;
@@ -1484,6 +1550,7 @@ extern "C" mpm_status mpm_set_stage_timing(mpm_engine* e, int32_t max_substeps) 
         for (int i = 0; i < total; ++i) CK(e, cudaEventCreate(&e->tev[i]));
     }
     if (e->initialized) return capture_graphs(e);
+    destroy_graphs(e);  // they may embed the earlier timing events
     return MPM_OK;
 }
 
