@@ -121,6 +121,7 @@ struct mpm_engine {
     uint32_t* ctl = nullptr;
     mpm::OrderCtl order{};
     uint32_t* d_flags = nullptr;  // [0] health bits, [1] kernel status bits
+    uint32_t* h_flags = nullptr;  // their values at the last positions export (mapped host memory)
     uint32_t wait_test = 0;       // MPM_WAIT_TEST_* (test hooks of the bounded device waits)
 
     float* staging = nullptr;  // device staging for imports/exports
@@ -540,10 +541,14 @@ void free_timing(mpm_engine* e) {
     e->timing_used = 0;
 }
 
-mpm_status sync_and_collect(mpm_engine* e) {
+// Waits for the stream and collects the flags.  `exported`: nothing has been
+// enqueued since export_positions, which left them in h_flags.
+mpm_status sync_and_collect(mpm_engine* e, bool exported = false) {
     uint32_t flags[2] = {0, 0};
-    CK(e, cudaMemcpyAsync(flags, e->d_flags, sizeof(flags), cudaMemcpyDeviceToHost, e->stream));
+    exported = exported && e->n > 0;
+    if (!exported) CK(e, cudaMemcpyAsync(flags, e->d_flags, sizeof(flags), cudaMemcpyDeviceToHost, e->stream));
     CK(e, cudaStreamSynchronize(e->stream));
+    if (exported) flags[0] = e->h_flags[0], flags[1] = e->h_flags[1];
     e->health |= flags[0];
     if (flags[1] & (mpm::kStatusTimeout | mpm::kStatusBinning | mpm::kStatusCrowdList)) {
         CK(e, cudaMemsetAsync(e->d_flags + 1, 0, sizeof(uint32_t), e->stream));
@@ -643,7 +648,8 @@ mpm_status export_positions(mpm_engine* e) {
     const int b = 1 - e->pos_cur;
     CK(e, cudaStreamWaitEvent(e->stream, e->copy_done[b], 0));
     e->kernel_launches +=
-        mpm::launch_positions_export(e->n, e->P[e->parity], e->sigma[e->parity], e->pos_buf[b], e->stream);
+        mpm::launch_positions_export(e->n, e->P[e->parity], e->sigma[e->parity], e->pos_buf[b], e->d_flags,
+                                     e->h_flags, e->stream);
     CK(e, cudaGetLastError());
     CK(e, cudaEventRecord(e->pos_ready[b], e->stream));
     e->pos_cur = b;
@@ -819,6 +825,7 @@ mpm_status create_engine(const mpm_config* cfgs, int32_t count, int32_t device, 
         (err = cudaMalloc(&e->vgrid, (size_t)g_total * sizeof(float4))) != cudaSuccess ||
         (err = cudaMalloc(&e->sdf, (size_t)g_total * sizeof(float))) != cudaSuccess ||
         (err = cudaMalloc(&e->d_flags, 2 * sizeof(uint32_t))) != cudaSuccess ||
+        (err = cudaHostAlloc(&e->h_flags, 2 * sizeof(uint32_t), cudaHostAllocMapped)) != cudaSuccess ||
         (err = cudaMalloc(&e->ctl, kCtlBytes)) != cudaSuccess ||
         (err = cudaMalloc(&e->bins_mem, bins_bytes(e))) != cudaSuccess ||
         (err = cudaMalloc(&e->tiles_mem, tiles_bytes(e))) != cudaSuccess ||
@@ -1137,6 +1144,7 @@ extern "C" void mpm_destroy(mpm_engine* e) {
     free_dev(e->d_goff);
     free_dev(e->d_boff);
     free_dev(e->d_flags);
+    if (e->h_flags) cudaFreeHost(e->h_flags);
     free_dev(e->staging);
     free_dev(e->d_prm_large);
     free_dev(e->mlp);
@@ -1264,7 +1272,7 @@ extern "C" mpm_status mpm_step(mpm_engine* e, int32_t nsub) {
     mpm_status s = enter(e);
     if (s != MPM_OK) return s;
     if ((s = run_steps(e, nsub)) != MPM_OK) return s;
-    if ((s = sync_and_collect(e)) != MPM_OK) return s;
+    if ((s = sync_and_collect(e, true)) != MPM_OK) return s;
     return check_health(e);
 }
 
@@ -1686,7 +1694,7 @@ extern "C" mpm_status mpm_step_learned(mpm_engine* e, int32_t nlarge, mpm_learne
         stats->fallbacks = e->fallbacks;
         stats->last_density_change = e->last_density_change;
     }
-    if ((s = sync_and_collect(e)) != MPM_OK) return s;
+    if ((s = sync_and_collect(e, true)) != MPM_OK) return s;
     return check_health(e);
 }
 

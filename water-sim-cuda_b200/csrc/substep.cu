@@ -1432,11 +1432,16 @@ __global__ void __launch_bounds__(256) state_export_kernel(SimParams p, const fl
 // fetched for it (2M particles: 199 MB read, 5.7 TB/s), and laying out the
 // triples in shared memory for denser stores changed nothing.
 // One launch for all scenes, not one each: 64 scenes with 6.1M particles 290 /
-// 99 us; 2M particles 38.5 us either way.
+// 99 us; 2M particles 38.5 us either way.  The export follows every frame, so it
+// also hands the two flag words to the host, in mapped memory: a copy of its
+// own for eight bytes cost a frame about 7 us.
 __global__ void __launch_bounds__(256) positions_export_kernel(long long n, const float* __restrict__ P,
                                                                const int32_t* __restrict__ sigma,
-                                                               float* __restrict__ xyz) {
+                                                               float* __restrict__ xyz,
+                                                               const uint32_t* __restrict__ flags,
+                                                               uint32_t* __restrict__ flags_host) {
     const long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (j < 2) flags_host[j] = flags[j];
     if (j >= n) return;
     const long long o = __ldg(sigma + j);
     const float4 q = __ldg(reinterpret_cast<const float4*>(P + (size_t)j * kAFloats));
@@ -1613,9 +1618,10 @@ int launch_state_export(const SimParams& p, const float* P, const int32_t* sigma
     return 1;
 }
 
-int launch_positions_export(long long n, const float* P, const int32_t* sigma, float* xyz, cudaStream_t st) {
+int launch_positions_export(long long n, const float* P, const int32_t* sigma, float* xyz, const uint32_t* flags,
+                            uint32_t* flags_host, cudaStream_t st) {
     if (n <= 0) return 0;
-    positions_export_kernel<<<blocks_for(n, 256), 256, 0, st>>>(n, P, sigma, xyz);
+    positions_export_kernel<<<blocks_for(n, 256), 256, 0, st>>>(n, P, sigma, xyz, flags, flags_host);
     return 1;
 }
 
