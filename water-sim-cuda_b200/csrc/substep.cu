@@ -1037,18 +1037,20 @@ enum G2PMode : int { kG2PPlain = 0, kG2PLearned = 1, kG2PCollect = 2, kG2PLarge 
 // G2P per substep before / after (with 128-thread CTAs, whose barrier waits for
 // fewer warps: 94 us at 256; and with reductions instead of returning atomics
 // in the filing): 650k particles 37.6 / 30.4 us, 2M 104 / 83 us, 6.9M in 256^3
-// 325 / 258 us, the 64-scene batch 362 / 291 us.  DRAM then carries 3.9 of the
+// 325 / 258 us, the 64-scene batch 362 / 263 us.  DRAM then carries 3.9 of the
 // 6.5 TB/s; issue (57 % of slots) and the chain gidx - record - stores bound it.
 constexpr int kStagePlanes = 9;  // planes of 60 nodes: 8.6 KB per CTA
 
 // CTAs per SM: the learned tcgen05 mode fits four (64 registers, 128 TMEM
 // columns and about 45 KB of shared memory each), so one CTA's MMA waits
-// overlap the other three's work; mma.sync learned, collect and batched
-// modes need more registers.  The tcgen05 mode at 2M particles: 330 us with
+// overlap the other three's work; mma.sync learned and collect modes and the
+// batched large steps need more registers.  The batched substep would like 80
+// (64 spill 72 bytes), but a fourth CTA is worth more: 64 scenes with 6.1M
+// particles 291 / 263 us.  The tcgen05 mode at 2M particles: 330 us with
 // per-warp statistics, node-by-node sums and scalar GELU, 225 us now (three
 // CTAs of 80 registers without spills: 254 against 243 us before the row sums).
 template <bool kBatch, int kMode>
-__global__ void __launch_bounds__(256, kMode == 1 ? 2 : ((kBatch || kMode == 2) ? 3 : 4)) g2p_kernel(
+__global__ void __launch_bounds__(256, kMode == 1 ? 2 : (((kBatch && kMode != 0) || kMode == 2) ? 3 : 4)) g2p_kernel(
     SceneTable sc, SimParams p0, long long n_total, const float* __restrict__ Pin, float* __restrict__ Pout,
     const int32_t* __restrict__ gidx, const int2* __restrict__ edge, const int32_t* __restrict__ sig_in,
     int32_t* __restrict__ sig_out, const float4* __restrict__ vgrid_all, const float* __restrict__ sdf_all,
