@@ -39,13 +39,26 @@ def _meshes():
     }
 
 
+def _split(tris):
+    """Every triangle in four, at its edges' midpoints."""
+    a, b, c = np.split(tris.reshape(-1, 9), 3, axis=1)
+    h = np.float32(0.5)
+    ab, bc, ca = (a + b) * h, (b + c) * h, (c + a) * h
+    return np.concatenate([np.concatenate(q, 1) for q in ((a, ab, ca), (ab, b, bc), (ca, bc, c), (ab, bc, ca))])
+
+
+# Few nodes and triangles are summed at every node whatever the mesh: split
+# until the line (5e7 pairs, at least 65536 nodes counted) is passed.
+@pytest.mark.parametrize("split", [False, True])
 @pytest.mark.parametrize("name", sorted(["hole", "one_triangle", "one_flipped", "box_on_nodes", "inside_out", "nested",
                                          "crossing", "plate", "outside", "31_triangles", "33_triangles", "one_node",
                                          "degenerate", "needle"]))
-def test_sdf_sign_forms(gpu_ok, mpm, oracle64, name):
+def test_sdf_sign_forms(gpu_ok, mpm, oracle64, name, split):
     from mpm_b200 import scenes
     size, tris = _meshes()[name]
     tris = np.ascontiguousarray(tris, np.float32)
+    while split and len(tris) * max(int(np.prod(size)), 65536) <= 5e7:
+        tris = np.ascontiguousarray(_split(tris), np.float32)
     cfg = scenes._cfg(size)
     with mpm.Engine(cfg) as eng:
         eng.init_sdf(tris)

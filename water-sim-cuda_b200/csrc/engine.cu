@@ -2,12 +2,12 @@
 //
 // Restates the reference's `Engine` (engine.h:14-43, engine.cu:36-114) and
 // the config upload (config.cu:5-8, Simulation.cpp:56-77) with per-engine
-// state: one device, one stream, and a CUDA graph per substep parity.  An
-// engine holds one or more independent scenes (the batched form): their
-// particle, grid, cell and bin arrays are concatenated, a device table of
-// SimParams carries each scene's constants and offsets, and every substep
-// stage is one launch over all scenes.  The reference's single Engine is an
-// engine of one scene.
+// state: one device, one stream, and CUDA graphs of one substep and of four
+// per parity.  An engine holds one or more independent scenes (the batched
+// form): their particle, grid, cell and bin arrays are concatenated, a device
+// table of SimParams carries each scene's constants and offsets, and every
+// substep stage is one launch over all scenes.  The reference's single Engine
+// is an engine of one scene.
 //
 // Particle order.  The reference never moves particle data: every substep it
 // sorts (Morton key, 0..n-1) and gathers through the permutation, so that
@@ -16,8 +16,10 @@
 // 8 x 4 x 4 cells, which is what the P2G kernel needs: all particles of a
 // cell scatter to the same 27 nodes.  A substep from parity p, state P[p]
 // filed into counter set p:
-//   bin order: bin and cell starts from set p, gidx[new slot] = old slot;
-//   P2G: one warp per (bin, layer) item, lane = cell, reading P[p] via gidx;
+//   ordering: bin list, bin and cell starts from set p, P2G's items and the
+//       crowded-cell list, gidx[new slot] = old slot;
+//   P2G: one warp per item of 32 cells of a bin, lane = cell, reading P[p] via
+//       gidx, and per chunk of a crowded cell;
 //   grid update;
 //   G2P reads P[p] through gidx and writes P[1-p] at the new slot, i.e. the
 //       state is regrouped for free, carries sigma (slot -> original slot)
@@ -1212,28 +1214,26 @@ extern "C" mpm_status mpm_scene_init_sdf(mpm_engine* e, int32_t scene, const flo
         CK(e, cudaStreamSynchronize(e->stream));
         return MPM_OK;
     }
-    // One allocation: the triangles as given, then the sorted copy with its
-    // boxes (sdf.cu).  cudaMalloc: 256-byte aligned, as the kernel's
+    // One allocation and one copy: the triangles as given, then the sorted copy
+    // with its boxes (sdf.cu).  cudaMalloc: 256-byte aligned, as the kernel's
     // 16-byte bulk copies need; each part starts on a 16-byte boundary and 16
     // spare bytes cover the last tile's copy rounded up to 16 bytes.
-    const size_t bytes = (size_t)t * 9 * sizeof(float);
-    const size_t off = align_up(bytes, 16) + 16;
-    const size_t aux_floats = mpm::sdf_aux_floats((int)t);
-    std::vector<float> aux(aux_floats, 0.0f);
-    const bool closed = mpm::sdf_prepare_host(tris, (int)t, aux.data());
+    const size_t floats = (size_t)t * 9;
+    const size_t off = align_up(floats, 4) + 4;
+    std::vector<float> parts(off + mpm::sdf_aux_floats((int)t) + 4, 0.0f);
+    std::memcpy(parts.data(), tris, floats * sizeof(float));
+    const bool spread = mpm::sdf_prepare_host(tris, (int)t, p.g, parts.data() + off);
     float* d_tris = nullptr;
-    CK(e, cudaMalloc(&d_tris, off + aux_floats * sizeof(float) + 16));
-    float* d_aux = reinterpret_cast<float*>(reinterpret_cast<char*>(d_tris) + off);
-    cudaError_t err = cudaMemsetAsync(d_tris, 0, off + aux_floats * sizeof(float) + 16, e->stream);
-    if (err == cudaSuccess) err = cudaMemcpyAsync(d_tris, tris, bytes, cudaMemcpyHostToDevice, e->stream);
-    if (err == cudaSuccess)
-        err = cudaMemcpyAsync(d_aux, aux.data(), aux_floats * sizeof(float), cudaMemcpyHostToDevice, e->stream);
+    CK(e, cudaMalloc(&d_tris, parts.size() * sizeof(float)));
+    float* d_aux = d_tris + off;
+    cudaError_t err =
+        cudaMemcpyAsync(d_tris, parts.data(), parts.size() * sizeof(float), cudaMemcpyHostToDevice, e->stream);
     if (err == cudaSuccess) {
-        e->kernel_launches += mpm::launch_sdf_build(p, d_tris, d_aux, (int)t, closed, sdf, e->d_flags + 1, e->stream,
+        e->kernel_launches += mpm::launch_sdf_build(p, d_tris, d_aux, (int)t, spread, sdf, e->d_flags + 1, e->stream,
                                                     e->wait_test & (MPM_WAIT_TEST_SDF_GIVE_UP | MPM_WAIT_TEST_SDF_EXPIRE));
         err = cudaGetLastError();
     }
-    // aux is pageable host memory: the synchronisation below ends its copy.
+    // parts is pageable host memory: the synchronisation below ends its copy.
     const mpm_status s2 = err != cudaSuccess ? cuda_fail(e, err, "sdf build") : sync_and_collect(e);
     if (err != cudaSuccess) cudaStreamSynchronize(e->stream);
     cudaFree(d_tris);

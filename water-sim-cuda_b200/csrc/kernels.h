@@ -177,13 +177,14 @@ int launch_grid_export(const SimParams& p, const float4* grid, float* planes4, c
 // tris: 9*t floats on the device, allocation padded by >= 16 bytes.  aux:
 // sdf_aux_floats(t) floats on the device (16-byte aligned) holding what
 // sdf_prepare_host wrote: the triangles sorted by the Morton code of their
-// centroids, and the boxes of the triangles and of groups of them.  closed:
-// what sdf_prepare_host returned, whether the mesh is closed.
+// centroids, and the boxes of the triangles and of groups of them.  spread:
+// what sdf_prepare_host returned, whether the sign is spread (a closed mesh,
+// and enough nodes and triangles) or summed at every node.
 // wait_test: test hooks of the first triangle tile's wait (kWaitTestGiveUp /
 // kWaitTestExpire, corrector_tc.cuh), acted on after the real completion.
 size_t sdf_aux_floats(int t);
-bool sdf_prepare_host(const float* tris, int t, float* aux);
-int launch_sdf_build(const SimParams& p, const float* tris, const float* aux, int t, bool closed, float* sdf,
+bool sdf_prepare_host(const float* tris, int t, long long nodes, float* aux);
+int launch_sdf_build(const SimParams& p, const float* tris, const float* aux, int t, bool spread, float* sdf,
                      uint32_t* status, cudaStream_t st, uint32_t wait_test = 0u);
 int launch_fill(float* dst, long long count, float value, cudaStream_t st);
 // The learned step's fallback decision (one thread): rule 0 / 1 / 2 =

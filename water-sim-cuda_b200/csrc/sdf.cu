@@ -26,7 +26,8 @@
 //     distance, spreads its sign through overlapping balls, and repeats for
 //     the nodes left.  Nodes within kSdfOnMesh of the mesh, where the sum
 //     itself decides, get the sum over every triangle in the order given.
-//     Other meshes: sdf_winding_kernel takes that sum for every node.
+//     Other meshes, and small ones on small grids (kSumPairs):
+//     sdf_winding_kernel takes that sum for every node.
 //     Both stream triangles through shared memory in tiles of 512: one thread
 //     issues a bulk async copy (cp.async.bulk, the 1-D TMA path) of the next
 //     tile into the second buffer while the CTA evaluates the current one,
@@ -49,6 +50,7 @@
 #include <vector>
 
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace mpm {
 namespace {
@@ -238,6 +240,7 @@ static_assert(kBrickX * kBrickY * kBrickZ == kSdfThreads, "one node per thread")
 __global__ void __launch_bounds__(kSdfThreads) sdf_winding_kernel(SimParams p, const float* __restrict__ tris,
                                                                   int t_count, float* __restrict__ sdf,
                                                                   uint32_t* __restrict__ status, uint32_t wait_test) {
+    pdl_wait();
     __shared__ __align__(128) float s_tri[2][kTriTile * kTriFloats];
     __shared__ __align__(8) uint64_t s_bar[2];
     const int nbx = (p.sx + kBrickX - 1) / kBrickX, nby = (p.sy + kBrickY - 1) / kBrickY;
@@ -383,6 +386,7 @@ enum : uint8_t { kSignOpen = 0, kSignOut = 1, kSignIn = 2, kSignSum = 3 };
 __global__ void __launch_bounds__(kSdfThreads) sdf_sign_kernel(SimParams p, const float* __restrict__ tris, int t_count,
                                                                float* __restrict__ sdf, uint32_t* __restrict__ status,
                                                                uint32_t wait_test) {
+    pdl_wait();
     __shared__ __align__(128) float s_tri[2][kTriTile * kTriFloats];
     __shared__ __align__(8) uint64_t s_bar[2];
     __shared__ float s_d[kSignNodes];
@@ -607,7 +611,14 @@ size_t sdf_aux_floats(int t) {
     return (size_t)t * (kAuxTri + kAuxBox) + groups * kAuxBox;
 }
 
-bool sdf_prepare_host(const float* tris, int t, float* aux) {
+// Sums over every triangle for every node (sdf_winding_kernel) below this many
+// pairs, a grid counting for at least kSumNodes nodes (what fills the GPU): the
+// sign kernel's chain of sums takes 150 to 370 us on any mesh.  Sign / sums:
+// 12 triangles at 128^3 262 / 160 us, 48 at 64^3 319 / 80 and at 128^3 306 / 585,
+// 192 at 64^3 349 / 307, 480 at 32^3 193 / 181, 960 at 32^3 196 / 357.
+constexpr long long kSumPairs = 50000000, kSumNodes = 65536;
+
+bool sdf_prepare_host(const float* tris, int t, long long nodes, float* aux) {
     float lo[3] = {1e30f, 1e30f, 1e30f}, hi[3] = {-1e30f, -1e30f, -1e30f};
     for (int i = 0; i < t; ++i)
         for (int k = 0; k < 9; ++k) {
@@ -651,10 +662,10 @@ bool sdf_prepare_host(const float* tris, int t, float* aux) {
         box(l, h, tbox + (size_t)i * kAuxBox);
         if (i % kGroup == kGroup - 1 || i == t - 1) box(gl, gh, gbox + (size_t)(i / kGroup) * kAuxBox);
     }
-    return closed_mesh(tris, t);
+    return t * std::max(nodes, kSumNodes) > kSumPairs && closed_mesh(tris, t);
 }
 
-int launch_sdf_build(const SimParams& p, const float* tris, const float* aux, int t, bool closed, float* sdf,
+int launch_sdf_build(const SimParams& p, const float* tris, const float* aux, int t, bool spread, float* sdf,
                      uint32_t* status, cudaStream_t st, uint32_t wait_test) {
     if (p.g <= 0 || t <= 0) return 0;
     auto bricks = [&](int ex, int ey, int ez) {
@@ -664,12 +675,12 @@ int launch_sdf_build(const SimParams& p, const float* tris, const float* aux, in
     const float4* tbox = reinterpret_cast<const float4*>(aux + (size_t)t * kAuxTri);
     const float4* gbox = reinterpret_cast<const float4*>(aux + (size_t)t * (kAuxTri + kAuxBox));
     sdf_distance_kernel<<<(unsigned)((bricks(4, 4, 2) + 7) / 8), 256, 0, st>>>(p, tri, tbox, gbox, t, sdf);
-    if (closed)
-        sdf_sign_kernel<<<(unsigned)bricks(kSignCore, kSignCore, kSignCore), kSdfThreads, 0, st>>>(p, tris, t, sdf, status,
-                                                                                                  wait_test);
+    if (spread)
+        launch_dep(sdf_sign_kernel, (unsigned)bricks(kSignCore, kSignCore, kSignCore), kSdfThreads, 0, st, p, tris, t, sdf,
+                   status, wait_test);
     else
-        sdf_winding_kernel<<<(unsigned)bricks(kBrickX, kBrickY, kBrickZ), kSdfThreads, 0, st>>>(p, tris, t, sdf, status,
-                                                                                               wait_test);
+        launch_dep(sdf_winding_kernel, (unsigned)bricks(kBrickX, kBrickY, kBrickZ), kSdfThreads, 0, st, p, tris, t, sdf,
+                   status, wait_test);
     return 2;
 }
 
