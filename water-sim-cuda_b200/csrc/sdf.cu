@@ -552,11 +552,17 @@ static uint32_t morton10(float x, float y, float z) {
 
 // Whether the winding number is a whole number off the mesh and the kernels
 // may rely on the distances: every edge is run through as often one way as the
-// other (vertices compared by value), the coordinates are moderate, and no
-// triangle is a needle (height below a thousandth of its longest edge), whose
-// distance FP32 can miss.  The edges are matched by adding up a 128-bit hash
+// other (vertices compared by value), and FP32 distances are good to half of
+// the 0.001 by which the sign kernel's balls fall short of them.  They err by a
+// few units in the last place of the coordinates, hence kSpreadCoord, and on
+// long thin triangles by the barycentric coordinates' cancellation, which
+// grows like L (L / h)^2 with the longest edge L and the height h: in FP32
+// against 64 bits over rotated boxes at most 1e-4 at 1.6e4, 8e-4 at 1.1e5 and
+// 2.3e-3 at 2.5e5, hence kSpreadSliver.  The edges are matched by adding up a 128-bit hash
 // of each, with the sign of its direction: the sums vanish when every edge
 // cancels, and else with a probability of 2^-128.
+constexpr float kSpreadCoord = 1024.0f;
+constexpr double kSpreadSliver = 4e4;
 static bool closed_mesh(const float* tris, int t) {
     auto mix = [](uint64_t v) {  // the finaliser of MurmurHash3 (public domain)
         v ^= v >> 33;
@@ -573,7 +579,7 @@ static bool closed_mesh(const float* tris, int t) {
             uint32_t b[3];
             for (int a = 0; a < 3; ++a) {
                 const float f = v[3 * k + a] + 0.0f;  // -0 becomes 0
-                if (!(std::fabs(f) <= 16384.0f)) return false;
+                if (!(std::fabs(f) <= kSpreadCoord)) return false;
                 std::memcpy(&b[a], &f, 4);
             }
             const uint64_t xy = ((uint64_t)b[0] << 32) | b[1];
@@ -592,7 +598,8 @@ static bool closed_mesh(const float* tris, int t) {
         }
         const double nx = e[0][1] * e[1][2] - e[0][2] * e[1][1], ny = e[0][2] * e[1][0] - e[0][0] * e[1][2],
                      nz = e[0][0] * e[1][1] - e[0][1] * e[1][0];
-        if (nx * nx + ny * ny + nz * nz < 1e-6 * longest * longest || longest == 0.0) return false;
+        // L (L / h)^2 = L^5 / |n|^2, n the cross product of two edges
+        if (!(longest * longest * std::sqrt(longest) < kSpreadSliver * (nx * nx + ny * ny + nz * nz))) return false;
         for (int k = 0; k < 3; ++k)
             for (int w = 0; w < 2; ++w) {
                 const uint64_t a = h[k][w], b = h[(k + 1) % 3][w];
@@ -639,12 +646,14 @@ bool sdf_prepare_host(const float* tris, int t, long long nodes, float* aux) {
     float* sorted = aux;
     float* tbox = aux + (size_t)t * kAuxTri;
     float* gbox = tbox + (size_t)t * kAuxBox;
-    // Centre and half extents of [lo, hi], the latter rounded up to cover it.
+    // Centre and half extents of [lo, hi], the latter enlarged to cover it with
+    // room for the rounding of the kernel's differences with centre and extents.
     auto box = [](const float* l, const float* h, float* out) {
         float half[3];
         for (int a = 0; a < 3; ++a) {
             out[a] = 0.5f * l[a] + 0.5f * h[a];
-            half[a] = std::nextafter(std::max(h[a] - out[a], out[a] - l[a]), INFINITY);
+            half[a] = std::max(h[a] - out[a], out[a] - l[a]);
+            half[a] = std::nextafter(half[a] + 5e-7f * (std::fabs(out[a]) + half[a]), INFINITY);
         }
         out[3] = half[0], out[4] = half[1], out[5] = half[2], out[6] = out[7] = 0.0f;
     };
