@@ -143,6 +143,11 @@ __device__ __forceinline__ int cell_of(const SimParams& p, float x, float y, flo
     return b * kBinCells + ((uz % kBinZ) * kBinY + uy % kBinY) * kBinX + ux % kBinX;
 }
 
+// Whether o <= b < o + n, for any b (stencil_base saturates: a particle at 2^31
+// or beyond, infinities among them, has a base that a sum would wrap), n >= 0
+// and |o| + n below 2^30.
+__host__ __device__ __forceinline__ bool in_range(int b, int o, int n) { return (unsigned)b - (unsigned)o < (unsigned)n; }
+
 // Node (0, 0, 0) of the stencil of the bin's first cell.  Bins number below
 // 2^24 (cells below 2^31), so the products stay below 2^64 and the quotients
 // by the reciprocals rounded up are exact: with m = (2^48 + e) / d, 0 <= e < d,

@@ -1092,9 +1092,9 @@ __global__ void __launch_bounds__(256, kMode == 1 ? 2 : (((kBatch && kMode != 0)
     const float4* vgrid = vgrid_all + p.goff;
     const float* sdf = sdf_all + p.goff;
     const int src = __ldg(gidx + j);
-    // The CTA's two regions: node origin (o*) of the first staged plane, and
-    // planes (nz*).
-    int ox0, oy0, oz0, nz0, ox1, oy1, oz1, nz1;
+    // The CTA's two regions: node origin (o*) of the first staged plane, layers
+    // of stencil bases (lz*), and planes (nz*: two more than layers).
+    int ox0, oy0, oz0, lz0, nz0, ox1, oy1, oz1, lz1;
     const int scene0 = look.scene(cta0), scene1 = look.scene(cta1 - 1);
     {
         const SimParams& pa = kBatch ? look.params(scene0) : p0;
@@ -1104,9 +1104,11 @@ __global__ void __launch_bounds__(256, kMode == 1 ? 2 : (((kBatch && kMode != 0)
         const int bin0 = l0 / kBinCells, bin1 = l1 / kBinCells;
         const int z0 = l0 % kBinCells / 32, z1 = l1 % kBinCells / 32;
         const bool one = bin0 == bin1 && scene0 == scene1;
-        nz0 = bin0 >= pa.nb ? 0 : (one ? z1 : kBinZ - 1) - z0 + 3;  // the overflow bin reaches no node
-        nz1 = one || bin1 >= pb.nb ? 0 : z1 + 3;
-        if (nz0 + nz1 > kStagePlanes) nz1 = 0;
+        lz0 = bin0 >= pa.nb ? 0 : (one ? z1 : kBinZ - 1) - z0 + 1;  // the overflow bin reaches no node
+        lz1 = one || bin1 >= pb.nb ? 0 : z1 + 1;
+        nz0 = lz0 > 0 ? lz0 + 2 : 0;
+        if (nz0 + lz1 + 2 > kStagePlanes) lz1 = 0;
+        const int nz1 = lz1 > 0 ? lz1 + 2 : 0;
         bin_origin(pa, bin0, &ox0, &oy0, &oz0);
         bin_origin(pb, bin1, &ox1, &oy1, &oz1);
         oz0 += z0;
@@ -1157,11 +1159,9 @@ __global__ void __launch_bounds__(256, kMode == 1 ? 2 : (((kBatch && kMode != 0)
     // This particle's first node in the staged planes, -1 if it is in neither
     // region.
     int at = -1;
-    if ((!kBatch || scene == scene1) && (unsigned)(bx - ox1) < kBinX && (unsigned)(by - oy1) < kBinY && bz >= oz1 &&
-        bz - oz1 + 3 <= nz1)
+    if ((!kBatch || scene == scene1) && in_range(bx, ox1, kBinX) && in_range(by, oy1, kBinY) && in_range(bz, oz1, lz1))
         at = ((nz0 + bz - oz1) * kTY + by - oy1) * kTX + bx - ox1;
-    if ((!kBatch || scene == scene0) && (unsigned)(bx - ox0) < kBinX && (unsigned)(by - oy0) < kBinY && bz >= oz0 &&
-        bz - oz0 + 3 <= nz0)
+    if ((!kBatch || scene == scene0) && in_range(bx, ox0, kBinX) && in_range(by, oy0, kBinY) && in_range(bz, oz0, lz0))
         at = ((bz - oz0) * kTY + by - oy0) * kTX + bx - ox0;
     // The SDF at the particle, for the features: loaded while the nodes arrive.
     constexpr bool kFeatures = kMode == kG2PLearned || kMode == kG2PCollect || kMode == kG2PLearnedTc;
