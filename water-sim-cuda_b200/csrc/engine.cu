@@ -135,10 +135,14 @@ struct mpm_engine {
     bool accum_dirty = false;
     GridView grid_view = GridView::kVelocity;
 
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};
-    cudaGraph_t graph_src[2] = {nullptr, nullptr};
+    // Captured when first needed; stale: to be captured again before its next
+    // launch (reset_graphs).
+    cudaGraphExec_t graph[2] = {nullptr, nullptr};  // one substep from parity 0 / 1
+    cudaGraph_t graph_src[2] = {nullptr, nullptr};  // kept for the nodes of the stage timing
+    bool graph_stale[2] = {false, false};
     int graph_kernels[2] = {0, 0};
-    cudaGraphExec_t chain[2] = {nullptr, nullptr};  // kChain substeps from parity 0 / 1, captured when first needed
+    cudaGraphExec_t chain[2] = {nullptr, nullptr};  // kChain substeps from parity 0 / 1
+    bool chain_stale[2] = {false, false};
     int chain_kernels[2] = {0, 0};
     bool chain_off = false;  // the chains could not be captured
     // What the graphs embed beside addresses that change with the particle
@@ -437,58 +441,90 @@ int enqueue_substep(mpm_engine* e, int par, int from, int upto, const cudaEvent_
     return launches;
 }
 
-mpm_status capture_graphs(mpm_engine* e) {
+// The substep graphs are captured again, with the launch shapes and sizes of
+// now, when next launched (substep_graph, chain_graph).  Their executables are
+// kept to be updated in place, but for those with stage-timing nodes.
+mpm_status reset_graphs(mpm_engine* e) {
     destroy_learned_graphs(e);  // they embed the launch shapes too
     // Touched tiles only: after updates of every node any tile may hold
     // velocities, so the first tile update resets every tile not marked.
     if (active_tiles(e).mark) CK(e, cudaMemsetAsync(e->tiles.dirty, 1, (size_t)e->bins_total, e->stream));
-    const bool timed = e->timing_cap > 0;
-    destroy_graphs(e);
-    for (int par = 0; par < 2; ++par) {
-        cudaGraph_t g = nullptr;
-        CK(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
-        const int launches = enqueue_substep(e, par, MPM_STAGE_SORT, MPM_STAGE_G2P, timed ? e->tscratch : nullptr);
-        const cudaError_t launch_err = cudaGetLastError();
-        const cudaError_t end_err = cudaStreamEndCapture(e->stream, &g);
-        if (launch_err != cudaSuccess) {
-            if (g) cudaGraphDestroy(g);
-            return cuda_fail(e, launch_err, "substep capture");
-        }
-        CK(e, end_err);
-        e->graph_src[par] = g;
-        if (timed) {
-            for (int k = 0; k < mpm_engine::kTimingMarks; ++k) e->tnode[par][k] = nullptr;
-            // Find the event-record nodes by the scratch event each records.
-            size_t count = 0;
-            CK(e, cudaGraphGetNodes(g, nullptr, &count));
-            std::vector<cudaGraphNode_t> nodes(count);
-            CK(e, cudaGraphGetNodes(g, nodes.data(), &count));
-            for (cudaGraphNode_t nd : nodes) {
-                cudaGraphNodeType type;
-                CK(e, cudaGraphNodeGetType(nd, &type));
-                if (type != cudaGraphNodeTypeEventRecord) continue;
-                cudaEvent_t ev;
-                CK(e, cudaGraphEventRecordNodeGetEvent(nd, &ev));
-                for (int k = 0; k < mpm_engine::kTimingMarks; ++k)
-                    if (ev == e->tscratch[k]) e->tnode[par][k] = nd;
-            }
-            for (int k = 0; k < mpm_engine::kTimingMarks; ++k)
-                if (!e->tnode[par][k]) return record(e, MPM_ERR_CUDA, "stage-timing event node missing from the graph");
-        }
-        CK(e, cudaGraphInstantiate(&e->graph[par], g, 0));
-        e->graph_kernels[par] = launches;
-    }
+    if (e->timing_cap > 0 || e->graph_timing > 0) destroy_graphs(e);
+    for (int k = 0; k < 2; ++k) e->graph_stale[k] = e->chain_stale[k] = true;
+    e->chain_off = false;
     e->graph_prm = e->prm;
     e->graph_tune = e->tune;
     e->graph_timing = e->timing_cap;
     return MPM_OK;
 }
 
-// Whether the captured graphs fit the current state.  Capturing them for every
-// new state took most of a small one's init: 8k particles 333 / 92 us.
+// Makes *exec run `g`: a captured sequence of the same kernels as before, with
+// other counts and grid sizes, updates the executable in place; else a new one.
+// Load of a state of another count / load and a frame of four substeps, 8k
+// particles: both single graphs captured and instantiated in the load, then the
+// chain, 361 / 643 us; only the chain, updated, 125 / 257 us (a state of the
+// same count, whose graphs are kept: 125 / 227 us).
+cudaError_t load_graph(cudaGraphExec_t* exec, cudaGraph_t g) {
+    if (*exec) {
+        cudaGraphExecUpdateResultInfo info;
+        if (cudaGraphExecUpdate(*exec, g, &info) == cudaSuccess) return cudaSuccess;
+        cudaGetLastError();
+        cudaGraphExecDestroy(*exec);
+        *exec = nullptr;
+    }
+    return cudaGraphInstantiate(exec, g, 0);
+}
+
+// Makes graph[par], one substep from parity `par`, fit to be launched.  A frame
+// of four substeps launches none (chain_graph), so that init captures nothing.
+mpm_status substep_graph(mpm_engine* e, int par) {
+    if (e->graph[par] && !e->graph_stale[par]) return MPM_OK;
+    const bool timed = e->timing_cap > 0;
+    cudaGraph_t g = nullptr;
+    CK(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
+    const int launches = enqueue_substep(e, par, MPM_STAGE_SORT, MPM_STAGE_G2P, timed ? e->tscratch : nullptr);
+    const cudaError_t launch_err = cudaGetLastError();
+    const cudaError_t end_err = cudaStreamEndCapture(e->stream, &g);
+    if (launch_err != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
+        return cuda_fail(e, launch_err, "substep capture");
+    }
+    CK(e, end_err);
+    e->graph_kernels[par] = launches;
+    if (!timed) {
+        const cudaError_t err = load_graph(&e->graph[par], g);
+        cudaGraphDestroy(g);
+        CK(e, err);
+    } else {
+        if (e->graph_src[par]) cudaGraphDestroy(e->graph_src[par]);  // of an attempt that failed below
+        e->graph_src[par] = g;
+        for (int k = 0; k < mpm_engine::kTimingMarks; ++k) e->tnode[par][k] = nullptr;
+        // Find the event-record nodes by the scratch event each records.
+        size_t count = 0;
+        CK(e, cudaGraphGetNodes(g, nullptr, &count));
+        std::vector<cudaGraphNode_t> nodes(count);
+        CK(e, cudaGraphGetNodes(g, nodes.data(), &count));
+        for (cudaGraphNode_t nd : nodes) {
+            cudaGraphNodeType type;
+            CK(e, cudaGraphNodeGetType(nd, &type));
+            if (type != cudaGraphNodeTypeEventRecord) continue;
+            cudaEvent_t ev;
+            CK(e, cudaGraphEventRecordNodeGetEvent(nd, &ev));
+            for (int k = 0; k < mpm_engine::kTimingMarks; ++k)
+                if (ev == e->tscratch[k]) e->tnode[par][k] = nd;
+        }
+        for (int k = 0; k < mpm_engine::kTimingMarks; ++k)
+            if (!e->tnode[par][k]) return record(e, MPM_ERR_CUDA, "stage-timing event node missing from the graph");
+        CK(e, cudaGraphInstantiate(&e->graph[par], g, 0));
+    }
+    e->graph_stale[par] = false;
+    return MPM_OK;
+}
+
+// Whether graphs captured earlier fit the current state.
 bool graphs_fit(const mpm_engine* e) {
     const mpm_tuning &a = e->graph_tune, &b = e->tune;
-    return e->graph[0] && e->graph[1] && e->graph_timing == e->timing_cap && a.p2g_ctas_per_sm == b.p2g_ctas_per_sm &&
+    return !e->graph_prm.empty() && e->graph_timing == e->timing_cap && a.p2g_ctas_per_sm == b.p2g_ctas_per_sm &&
            a.g2p_block == b.g2p_block && a.grid_block == b.grid_block && a.p2g_cell_cap == b.p2g_cell_cap &&
            e->graph_prm.size() == e->prm.size() &&
            std::memcmp(e->graph_prm.data(), e->prm.data(), e->prm.size() * sizeof(SimParams)) == 0;
@@ -496,19 +532,15 @@ bool graphs_fit(const mpm_engine* e) {
 
 // kChain substeps as one graph: three launches and the gaps of about 3 us
 // before their first kernels fewer.  A chain ends at the parity it began with.
-// Captured when first needed.  A frame of 4 substeps at 8k particles, single
+// A frame of 4 substeps at 8k particles, single
 // graphs / a chain: 118 / 108 us; 113k 159 / 156; no difference from 2M on.
 constexpr int kChain = 4;
 
 // The chain from the current parity, or null: single substeps instead.
 cudaGraphExec_t chain_graph(mpm_engine* e) {
     const int par = e->parity;
-    if (e->chain[par] || e->chain_off || e->timing_cap > 0) return e->timing_cap > 0 ? nullptr : e->chain[par];
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(e->stream, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        return nullptr;  // the caller's own capture
-    }
+    if (e->timing_cap > 0 || e->chain_off) return nullptr;
+    if (e->chain[par] && !e->chain_stale[par]) return e->chain[par];
     e->chain_off = true;
     if (cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
         cudaGetLastError();
@@ -519,12 +551,13 @@ cudaGraphExec_t chain_graph(mpm_engine* e) {
     const bool launched = cudaGetLastError() == cudaSuccess;
     cudaGraph_t g = nullptr;
     const bool ended = cudaStreamEndCapture(e->stream, &g) == cudaSuccess;
-    e->chain_off = !(launched && ended && cudaGraphInstantiate(&e->chain[par], g, 0) == cudaSuccess);
+    e->chain_off = !(launched && ended && load_graph(&e->chain[par], g) == cudaSuccess);
     if (g) cudaGraphDestroy(g);
     if (e->chain_off) {
         cudaGetLastError();
-        e->chain[par] = nullptr;
+        return nullptr;
     }
+    e->chain_stale[par] = false;
     e->chain_kernels[par] = launches;
     return e->chain[par];
 }
@@ -625,7 +658,7 @@ mpm_status load_states(mpm_engine* e, const float* const* soa26_host, bool init_
     mpm_status st = export_positions(e);
     if (st != MPM_OK) return st;
     if (graphs_fit(e)) destroy_learned_graphs(e);
-    else if ((st = capture_graphs(e)) != MPM_OK) return st;
+    else if ((st = reset_graphs(e)) != MPM_OK) return st;
     e->initialized = true;
     return sync_and_collect(e);
 }
@@ -678,18 +711,19 @@ mpm_status run_steps(mpm_engine* e, int32_t nsub) {
             s += kChain;
         }
         if (s == nsub) break;
+        const int par = e->parity;
+        if ((st = substep_graph(e, par)) != MPM_OK) return st;
         if (e->timing_cap > 0) {
-            const int par = e->parity;
             const bool slot = e->timing_used < e->timing_cap;
             const cudaEvent_t* evs = slot ? e->tev + (size_t)e->timing_used * mpm_engine::kTimingMarks : e->tscratch;
             for (int k = 0; k < mpm_engine::kTimingMarks; ++k)
                 CK(e, cudaGraphExecEventRecordNodeSetEvent(e->graph[par], e->tnode[par][k], evs[k]));
             if (slot) ++e->timing_used;
         }
-        CK(e, cudaGraphLaunch(e->graph[e->parity], e->stream));
-        e->kernel_launches += e->graph_kernels[e->parity];
-        e->sort_src = e->parity;
-        e->parity ^= 1;
+        CK(e, cudaGraphLaunch(e->graph[par], e->stream));
+        e->kernel_launches += e->graph_kernels[par];
+        e->sort_src = par;
+        e->parity = 1 - par;
         ++e->substeps;
     }
     if (nsub > 0) e->grid_view = GridView::kVelocity;
@@ -963,10 +997,13 @@ mpm_status rebin(mpm_engine* e, int par) {
 // `count` plain substeps through the captured graphs.
 mpm_status plain_substeps(mpm_engine* e, int count) {
     for (int s = 0; s < count; ++s) {
-        CK(e, cudaGraphLaunch(e->graph[e->parity], e->stream));
-        e->kernel_launches += e->graph_kernels[e->parity];
-        e->sort_src = e->parity;
-        e->parity ^= 1;
+        const int par = e->parity;
+        const mpm_status st = substep_graph(e, par);
+        if (st != MPM_OK) return st;
+        CK(e, cudaGraphLaunch(e->graph[par], e->stream));
+        e->kernel_launches += e->graph_kernels[par];
+        e->sort_src = par;
+        e->parity = 1 - par;
         ++e->substeps;
     }
     return MPM_OK;
@@ -1557,7 +1594,7 @@ extern "C" mpm_status mpm_set_stage_timing(mpm_engine* e, int32_t max_substeps) 
         e->timing_cap = max_substeps;
         for (int i = 0; i < total; ++i) CK(e, cudaEventCreate(&e->tev[i]));
     }
-    if (e->initialized) return capture_graphs(e);
+    if (e->initialized) return reset_graphs(e);
     destroy_graphs(e);  // they may embed the earlier timing events
     return MPM_OK;
 }
@@ -1980,7 +2017,7 @@ extern "C" mpm_status mpm_set_tuning(mpm_engine* e, const mpm_tuning* t) {
     e->tune.g2p_block = t->g2p_block;
     e->tune.grid_block = t->grid_block;
     e->tune.p2g_cell_cap = t->p2g_cell_cap;
-    return e->initialized ? capture_graphs(e) : MPM_OK;
+    return e->initialized ? reset_graphs(e) : MPM_OK;
 }
 
 extern "C" mpm_status mpm_get_tuning(mpm_engine* e, mpm_tuning* t) {
@@ -2052,7 +2089,7 @@ extern "C" mpm_status mpm_autotune(mpm_engine* e, int32_t repeats, mpm_tuning* o
     cudaEventDestroy(b);
     e->tune = best;
     if (s != MPM_OK) return s;
-    if ((s = capture_graphs(e)) != MPM_OK) return s;
+    if ((s = reset_graphs(e)) != MPM_OK) return s;
     if (out) *out = best;
     return MPM_OK;
 }
