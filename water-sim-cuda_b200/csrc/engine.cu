@@ -31,9 +31,12 @@
 // the original order.
 #include <cuda_runtime.h>
 
+#include <unistd.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -123,7 +126,9 @@ struct mpm_engine {
     uint32_t* ctl = nullptr;
     mpm::OrderCtl order{};
     uint32_t* d_flags = nullptr;  // [0] health bits, [1] kernel status bits
-    uint32_t* h_flags = nullptr;  // their values at the last positions export (mapped host memory)
+    uint32_t* h_flags = nullptr;  // their values at the last positions export (a mapped host page, map_flags)
+    uint32_t* h_flags_dev = nullptr;  // the page's device address; null: the flags are copied
+    int exports = 0;                  // positions exports, counted until map_flags
     uint32_t wait_test = 0;       // MPM_WAIT_TEST_* (test hooks of the bounded device waits)
 
     float* staging = nullptr;  // device staging for imports/exports
@@ -580,7 +585,7 @@ void free_timing(mpm_engine* e) {
 // enqueued since export_positions, which left them in h_flags.
 mpm_status sync_and_collect(mpm_engine* e, bool exported = false) {
     uint32_t flags[2] = {0, 0};
-    exported = exported && e->n > 0;
+    exported = exported && e->n > 0 && e->h_flags_dev;
     if (!exported) CK(e, cudaMemcpyAsync(flags, e->d_flags, sizeof(flags), cudaMemcpyDeviceToHost, e->stream));
     CK(e, cudaStreamSynchronize(e->stream));
     if (exported) flags[0] = e->h_flags[0], flags[1] = e->h_flags[1];
@@ -679,12 +684,35 @@ mpm_status enter_scene(mpm_engine* e, int32_t scene) {
 
 // Exports the current positions into the other position buffer, once any
 // read-back of that buffer has finished, and makes it the current one.
+// The host page that the positions export writes the flags to: a copy of their
+// own costs every frame 7 us.  Registering a page takes 0.3 ms and giving it
+// back 0.2 (eight bytes from cudaHostAlloc 2.4 ms and 0.4 where the process holds
+// no other pinned memory, of the 4.6 ms that make a 64^3 engine), so the
+// kFlagsFrom-th export does it: an engine of few frames copies the flags, and so
+// does one whose page cannot be registered.
+constexpr int kFlagsFrom = 64;
+void map_flags(mpm_engine* e) {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    // Another thread's stream capture must not see it.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    void* dev = nullptr;
+    e->h_flags = static_cast<uint32_t*>(std::aligned_alloc(page, page));
+    if (e->h_flags && cudaHostRegister(e->h_flags, page, cudaHostRegisterMapped) == cudaSuccess &&
+        cudaHostGetDevicePointer(&dev, e->h_flags, 0) != cudaSuccess)
+        cudaHostUnregister(e->h_flags);
+    e->h_flags_dev = static_cast<uint32_t*>(dev);
+    if (!dev) cudaGetLastError();
+    cudaThreadExchangeStreamCaptureMode(&mode);
+}
+
 mpm_status export_positions(mpm_engine* e) {
+    if (e->exports < kFlagsFrom && ++e->exports == kFlagsFrom) map_flags(e);
     const int b = 1 - e->pos_cur;
     CK(e, cudaStreamWaitEvent(e->stream, e->copy_done[b], 0));
     e->kernel_launches +=
         mpm::launch_positions_export(e->n, e->P[e->parity], e->sigma[e->parity], e->pos_buf[b], e->d_flags,
-                                     e->h_flags, e->stream);
+                                     e->h_flags_dev, e->stream);
     CK(e, cudaGetLastError());
     CK(e, cudaEventRecord(e->pos_ready[b], e->stream));
     e->pos_cur = b;
@@ -734,8 +762,6 @@ mpm_status run_steps(mpm_engine* e, int32_t nsub) {
 // default, and from which the autotuner tries it.
 constexpr long long kTilesFrom = 1LL << 20;
 
-// Engine with `count` scenes; grid arrays, counter sets and the scene table
-// are allocated here, particle arrays by the first init.
 // The P2G accumulation grid as a persisting L2 window on the engine's
 // stream (the substep graphs captured from it carry the window): its
 // red.global.add reductions and the grid update's pass over it then hit L2
@@ -775,6 +801,8 @@ void keep_accum_in_l2(mpm_engine* e, int device) {
     e->l2_window = true;
 }
 
+// Engine with `count` scenes; grid arrays, counter sets and the scene table
+// are allocated here, particle arrays by the first init.
 mpm_status create_engine(const mpm_config* cfgs, int32_t count, int32_t device, mpm_engine** out) {
     g_global_error.clear();
     if (!cfgs || !out) return record(nullptr, MPM_ERR_INVALID_ARGUMENT, "configs and out must be non-NULL");
@@ -861,7 +889,6 @@ mpm_status create_engine(const mpm_config* cfgs, int32_t count, int32_t device, 
         (err = cudaMalloc(&e->vgrid, (size_t)g_total * sizeof(float4))) != cudaSuccess ||
         (err = cudaMalloc(&e->sdf, (size_t)g_total * sizeof(float))) != cudaSuccess ||
         (err = cudaMalloc(&e->d_flags, 2 * sizeof(uint32_t))) != cudaSuccess ||
-        (err = cudaHostAlloc(&e->h_flags, 2 * sizeof(uint32_t), cudaHostAllocMapped)) != cudaSuccess ||
         (err = cudaMalloc(&e->ctl, kCtlBytes)) != cudaSuccess ||
         (err = cudaMalloc(&e->bins_mem, bins_bytes(e))) != cudaSuccess ||
         (err = cudaMalloc(&e->tiles_mem, tiles_bytes(e))) != cudaSuccess ||
@@ -1183,7 +1210,8 @@ extern "C" void mpm_destroy(mpm_engine* e) {
     free_dev(e->d_goff);
     free_dev(e->d_boff);
     free_dev(e->d_flags);
-    if (e->h_flags) cudaFreeHost(e->h_flags);
+    if (e->h_flags_dev) cudaHostUnregister(e->h_flags);
+    std::free(e->h_flags);
     free_dev(e->staging);
     free_dev(e->d_prm_large);
     free_dev(e->mlp);

@@ -167,7 +167,7 @@ int launch_reference_keys(const SimParams& p, const float* P, const int32_t* sig
 int launch_state_export(const SimParams& p, const float* P, const int32_t* sigma, float* soa26, cudaStream_t st);
 // Float3 positions in original order (changeFormat, kernels.cu:341-347), all
 // scenes in one launch: xyz triple sigma[j] from slot j of P, j < n.  Also
-// flags_host[0..1] = flags[0..1].
+// flags_host[0..1] = flags[0..1] (flags_host may be null).
 int launch_positions_export(long long n, const float* P, const int32_t* sigma, float* xyz, const uint32_t* flags,
                             uint32_t* flags_host, cudaStream_t st);
 // Node float4 (mass, x, y, z) -> 4 planes.

@@ -1443,7 +1443,7 @@ __global__ void __launch_bounds__(256) positions_export_kernel(long long n, cons
                                                                const uint32_t* __restrict__ flags,
                                                                uint32_t* __restrict__ flags_host) {
     const long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (j < 2) flags_host[j] = flags[j];
+    if (flags_host && j < 2) flags_host[j] = flags[j];
     if (j >= n) return;
     const long long o = __ldg(sigma + j);
     const float4 q = __ldg(reinterpret_cast<const float4*>(P + (size_t)j * kAFloats));
