@@ -48,7 +48,7 @@ cudaError_t Readback::read(void* dst, const void* src, size_t bytes, cudaStream_
     }
     if (at.type != cudaMemoryTypeUnregistered) return plain();
     std::lock_guard<std::mutex> turn(turn_);
-    if (!slots_ && bytes < kAllocFrom) return plain();
+    if (!slots_ && (bytes < kCountFrom || (read_ += bytes) < kAllocFrom)) return plain();
     int device = 0;
     if (!prepare() || cudaGetDevice(&device) != cudaSuccess) return plain();
 

@@ -19,9 +19,13 @@
 
 namespace mpm {
 
-// The pinned slots belong to one engine or renderer: allocated by its first
-// read of kAllocFrom bytes or more (kThreads * kSlots * kChunk = 8 MB), given
-// back by the destructor.  Reads of several threads take turns.
+// The pinned slots (kThreads * kSlots * kChunk = 8 MB) belong to one engine or
+// renderer and are given back by its destructor.  Having them costs 4 to 8 ms
+// once, what 25 to 50 MB of reads into fresh pages gain, so they are allocated
+// when the object's reads of kCountFrom bytes or more have come to kAllocFrom:
+// allocated by the first such read, one of 17 / 21 / 31 MB took 6.9 / 12 / 10 ms,
+// plain ones 4.4 / 5.4 / 7.3; a first read of 208 MB takes 18 ms with them and 45
+// without.  Reads of several threads take turns.
 class Readback {
 public:
     Readback() = default;
@@ -32,8 +36,8 @@ public:
     // Copies `bytes` from device memory `src` to host memory `dst` after the
     // work enqueued on `st`; the data is there on return.  Pinned destinations and
     // reads of less than two threads' shares take one cudaMemcpyAsync, and so does
-    // every read where the slots cannot be had, or are not there yet and the read
-    // would not earn their allocation (a few milliseconds the first time).
+    // every read where the slots cannot be had, or are not there yet and the
+    // reads so far would not earn their allocation.
     cudaError_t read(void* dst, const void* src, size_t bytes, cudaStream_t st);
 
 private:
@@ -41,12 +45,14 @@ private:
     static constexpr int kSlots = 2;
     static constexpr size_t kChunk = size_t{512} << 10;
     static constexpr size_t kShare = size_t{4} << 20;  // bytes a thread is worth starting for
-    static constexpr size_t kAllocFrom = size_t{16} << 20;
+    static constexpr size_t kCountFrom = size_t{16} << 20;
+    static constexpr size_t kAllocFrom = size_t{128} << 20;
 
     bool prepare();
     void release();
 
     std::mutex turn_;
+    size_t read_ = 0;  // bytes of the reads counted before the slots were there
     char* slots_ = nullptr;
     cudaEvent_t done_[kThreads * kSlots] = {};
 };
