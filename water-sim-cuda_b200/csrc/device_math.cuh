@@ -49,7 +49,7 @@ struct SimParams {
     long long goff;       // first grid node
     long long coff;       // first cell: (nb + 1) * kBinCells cells per scene
     long long boff;       // first bin entry: nb + 2 entries per scene
-    unsigned long long inv_nbx, inv_nby;  // 2^48 / nbx and nby, rounded up: bin / nbx = bin * inv_nbx >> 48
+    unsigned long long inv_nbx, inv_nby;  // bin_reciprocal(nbx) and (nby), for bin_origin
 };
 
 // The scenes of an engine on the device: prm[s], and the prefix arrays
@@ -148,14 +148,19 @@ __device__ __forceinline__ int cell_of(const SimParams& p, float x, float y, flo
 // and |o| + n below 2^30.
 __host__ __device__ __forceinline__ bool in_range(int b, int o, int n) { return (unsigned)b - (unsigned)o < (unsigned)n; }
 
-// Node (0, 0, 0) of the stencil of the bin's first cell.  Bins number below
-// 2^24 (cells below 2^31), so the products stay below 2^64 and the quotients
-// by the reciprocals rounded up are exact: with m = (2^48 + e) / d, 0 <= e < d,
-// n m / 2^48 exceeds n / d by n e / (d 2^48) < 2^-24, less than the 1 / d it
-// would take to reach the next whole number.
-__device__ __forceinline__ void bin_origin(const SimParams& p, int bin, int* x, int* y, int* z) {
-    const int row = (int)((unsigned long long)bin * p.inv_nbx >> 48);
-    const int slab = (int)((unsigned long long)row * p.inv_nby >> 48);
+// n / d for 0 <= n < 2^31 and d > 0 by the reciprocal m = bin_reciprocal(d) =
+// (2^64 - 1 - r) / d, 0 <= r < d: the high 64 bits of (n + 1) m.  (n + 1) m / 2^64
+// falls short of (n + 1) / d by (n + 1) (1 + r) / (d 2^64), more than 0 and less
+// than the 1 / d from (n + 1) / d down to n / d, so its whole part is n / d's.
+__host__ __device__ __forceinline__ unsigned long long bin_reciprocal(int d) { return ~0ull / (unsigned)d; }
+__host__ __device__ __forceinline__ int bin_quotient(int n, unsigned long long m) {
+    const unsigned long long k = (unsigned)n + 1u;
+    return (int)(((k * (m & 0xFFFFFFFFull) >> 32) + k * (m >> 32)) >> 32);
+}
+
+// Node (0, 0, 0) of the stencil of the bin's first cell.
+__host__ __device__ __forceinline__ void bin_origin(const SimParams& p, int bin, int* x, int* y, int* z) {
+    const int row = bin_quotient(bin, p.inv_nbx), slab = bin_quotient(row, p.inv_nby);
     *x = (bin - row * p.nbx) * kBinX - 2;
     *y = (row - slab * p.nby) * kBinY - 2;
     *z = slab * kBinZ - 2;

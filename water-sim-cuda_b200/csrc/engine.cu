@@ -834,8 +834,8 @@ mpm_status create_engine(const mpm_config* cfgs, int32_t count, int32_t device, 
         p.nby = (cfg->size_y + 2 + mpm::kBinY - 1) / mpm::kBinY;
         p.nbz = (cfg->size_z + 2 + mpm::kBinZ - 1) / mpm::kBinZ;
         p.nb = p.nbx * p.nby * p.nbz;
-        p.inv_nbx = ((1ull << 48) + p.nbx - 1) / p.nbx;
-        p.inv_nby = ((1ull << 48) + p.nby - 1) / p.nby;
+        p.inv_nbx = mpm::bin_reciprocal(p.nbx);
+        p.inv_nby = mpm::bin_reciprocal(p.nby);
         p.poff = 0;
         p.goff = g_total;
         p.coff = cells_total;
