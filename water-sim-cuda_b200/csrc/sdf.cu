@@ -552,17 +552,23 @@ static uint32_t morton10(float x, float y, float z) {
 
 // Whether the winding number is a whole number off the mesh and the kernels
 // may rely on the distances: every edge is run through as often one way as the
-// other (vertices compared by value), and FP32 distances are good to half of
-// the 0.001 by which the sign kernel's balls fall short of them.  They err by a
-// few units in the last place of the coordinates, hence kSpreadCoord, and on
-// long thin triangles by the barycentric coordinates' cancellation, which
-// grows like L (L / h)^2 with the longest edge L and the height h: in FP32
-// against 64 bits over rotated boxes at most 1e-4 at 1.6e4, 8e-4 at 1.1e5 and
-// 2.3e-3 at 2.5e5, hence kSpreadSliver.  The edges are matched by adding up a 128-bit hash
+// other (vertices compared by value), and FP32 distances exceed the true ones
+// by less than half of the 0.001 by which the sign kernel's balls fall short of
+// them (a distance that is too small costs a spread, never a sign).  A closest
+// point errs by a few units in the last place of the coordinates, hence
+// kSpreadCoord, and within the triangle's plane by the cancellation in its
+// barycentric coordinates, d = about 5e-8 L (L / h)^2 with the longest edge L and
+// the height h, which lengthens a distance D by d^2 / 2D: most at the smallest
+// that takes part in the spread (kSdfOnMesh; nodes nearer get a sum of their
+// own), hence kSpreadSliver.  Measured against 64 bits, with and without
+// contraction, over 1e9 pairs of a triangle and a point at 0.01 or more from
+// it: at most 1.8e-4 within both limits together, 3e-5 within kSpreadSliver
+// alone at coordinates of 64 (1.2e-4 at twice the limit, 5e-4 at five times).
+// The edges are matched by adding up a 128-bit hash
 // of each, with the sign of its direction: the sums vanish when every edge
 // cancels, and else with a probability of 2^-128.
 constexpr float kSpreadCoord = 1024.0f;
-constexpr double kSpreadSliver = 4e4;
+constexpr double kSpreadSliver = 2e4;
 static bool closed_mesh(const float* tris, int t) {
     auto mix = [](uint64_t v) {  // the finaliser of MurmurHash3 (public domain)
         v ^= v >> 33;
