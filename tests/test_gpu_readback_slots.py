@@ -1,6 +1,6 @@
-"""The read-back's pinned slots: a first large read does not pay for them, and
-reads on both sides of the line from which they are used (128 MiB of large reads
-of one object), of one thread and of several, give the same bytes."""
+"""The read-back's pinned slots: a first large read takes no longer for them than
+one plain copy into a new array takes (a quarter more allowed), and reads of one
+thread and of several through them give the bytes of a pinned read."""
 import threading
 import time
 
@@ -9,7 +9,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-N = 300001  # a state of 31.2 MB: the fifth read crosses the line
+N = 300001  # a state of 31.2 MB
 
 
 def _engine(mpm, n):
@@ -28,14 +28,14 @@ def _pinned_state(mpm, e, n):
     return want
 
 
-def test_reads_across_the_line(gpu_ok, mpm):
+def test_reads(gpu_ok, mpm):
     with _engine(mpm, N) as e:
         want = _pinned_state(mpm, e, N)
-        for _ in range(7):
+        for _ in range(3):
             assert np.array_equal(e.get_buffer().view(np.uint32), want.view(np.uint32))
 
 
-def test_first_read_of_the_line_itself(gpu_ok, mpm):
+def test_large_first_read(gpu_ok, mpm):
     n = 1300000  # 135 MB in one read
     with _engine(mpm, n) as e:
         want = _pinned_state(mpm, e, n)
@@ -43,7 +43,7 @@ def test_first_read_of_the_line_itself(gpu_ok, mpm):
             assert np.array_equal(e.get_buffer().view(np.uint32), want.view(np.uint32))
 
 
-def test_threads_across_the_line(gpu_ok, mpm):
+def test_threads(gpu_ok, mpm):
     from mpm_b200 import scenes
     cfg, st, tris = scenes.small_scene(2000, (189, 183, 181), seed=4)  # a field of 25 MB
     with mpm.Engine(cfg) as e:
@@ -64,16 +64,21 @@ def test_threads_across_the_line(gpu_ok, mpm):
             assert np.array_equal(g, want)
 
 
-def test_first_read_is_no_slower_than_the_second(gpu_ok, mpm):
-    n = 200000  # 20.8 MB; both reads are plain copies into new arrays
+def test_first_read_is_no_slower_than_one_copy(gpu_ok, mpm):
+    import torch
+    n = 165000  # 17.2 MB: the slots come with this read
     ratio = []
-    for _ in range(5):
+    for _ in range(7):
         with _engine(mpm, n) as e:
+            on_device = torch.zeros((26, n), device="cuda")
+            torch.cuda.synchronize()
             took = []
-            for _ in range(2):
-                out = np.empty((26, n), np.float32)
+            for read in (lambda o: mpm.lib.mpm_get_state(e._h, o.ctypes.data),
+                         lambda o: torch.from_numpy(o).copy_(on_device) is None):
+                # of an array too large for the allocator to recycle: new pages
+                out = np.empty(12000000, np.float32)[:26 * n].reshape(26, n)
                 begin = time.perf_counter()
-                assert mpm.lib.mpm_get_state(e._h, out.ctypes.data) == 0
+                assert not read(out)
                 took.append(time.perf_counter() - begin)
             ratio.append(took[0] / took[1])
-    assert sorted(ratio)[2] < 2.0, ratio  # 4 to 7 with the slots allocated by the first
+    assert sorted(ratio)[3] <= 1.25, ratio  # 1.4 to 2.4 with slots from cudaHostAlloc

@@ -31,12 +31,9 @@
 // the original order.
 #include <cuda_runtime.h>
 
-#include <unistd.h>
-
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
-#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -126,7 +123,8 @@ struct mpm_engine {
     uint32_t* ctl = nullptr;
     mpm::OrderCtl order{};
     uint32_t* d_flags = nullptr;  // [0] health bits, [1] kernel status bits
-    uint32_t* h_flags = nullptr;  // their values at the last positions export (a mapped host page, map_flags)
+    mpm::PinnedPages flags_page;
+    uint32_t* h_flags = nullptr;  // in it: their values at the last positions export (map_flags)
     uint32_t* h_flags_dev = nullptr;  // the page's device address; null: the flags are copied
     int exports = 0;                  // positions exports, counted until map_flags
     uint32_t wait_test = 0;       // MPM_WAIT_TEST_* (test hooks of the bounded device waits)
@@ -685,24 +683,21 @@ mpm_status enter_scene(mpm_engine* e, int32_t scene) {
 // Exports the current positions into the other position buffer, once any
 // read-back of that buffer has finished, and makes it the current one.
 // The host page that the positions export writes the flags to: a copy of their
-// own costs every frame 7 us.  Registering a page takes 0.3 ms and giving it
-// back 0.2 (eight bytes from cudaHostAlloc 2.4 ms and 0.4 where the process holds
-// no other pinned memory, of the 4.6 ms that make a 64^3 engine), so the
-// kFlagsFrom-th export does it: an engine of few frames copies the flags, and so
-// does one whose page cannot be registered.
+// own costs every frame 7 us.  The page costs an engine 0.5 ms, so the
+// kFlagsFrom-th export takes it: an engine of few frames copies the flags, and so
+// does one that cannot have the page.  (Eight bytes from cudaHostAlloc at
+// creation took a 64^3 engine's from 4.6 to 7.1 ms.)
 constexpr int kFlagsFrom = 64;
 void map_flags(mpm_engine* e) {
-    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
     // Another thread's stream capture must not see it.
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     cudaThreadExchangeStreamCaptureMode(&mode);
     void* dev = nullptr;
-    e->h_flags = static_cast<uint32_t*>(std::aligned_alloc(page, page));
-    if (e->h_flags && cudaHostRegister(e->h_flags, page, cudaHostRegisterMapped) == cudaSuccess &&
-        cudaHostGetDevicePointer(&dev, e->h_flags, 0) != cudaSuccess)
-        cudaHostUnregister(e->h_flags);
+    if (e->flags_page.allocate(2 * sizeof(uint32_t), false) &&
+        cudaHostGetDevicePointer(&dev, e->flags_page.data(), 0) != cudaSuccess)
+        cudaGetLastError();
+    e->h_flags = static_cast<uint32_t*>(e->flags_page.data());
     e->h_flags_dev = static_cast<uint32_t*>(dev);
-    if (!dev) cudaGetLastError();
     cudaThreadExchangeStreamCaptureMode(&mode);
 }
 
@@ -1210,8 +1205,6 @@ extern "C" void mpm_destroy(mpm_engine* e) {
     free_dev(e->d_goff);
     free_dev(e->d_boff);
     free_dev(e->d_flags);
-    if (e->h_flags_dev) cudaHostUnregister(e->h_flags);
-    std::free(e->h_flags);
     free_dev(e->staging);
     free_dev(e->d_prm_large);
     free_dev(e->mlp);

@@ -1,7 +1,10 @@
 #include "readback.h"
 
+#include <sys/mman.h>
+
 #include <algorithm>
 #include <atomic>
+#include <cstdint>
 #include <cstring>
 #include <thread>
 
@@ -14,8 +17,37 @@ void Readback::release() {
         if (e) cudaEventDestroy(e);
         e = nullptr;
     }
-    if (slots_) cudaFreeHost(slots_);
     slots_ = nullptr;
+    memory_.release();
+}
+
+bool PinnedPages::allocate(size_t bytes, bool huge) {
+    constexpr size_t kHugePage = size_t{2} << 20;
+    const size_t align = huge ? kHugePage : 1;
+    mapped_ = bytes + align - 1;
+    base_ = mmap(nullptr, mapped_, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (base_ == MAP_FAILED) {
+        base_ = nullptr;
+        return false;
+    }
+    const uintptr_t at = (reinterpret_cast<uintptr_t>(base_) + align - 1) / align * align;
+    data_ = reinterpret_cast<void*>(at);
+    if (huge) madvise(data_, bytes, MADV_HUGEPAGE);  // only a hint
+    // A forked child must not share the pages: the first write after a fork
+    // could otherwise leave this process with a copy the device knows nothing of.
+    madvise(data_, bytes, MADV_DONTFORK);
+    if (cudaHostRegister(data_, bytes, cudaHostRegisterMapped) == cudaSuccess) return true;
+    cudaGetLastError();
+    munmap(base_, mapped_);
+    base_ = data_ = nullptr;
+    return false;
+}
+
+void PinnedPages::release() {
+    if (!base_) return;
+    cudaHostUnregister(data_);
+    munmap(base_, mapped_);
+    base_ = data_ = nullptr;
 }
 
 bool Readback::prepare() {
@@ -23,7 +55,8 @@ bool Readback::prepare() {
     // Allocations that another thread's stream capture must not see.
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     cudaThreadExchangeStreamCaptureMode(&mode);
-    cudaError_t err = cudaHostAlloc(reinterpret_cast<void**>(&slots_), kThreads * kSlots * kChunk, cudaHostAllocDefault);
+    cudaError_t err = memory_.allocate(kThreads * kSlots * kChunk, true) ? cudaSuccess : cudaErrorMemoryAllocation;
+    slots_ = static_cast<char*>(memory_.data());
     for (int k = 0; k < kThreads * kSlots && err == cudaSuccess; ++k)
         err = cudaEventCreateWithFlags(&done_[k], cudaEventDisableTiming);
     cudaThreadExchangeStreamCaptureMode(&mode);
@@ -48,7 +81,7 @@ cudaError_t Readback::read(void* dst, const void* src, size_t bytes, cudaStream_
     }
     if (at.type != cudaMemoryTypeUnregistered) return plain();
     std::lock_guard<std::mutex> turn(turn_);
-    if (!slots_ && (bytes < kCountFrom || (read_ += bytes) < kAllocFrom)) return plain();
+    if (!slots_ && bytes < kAllocFrom) return plain();
     int device = 0;
     if (!prepare() || cudaGetDevice(&device) != cudaSuccess) return plain();
 

@@ -19,13 +19,33 @@
 
 namespace mpm {
 
+// Page-locked, mapped host memory of whole pages: ordinary pages, registered.
+// One page takes 0.3 ms and 0.2 to give back, 8 MB of huge pages 0.7 and 0.3;
+// cudaHostAlloc takes 2.4 and 0.4 ms for 8 bytes where the process holds no
+// other pinned memory, 5.9 and 1.0 for 8 MB.
+class PinnedPages {
+public:
+    PinnedPages() = default;
+    PinnedPages(const PinnedPages&) = delete;
+    PinnedPages& operator=(const PinnedPages&) = delete;
+    ~PinnedPages() { release(); }
+
+    bool allocate(size_t bytes, bool huge);  // false: it cannot be had, nothing is held
+    void release();
+    void* data() const { return data_; }
+
+private:
+    void* base_ = nullptr;
+    void* data_ = nullptr;
+    size_t mapped_ = 0;
+};
+
 // The pinned slots (kThreads * kSlots * kChunk = 8 MB) belong to one engine or
-// renderer and are given back by its destructor.  Having them costs 4 to 8 ms
-// once, what 25 to 50 MB of reads into fresh pages gain, so they are allocated
-// when the object's reads of kCountFrom bytes or more have come to kAllocFrom:
-// allocated by the first such read, one of 17 / 21 / 31 MB took 6.9 / 12 / 10 ms,
-// plain ones 4.4 / 5.4 / 7.3; a first read of 208 MB takes 18 ms with them and 45
-// without.  Reads of several threads take turns.
+// renderer: allocated by its first read of kAllocFrom bytes or more, given back
+// by the destructor.  That read pays for them: 17 / 21 / 31 MB into new arrays
+// take 2.7 / 2.9 / 3.1 ms the first time, 1.6 / 1.9 / 2.4 then, one copy 4.2 / 5.1
+// / 7.3 (the first time with slots from cudaHostAlloc 7 / 9 / 9 ms).  Reads of
+// several threads take turns.
 class Readback {
 public:
     Readback() = default;
@@ -36,8 +56,8 @@ public:
     // Copies `bytes` from device memory `src` to host memory `dst` after the
     // work enqueued on `st`; the data is there on return.  Pinned destinations and
     // reads of less than two threads' shares take one cudaMemcpyAsync, and so does
-    // every read where the slots cannot be had, or are not there yet and the
-    // reads so far would not earn their allocation.
+    // every read where the slots cannot be had, or are not there yet and the read
+    // would not earn their allocation.
     cudaError_t read(void* dst, const void* src, size_t bytes, cudaStream_t st);
 
 private:
@@ -45,15 +65,14 @@ private:
     static constexpr int kSlots = 2;
     static constexpr size_t kChunk = size_t{512} << 10;
     static constexpr size_t kShare = size_t{4} << 20;  // bytes a thread is worth starting for
-    static constexpr size_t kCountFrom = size_t{16} << 20;
-    static constexpr size_t kAllocFrom = size_t{128} << 20;
+    static constexpr size_t kAllocFrom = size_t{16} << 20;
 
     bool prepare();
     void release();
 
     std::mutex turn_;
-    size_t read_ = 0;  // bytes of the reads counted before the slots were there
     char* slots_ = nullptr;
+    PinnedPages memory_;
     cudaEvent_t done_[kThreads * kSlots] = {};
 };
 
