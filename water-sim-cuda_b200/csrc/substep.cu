@@ -1043,19 +1043,20 @@ constexpr int kStagePlanes = 9;  // planes of 60 nodes: 8.6 KB per CTA
 
 // CTAs per SM: the learned tcgen05 mode fits four (64 registers, 128 TMEM
 // columns and about 45 KB of shared memory each), so one CTA's MMA waits
-// overlap the other three's work; mma.sync learned and collect modes and the
-// batched large steps need more registers.  The batched substep would like 80
+// overlap the other three's work; mma.sync learned and collect modes need more
+// registers.  Large steps are of one scene (launch_g2p).  The batched substep would like 80
 // (64 spill 72 bytes), but a fourth CTA is worth more: 64 scenes with 6.1M
 // particles 291 / 263 us.  The tcgen05 mode at 2M particles: 330 us with
 // per-warp statistics, node-by-node sums and scalar GELU, 225 us now (three
 // CTAs of 80 registers without spills: 254 against 243 us before the row sums).
 template <bool kBatch, int kMode>
-__global__ void __launch_bounds__(256, kMode == 1 ? 2 : (((kBatch && kMode != 0) || kMode == 2) ? 3 : 4)) g2p_kernel(
+__global__ void __launch_bounds__(256, kMode == kG2PLearned ? 2 : (kMode == kG2PCollect ? 3 : 4)) g2p_kernel(
     SceneTable sc, SimParams p0, long long n_total, const float* __restrict__ Pin, float* __restrict__ Pout,
     const int32_t* __restrict__ gidx, const int2* __restrict__ edge, const int32_t* __restrict__ sig_in,
     int32_t* __restrict__ sig_out, const float4* __restrict__ vgrid_all, const float* __restrict__ sdf_all,
     int32_t* __restrict__ pcell, BinSet next, uint32_t* __restrict__ crowded, uint32_t* __restrict__ health,
     LearnArgs la) {
+    static_assert(!kBatch || kMode == kG2PPlain, "large steps are of one scene");
     pdl_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) *crowded = 0u;  // P2G has taken its crowded-cell list
     __shared__ SimParams s_prm[kBatch ? kTableScenes : 1];
@@ -1584,7 +1585,7 @@ int launch_g2p(const SceneTable& sc, const SimParams& p0, long long n, const flo
                const int32_t* gidx, const int2* edge, const int32_t* sig_in, int32_t* sig_out, const float4* vgrid,
                const float* sdf, int32_t* pcell, const BinSet& next, uint32_t* crowded, uint32_t* health,
                cudaStream_t st, const LearnArgs* learn, int block) {
-    if (n <= 0) return 0;
+    if (n <= 0 || (learn && sc.count != 1)) return 0;  // learned_ready refuses batches
     const LearnArgs la = learn ? *learn : LearnArgs{};
     // The learned modes work on 256 particles per CTA; the others take 128 too.
     auto go = [&](auto kernel, int threads, size_t smem) {
@@ -1592,10 +1593,10 @@ int launch_g2p(const SceneTable& sc, const SimParams& p0, long long n, const flo
                    vgrid, sdf, pcell, next, crowded, health, la);
     };
     const int plain = block == 128 ? 128 : 256;
-    if (learn && sc.count == 1 && la.mlp_tc) go(g2p_kernel<false, kG2PLearnedTc>, 256, sizeof(MlpTcSmem));
-    else if (learn && sc.count == 1 && la.mlp) go(g2p_kernel<false, kG2PLearned>, 256, 0);
-    else if (learn && sc.count == 1 && la.feat) go(g2p_kernel<false, kG2PCollect>, 256, 0);
-    else if (learn && sc.count == 1) go(g2p_kernel<false, kG2PLarge>, 256, 0);
+    if (learn && la.mlp_tc) go(g2p_kernel<false, kG2PLearnedTc>, 256, sizeof(MlpTcSmem));
+    else if (learn && la.mlp) go(g2p_kernel<false, kG2PLearned>, 256, 0);
+    else if (learn && la.feat) go(g2p_kernel<false, kG2PCollect>, 256, 0);
+    else if (learn) go(g2p_kernel<false, kG2PLarge>, 256, 0);
     else if (sc.count == 1) go(g2p_kernel<false, kG2PPlain>, plain, 0);
     else go(g2p_kernel<true, kG2PPlain>, plain, 0);
     return 1;
