@@ -77,6 +77,8 @@ __device__ __forceinline__ float ord_dec(unsigned u) {
 // smaller) drops those before the atomic.  Particles go last to first, since
 // scenes are seeded with z ascending and the default camera looks down -z, so
 // that near ones mostly come first.  2M particles, 1920 x 1600: 1064 -> 401 us.
+// From behind they come last, the order's worst case; the drop then gains less
+// (all passes of a frame 1.22 / 0.82 ms, from the front 0.87 / 0.44).
 __global__ void splat_kernel(const float* __restrict__ xyz, long long n, Cam c, unsigned* zbuf) {
     const long long i = n - 1 - (blockIdx.x * (long long)blockDim.x + threadIdx.x);
     if (i < 0) return;

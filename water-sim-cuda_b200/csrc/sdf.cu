@@ -36,7 +36,7 @@
 // Measured (distance + sign): 128^3 nodes and 2,304 triangles 30.9 -> 0.52 +
 // 0.36 ms, 256^3 and 3,276 triangles 330 -> 2.96 + 1.81 ms; with an open mesh,
 // whose sign takes the sum at every node, 31.1 -> 27.3 and 330 -> 301 ms.  The
-// distance kernel is bound by issue (79 % of issue slots, about 130 box tests
+// distance kernel is bound by issue (81 % of issue slots, about 130 box tests
 // and 30 triangles a brick), the sign kernel by the chain of sums of the few
 // bricks that the mesh crosses.
 //

@@ -171,8 +171,8 @@ struct SceneLookup {
 // (cell_scan_kernel).  Unlike the reference, no partial sum is dropped (it
 // drops shared-tile cells whose partial mass is <= 1e-9, kernels.cu:132).
 // What bounds it: the 108 sums leave room for 12 warps per SM, whose
-// instructions (about 510 per 32 particles) and waits take turns: 47 % of the
-// issue slots, DRAM at 2.5 TB/s.  2M particles 86.7 us (29 us for the records
+// instructions (about 670 per 32 particles) and waits take turns: 46 % of the
+// issue slots, DRAM at 2.9 TB/s.  2M particles 86.7 us (29 us for the records
 // alone), 6.1M in 64 scenes 253 us.  Taking the next unit while one is summed
 // or written out, to hide the unit's three dependent loads, made the last
 // units uneven: 93.1 and 88.7 us.
@@ -1028,7 +1028,7 @@ enum G2PMode : int { kG2PPlain = 0, kG2PLearned = 1, kG2PCollect = 2, kG2PLarge 
 // its threads still follow gidx to their records; the 27 node reads of a
 // particle then hit shared memory.  (Straight from global memory every row of
 // three nodes is an L1 or L2 round trip of its own, about ten in a row per
-// particle at 64 registers: 12.5 long-scoreboard stalls per issue.)  A
+// particle at 64 registers: 11 long-scoreboard stalls per issue, 5 now.)  A
 // particle of neither region (a run that crosses a third bin, as in sparse
 // fluid) reads the grid.  Nodes outside the grid are staged as zeros whose
 // mass has its sign bit set, like a node inside an obstacle: either way the
@@ -1037,7 +1037,7 @@ enum G2PMode : int { kG2PPlain = 0, kG2PLearned = 1, kG2PCollect = 2, kG2PLarge 
 // G2P per substep before / after (with 128-thread CTAs, whose barrier waits for
 // fewer warps: 94 us at 256; and with reductions instead of returning atomics
 // in the filing): 650k particles 37.6 / 30.4 us, 2M 104 / 83 us, 6.9M in 256^3
-// 325 / 258 us, the 64-scene batch 362 / 263 us.  DRAM then carries 3.9 of the
+// 325 / 258 us, the 64-scene batch 362 / 263 us.  DRAM then carries 4.5 of the
 // 6.5 TB/s; issue (57 % of slots) and the chain gidx - record - stores bound it.
 constexpr int kStagePlanes = 9;  // planes of 60 nodes: 8.6 KB per CTA
 
@@ -1432,7 +1432,7 @@ __global__ void __launch_bounds__(256) state_export_kernel(SimParams p, const fl
 // Positions of all particles of all scenes in original order; sigma numbers
 // particles across them, so no scene table is needed.  Bound by DRAM: a
 // position is 16 bytes of every 96, but every 128-byte line of the records is
-// fetched for it (2M particles: 199 MB read, 5.7 TB/s), and laying out the
+// fetched for it (2M particles: 191 MB of records in 32 us), and laying out the
 // triples in shared memory for denser stores changed nothing.
 // One launch for all scenes, not one each: 64 scenes with 6.1M particles 290 /
 // 99 us; 2M particles 38.5 us either way.  The export follows every frame, so it
