@@ -108,7 +108,7 @@ __device__ __forceinline__ int stencil_base(float pos) { return __float2int_rz(_
 // 2012), the sequence expandBits uses (common.cuh:277-284).  Inputs >= 1024
 // alias exactly as there, which keeps keys bit-exact for particles outside
 // a 1024^3 box.
-__device__ __forceinline__ uint32_t spread_bits3(uint32_t v) {
+__host__ __device__ __forceinline__ uint32_t spread_bits3(uint32_t v) {
     v = (v * 0x00010001u) & 0xFF0000FFu;
     v = (v * 0x00000101u) & 0x0F00F00Fu;
     v = (v * 0x00000011u) & 0xC30C30C3u;

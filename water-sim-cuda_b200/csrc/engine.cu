@@ -482,6 +482,7 @@ cudaError_t load_graph(cudaGraphExec_t* exec, cudaGraph_t g) {
 // of four substeps launches none (chain_graph), so that init captures nothing.
 mpm_status substep_graph(mpm_engine* e, int par) {
     if (e->graph[par] && !e->graph_stale[par]) return MPM_OK;
+    const mpm::OutsideCaptures outside;
     const bool timed = e->timing_cap > 0;
     cudaGraph_t g = nullptr;
     CK(e, cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
@@ -544,6 +545,7 @@ cudaGraphExec_t chain_graph(mpm_engine* e) {
     const int par = e->parity;
     if (e->timing_cap > 0 || e->chain_off) return nullptr;
     if (e->chain[par] && !e->chain_stale[par]) return e->chain[par];
+    const mpm::OutsideCaptures outside;
     e->chain_off = true;
     if (cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
         cudaGetLastError();
@@ -689,16 +691,13 @@ mpm_status enter_scene(mpm_engine* e, int32_t scene) {
 // creation took a 64^3 engine's from 4.6 to 7.1 ms.)
 constexpr int kFlagsFrom = 64;
 void map_flags(mpm_engine* e) {
-    // Another thread's stream capture must not see it.
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
+    const mpm::OutsideCaptures outside;
     void* dev = nullptr;
     if (e->flags_page.allocate(2 * sizeof(uint32_t), false) &&
         cudaHostGetDevicePointer(&dev, e->flags_page.data(), 0) != cudaSuccess)
         cudaGetLastError();
     e->h_flags = static_cast<uint32_t*>(e->flags_page.data());
     e->h_flags_dev = static_cast<uint32_t*>(dev);
-    cudaThreadExchangeStreamCaptureMode(&mode);
 }
 
 mpm_status export_positions(mpm_engine* e) {

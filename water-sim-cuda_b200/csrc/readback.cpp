@@ -52,14 +52,11 @@ void PinnedPages::release() {
 
 bool Readback::prepare() {
     if (slots_) return true;
-    // Allocations that another thread's stream capture must not see.
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
+    const OutsideCaptures outside;
     cudaError_t err = memory_.allocate(kThreads * kSlots * kChunk, true) ? cudaSuccess : cudaErrorMemoryAllocation;
     slots_ = static_cast<char*>(memory_.data());
     for (int k = 0; k < kThreads * kSlots && err == cudaSuccess; ++k)
         err = cudaEventCreateWithFlags(&done_[k], cudaEventDisableTiming);
-    cudaThreadExchangeStreamCaptureMode(&mode);
     if (err == cudaSuccess) return true;
     cudaGetLastError();
     release();

@@ -19,6 +19,20 @@
 
 namespace mpm {
 
+// While it lives, this thread's calls are not seen by a stream capture of another
+// library's or thread's (one in the global mode refuses allocations, captures
+// and instantiations everywhere, and is invalidated by them).
+class OutsideCaptures {
+public:
+    OutsideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    ~OutsideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    OutsideCaptures(const OutsideCaptures&) = delete;
+    OutsideCaptures& operator=(const OutsideCaptures&) = delete;
+
+private:
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
+
 // Page-locked, mapped host memory of whole pages: ordinary pages, registered.
 // One page takes 0.3 ms and 0.2 to give back, 8 MB of huge pages 0.7 and 0.3;
 // cudaHostAlloc takes 2.4 and 0.4 ms for 8 bytes where the process holds no

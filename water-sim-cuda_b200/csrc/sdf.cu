@@ -539,15 +539,8 @@ __global__ void __launch_bounds__(kSdfThreads) sdf_sign_kernel(SimParams p, cons
 
 // Morton code of a point in [0, 1)^3, 10 bits per axis.
 static uint32_t morton10(float x, float y, float z) {
-    auto spread = [](uint32_t v) {
-        v = (v * 0x00010001u) & 0xFF0000FFu;
-        v = (v * 0x00000101u) & 0x0F00F00Fu;
-        v = (v * 0x00000011u) & 0xC30C30C3u;
-        v = (v * 0x00000005u) & 0x49249249u;
-        return v;
-    };
     auto q = [](float f) { return (uint32_t)std::min(1023.0f, std::max(0.0f, f * 1024.0f)); };
-    return (spread(q(z)) << 2) | (spread(q(y)) << 1) | spread(q(x));
+    return (spread_bits3(q(z)) << 2) | (spread_bits3(q(y)) << 1) | spread_bits3(q(x));
 }
 
 // Whether the winding number is a whole number off the mesh and the kernels
