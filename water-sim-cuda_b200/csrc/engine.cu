@@ -138,8 +138,7 @@ struct mpm_engine {
     bool accum_dirty = false;
     GridView grid_view = GridView::kVelocity;
 
-    // Captured when first needed; stale: to be captured again before its next
-    // launch (reset_graphs).
+    // Stale: to be captured again before its next launch (reset_graphs).
     cudaGraphExec_t graph[2] = {nullptr, nullptr};  // one substep from parity 0 / 1
     cudaGraph_t graph_src[2] = {nullptr, nullptr};  // kept for the nodes of the stage timing
     bool graph_stale[2] = {false, false};
@@ -444,23 +443,6 @@ int enqueue_substep(mpm_engine* e, int par, int from, int upto, const cudaEvent_
     return launches;
 }
 
-// The substep graphs are captured again, with the launch shapes and sizes of
-// now, when next launched (substep_graph, chain_graph).  Their executables are
-// kept to be updated in place, but for those with stage-timing nodes.
-mpm_status reset_graphs(mpm_engine* e) {
-    destroy_learned_graphs(e);  // they embed the launch shapes too
-    // Touched tiles only: after updates of every node any tile may hold
-    // velocities, so the first tile update resets every tile not marked.
-    if (active_tiles(e).mark) CK(e, cudaMemsetAsync(e->tiles.dirty, 1, (size_t)e->bins_total, e->stream));
-    if (e->timing_cap > 0 || e->graph_timing > 0) destroy_graphs(e);
-    for (int k = 0; k < 2; ++k) e->graph_stale[k] = e->chain_stale[k] = true;
-    e->chain_off = false;
-    e->graph_prm = e->prm;
-    e->graph_tune = e->tune;
-    e->graph_timing = e->timing_cap;
-    return MPM_OK;
-}
-
 // Makes *exec run `g`: a captured sequence of the same kernels as before, with
 // other counts and grid sizes, updates the executable in place; else a new one.
 // Load of a state of another count / load and a frame of four substeps, 8k
@@ -479,7 +461,7 @@ cudaError_t load_graph(cudaGraphExec_t* exec, cudaGraph_t g) {
 }
 
 // Makes graph[par], one substep from parity `par`, fit to be launched.  A frame
-// of four substeps launches none (chain_graph), so that init captures nothing.
+// of four substeps launches none (chain_graph).
 mpm_status substep_graph(mpm_engine* e, int par) {
     if (e->graph[par] && !e->graph_stale[par]) return MPM_OK;
     const mpm::OutsideCaptures outside;
@@ -522,6 +504,29 @@ mpm_status substep_graph(mpm_engine* e, int par) {
         CK(e, cudaGraphInstantiate(&e->graph[par], g, 0));
     }
     e->graph_stale[par] = false;
+    return MPM_OK;
+}
+
+// The substep graphs are captured again, with the launch shapes and sizes of
+// now, when next launched (substep_graph, chain_graph).  Their executables are
+// kept to be updated in place, but for those with stage-timing nodes; the single
+// ones are made here where there are none, so that no later step depends on
+// memory being left for one (a chain that cannot be had is done without).
+mpm_status reset_graphs(mpm_engine* e) {
+    destroy_learned_graphs(e);  // they embed the launch shapes too
+    // Touched tiles only: after updates of every node any tile may hold
+    // velocities, so the first tile update resets every tile not marked.
+    if (active_tiles(e).mark) CK(e, cudaMemsetAsync(e->tiles.dirty, 1, (size_t)e->bins_total, e->stream));
+    if (e->timing_cap > 0 || e->graph_timing > 0) destroy_graphs(e);
+    for (int k = 0; k < 2; ++k) e->graph_stale[k] = e->chain_stale[k] = true;
+    e->chain_off = false;
+    e->graph_prm = e->prm;
+    e->graph_tune = e->tune;
+    e->graph_timing = e->timing_cap;
+    for (int par = 0; par < 2; ++par) {
+        const mpm_status st = e->graph[par] ? MPM_OK : substep_graph(e, par);
+        if (st != MPM_OK) return st;
+    }
     return MPM_OK;
 }
 
