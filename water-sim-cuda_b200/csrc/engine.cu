@@ -447,8 +447,8 @@ int enqueue_substep(mpm_engine* e, int par, int from, int upto, const cudaEvent_
 // other counts and grid sizes, updates the executable in place; else a new one.
 // Load of a state of another count / load and a frame of four substeps, 8k
 // particles: both single graphs captured and instantiated in the load, then the
-// chain, 361 / 643 us; only the chain, updated, 125 / 257 us (a state of the
-// same count, whose graphs are kept: 125 / 227 us).
+// chain, 361 / 643 us; only the chain, updated, 122 / 249 us (a state of the
+// same count, whose graphs are kept: 119 / 227 us).
 cudaError_t load_graph(cudaGraphExec_t* exec, cudaGraph_t g) {
     if (*exec) {
         cudaGraphExecUpdateResultInfo info;
